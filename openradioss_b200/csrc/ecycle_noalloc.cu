@@ -37,21 +37,36 @@
 #include <cstdlib>
 #include <mutex>
 #include <thread>
+#include <utility>
 #include <cuda_runtime.h>
 
 #include "../../include/or_ecycle.h"
 
 namespace {
 
-constexpr int NOALLOC_TILE = 128;
+// 64 hexas per CTA: the largest group is then 512 CTAs, one wave at the 4 CTAs per SM
+// that the element kernel's 210 registers allow; at 128 the 216 CTAs of a 27,648-hexa
+// group left most SMs with one CTA and some with two.
+constexpr int NOALLOC_TILE = 64;
+constexpr int NOALLOC_NODE_TILE = 128;
 
+// The time state and the reduction of a cycle are double-buffered by cycle parity:
+// the node kernel of a cycle derives the time step from the buffers of its parity,
+// every thread for itself, and one thread leaves the next cycle's in the others.
 struct NoallocScalars {
-  unsigned long long dtbits;   // min over elements of the element dt (double bits)
-  unsigned long long dtkey;    // min of (float(dt) bits << 32 | 0x80000000 | element): NELTS
+  unsigned long long dtbits[2];  // min over elements of the element dt (double bits)
+  unsigned long long dtkey[2];   // min of (float(dt) bits << 32 | 0x80000000 | element): NELTS
   int err_code;
   int err_index;
-  double time[8];              // tt, dt1, dt2, dt12, dt2old, ncycle, ityptst, neltst
+  double time[2][8];             // tt, dt1, dt2, dt12, dt2old, ncycle, ityptst, neltst
 };
+
+// Programmatic dependent launch (the protocol of the handle path's kernels): a kernel
+// waits for its predecessor before it reads what the predecessor wrote, and releases its
+// successor only after that wait, so whatever it reads ahead of the wait was written at
+// least two launches back.
+__device__ __forceinline__ void noalloc_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void noalloc_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // the shared scratch: FSKY slots (fx, fy, fz, unused) and the per-call scalars
 static __device__ __align__(256) double4 g_fsky_scratch[OR_NOALLOC_MAX_SLOTS];
@@ -99,20 +114,25 @@ __global__ void check_adsky_kernel(int nel, int numnod, const int* __restrict__ 
 // skyline slots IADS(k, e) given by the caller (FP64 throughout).
 __global__ void __launch_bounds__(NOALLOC_TILE)
 hex_fsky_kernel(int nel, const int* __restrict__ conn, const int* __restrict__ iads,
-                const double* __restrict__ x, const double* __restrict__ v,
+                const double* x, const double* v,
                 double* sig, double* eint, double* rho, double* qvis, double* pla, double* epsd,
                 const double* __restrict__ vol0, or_material mt, or_solid_prop pr, double dtfac,
-                double4* fsky, NoallocScalars* sc) {
+                double4* fsky, NoallocScalars* sc, int parity) {
   const int e = blockIdx.x * NOALLOC_TILE + threadIdx.x;
   __shared__ unsigned long long s_min[NOALLOC_TILE / 32], s_key[NOALLOC_TILE / 32];
   unsigned long long mybits = ~0ull, mykey = ~0ull;
+  int nd[8];
   if (e < nel) {
-    const double DT1 = sc->time[1];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) nd[k] = conn[8 * e + k];
+  }
+  noalloc_wait();        // X, V and the time state come from the previous node pass
+  noalloc_trigger();
+  if (e < nel) {
+    const double DT1 = sc->time[parity][2];     // DT1 = DT2 of the cycle before (resol.F:2639)
     double XD[8], YD[8], ZD[8], VX[8], VY[8], VZ[8];
-    int nd[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      nd[k] = conn[8 * e + k];
       XD[k] = x[3 * nd[k]]; YD[k] = x[3 * nd[k] + 1]; ZD[k] = x[3 * nd[k] + 2];
       VX[k] = v[3 * nd[k]]; VY[k] = v[3 * nd[k] + 1]; VZ[k] = v[3 * nd[k] + 2];
     }
@@ -335,61 +355,87 @@ hex_fsky_kernel(int nel, const int* __restrict__ conn, const int* __restrict__ i
       m = s_min[w] < m ? s_min[w] : m;
       q = s_key[w] < q ? s_key[w] : q;
     }
-    atomicMin(&sc->dtbits, m);
-    atomicMin(&sc->dtkey, q);
+    atomicMin(&sc->dtbits[parity], m);
+    atomicMin(&sc->dtkey[parity], q);
   }
 }
 
-// dt logic (resol.F:5853-6226) by one thread, then ASSPAR4 + ACCELE + BCS10 +
-// VELOCITY + DEPLA per node.  The dt state is advanced by the last block to finish.
-__global__ void dt_kernel(NoallocScalars* sc, double growth, double dtmx) {
-  double* t = sc->time;   // tt, dt1, dt2, dt12, dt2old, ncycle
-  const double dt2t = __longlong_as_double((long long)sc->dtbits);
+// dt logic (resol.F:5853-6226), the same in every thread, then ASSPAR4 + ACCELE + BCS10 +
+// VELOCITY + DEPLA per node.  A cycle is latency-bound at the sizes the scratch holds, so
+// it is two launches (elements, nodes), each released ahead of its predecessor's end: a call
+// of 50 cycles at 27,648 hexas took 1476 us with single-thread launches for the time step and
+// the cycle's start between them, 1085 us so.  A node's slots are loaded four at a time.
+__global__ void __launch_bounds__(NOALLOC_NODE_TILE)
+node_fsky_kernel(int numnod, int nslot, const int* __restrict__ adsky, const double4* fsky, double* x, double* d,
+                 double* v, const double* __restrict__ ms, const int* __restrict__ icodt, double growth, double dtmx,
+                 NoallocScalars* sc, int parity) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = n < numnod;
+  int k0 = 0, k1 = 0, c = 0;
+  double m = 0, vx = 0, vy = 0, vz = 0, px = 0, py = 0, pz = 0, qx = 0, qy = 0, qz = 0;
+  if (valid) {
+    k0 = max(adsky[n], 0); k1 = min(adsky[n + 1], nslot);   // within the scratch
+    m = ms[n]; c = icodt[n];
+    vx = v[3 * n]; vy = v[3 * n + 1]; vz = v[3 * n + 2];
+    px = x[3 * n]; py = x[3 * n + 1]; pz = x[3 * n + 2];
+    qx = d[3 * n]; qy = d[3 * n + 1]; qz = d[3 * n + 2];
+  }
+  double t[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) t[i] = sc->time[parity][i];
+  noalloc_wait();        // the slots and the reduction come from the element pass
+  noalloc_trigger();
+  const unsigned long long bits = sc->dtbits[parity], key = sc->dtkey[parity];
+  const double dt2t = __longlong_as_double((long long)bits);
   double DT2 = 1e6;
-  if (sc->dtbits != ~0ull && dt2t < DT2) {   // the element that set DT2 (ITYPTS = 1, NELTS)
+  if (bits != ~0ull && dt2t < DT2) {   // the element that set DT2 (ITYPTS = 1, NELTS)
     DT2 = dt2t;
     t[6] = 1.0;
-    t[7] = (double)(int)(sc->dtkey & 0x7fffffffull);
+    t[7] = (double)(int)(key & 0x7fffffffull);
   }
   DT2 = fmin(fmin(DT2, growth * t[4]), dtmx);
-  t[3] = 0.5 * (t[1] + DT2);
-  t[2] = DT2;
-  t[4] = DT2;
-  t[0] += DT2;
-  t[5] += 1.0;
-  sc->dtbits = ~0ull;
-  sc->dtkey = ~0ull;
-}
-
-__global__ void node_fsky_kernel(int numnod, int nslot, const int* __restrict__ adsky,
-                                 const double4* __restrict__ fsky, double* x, double* d, double* v,
-                                 const double* __restrict__ ms, const int* __restrict__ icodt, NoallocScalars* sc) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= numnod) return;
-  double ax = 0, ay = 0, az = 0;
-  const int k0 = max(adsky[n], 0), k1 = min(adsky[n + 1], nslot);   // within the scratch
-  for (int k = k0; k < k1; ++k) {
-    const double4 f = fsky[k];
-    ax += f.x; ay += f.y; az += f.z;
+  const double DT1 = t[2], DT12 = 0.5 * (DT1 + DT2);
+  if (n == 0) {
+    double* u = sc->time[1 - parity];
+    u[0] = t[0] + DT2; u[1] = DT1; u[2] = DT2; u[3] = DT12; u[4] = DT2; u[5] = t[5] + 1.0; u[6] = t[6]; u[7] = t[7];
+    sc->dtbits[1 - parity] = ~0ull;
+    sc->dtkey[1 - parity] = ~0ull;
   }
-  const double m = ms[n];
+  if (!valid) return;
+  double ax = 0, ay = 0, az = 0;
+  for (int k = k0; k < k1; k += 4) {
+    double4 f[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) f[i] = k + i < k1 ? fsky[k + i] : make_double4(0, 0, 0, 0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (k + i < k1) { ax += f[i].x; ay += f[i].y; az += f[i].z; }
+  }
   if (m > 0.0) { const double r = 1.0 / m; ax *= r; ay *= r; az *= r; } else { ax = ay = az = 0.0; }
   if (!isfinite(ax + ay + az)) noalloc_error(sc, OR_E_NAN, n);
-  double vx = v[3 * n], vy = v[3 * n + 1], vz = v[3 * n + 2];
-  const int c = icodt[n];
   if (c & 4) { vx = 0; ax = 0; }
   if (c & 2) { vy = 0; ay = 0; }
   if (c & 1) { vz = 0; az = 0; }
-  const double dt12 = sc->time[3], dt2 = sc->time[2];
-  vx += dt12 * ax; vy += dt12 * ay; vz += dt12 * az;
+  vx += DT12 * ax; vy += DT12 * ay; vz += DT12 * az;
   v[3 * n] = vx; v[3 * n + 1] = vy; v[3 * n + 2] = vz;
-  const double ux = dt2 * vx, uy = dt2 * vy, uz = dt2 * vz;
-  d[3 * n] += ux; d[3 * n + 1] += uy; d[3 * n + 2] += uz;
-  x[3 * n] += ux; x[3 * n + 1] += uy; x[3 * n + 2] += uz;
+  const double ux = DT2 * vx, uy = DT2 * vy, uz = DT2 * vz;
+  d[3 * n] = qx + ux; d[3 * n + 1] = qy + uy; d[3 * n + 2] = qz + uz;
+  x[3 * n] = px + ux; x[3 * n + 1] = py + uy; x[3 * n + 2] = pz + uz;
 }
 
-__global__ void start_cycle_kernel(NoallocScalars* sc) {
-  sc->time[1] = sc->time[2];   // DT1 = DT2 (resol.F:2639)
+// one of the cycle's two kernels, released ahead of its predecessor's end
+template <class... P, class... A>
+cudaError_t launch_ahead(void (*k)(P...), unsigned grid, unsigned block, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, k, std::forward<A>(args)...);
 }
 
 // Bounded wait for the call's own work, as the handle path's wait_stream.
@@ -454,13 +500,13 @@ extern "C" int or_ecycle_hex_step_noalloc(int device, void* stream, int ncycles,
   const int nslot = 8 * nel;
   // clear what must start at zero / +inf, load the caller's time state
   NoallocScalars init;
-  init.dtbits = ~0ull;
-  init.dtkey = ~0ull;
+  init.dtbits[0] = init.dtbits[1] = ~0ull;
+  init.dtkey[0] = init.dtkey[1] = ~0ull;
   init.err_code = 0;
   init.err_index = -1;
-  init.time[0] = t->tt; init.time[1] = t->dt1; init.time[2] = t->dt2; init.time[3] = t->dt12;
-  init.time[4] = t->dt2old; init.time[5] = (double)t->ncycle; init.time[6] = (double)t->ityptst;
-  init.time[7] = (double)t->neltst;
+  const double now[8] = {t->tt, t->dt1, t->dt2, t->dt12, t->dt2old, (double)t->ncycle, (double)t->ityptst,
+                         (double)t->neltst};
+  for (int i = 0; i < 8; ++i) init.time[0][i] = init.time[1][i] = now[i];
   if (cudaMemcpyAsync(p.sc, &init, sizeof init, cudaMemcpyHostToDevice, s) != cudaSuccess) return OR_E_CUDA;
   // check the caller's tables before anything is written (slot counters in the scratch)
   NoallocScalars out;
@@ -475,20 +521,20 @@ extern "C" int or_ecycle_hex_step_noalloc(int device, void* stream, int ncycles,
     if (out.err_code) { t->neltst = out.err_index; return out.err_code; }
   }
   const unsigned eb = (unsigned)((nel + NOALLOC_TILE - 1) / NOALLOC_TILE);
-  const unsigned nb = (unsigned)((numnod + 255) / 256);
+  const unsigned nb = (unsigned)((numnod + NOALLOC_NODE_TILE - 1) / NOALLOC_NODE_TILE);
   for (int c = 0; c < ncycles; ++c) {
-    start_cycle_kernel<<<1, 1, 0, s>>>(p.sc);
-    hex_fsky_kernel<<<eb, NOALLOC_TILE, 0, s>>>(nel, conn, iads, x, v, sig, eint, rho, qvis, pla, epsd, vol0, *mat,
-                                                 *prop, dtfac, p.fsky, p.sc);
-    dt_kernel<<<1, 1, 0, s>>>(p.sc, dt_growth, dtmx);
-    node_fsky_kernel<<<nb, 256, 0, s>>>(numnod, nslot, adsky, p.fsky, x, d, v, ms, icodt, p.sc);
+    if (launch_ahead(hex_fsky_kernel, eb, NOALLOC_TILE, s, nel, conn, iads, (const double*)x, (const double*)v, sig,
+                     eint, rho, qvis, pla, epsd, vol0, *mat, *prop, dtfac, p.fsky, p.sc, c & 1) != cudaSuccess ||
+        launch_ahead(node_fsky_kernel, nb, NOALLOC_NODE_TILE, s, numnod, nslot, adsky, (const double4*)p.fsky, x, d, v,
+                     ms, icodt, dt_growth, dtmx, p.sc, c & 1) != cudaSuccess)
+      return OR_E_CUDA;
   }
   if (cudaGetLastError() != cudaSuccess) return OR_E_CUDA;
   const int rc = read_scalars(s, p.sc, &out);
   if (rc) return rc;
-  t->tt = out.time[0]; t->dt1 = out.time[1]; t->dt2 = out.time[2]; t->dt12 = out.time[3];
-  t->dt2old = out.time[4]; t->ncycle = (int)out.time[5];
-  t->ityptst = (int)out.time[6]; t->neltst = (int)out.time[7];
+  const double* e = out.time[ncycles & 1];
+  t->tt = e[0]; t->dt1 = e[1]; t->dt2 = e[2]; t->dt12 = e[3]; t->dt2old = e[4]; t->ncycle = (int)e[5];
+  t->ityptst = (int)e[6]; t->neltst = (int)e[7];
   if (out.err_code) t->neltst = out.err_index;
   return out.err_code;
 }

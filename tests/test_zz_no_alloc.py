@@ -217,3 +217,22 @@ def test_noalloc_rejects_oversized_group():
            dummy, dummy, dummy, C.byref(mat), C.byref(prop), C.c_double(0.9), C.c_double(1e20), C.c_double(1.1),
            dummy, dummy, dummy, dummy, dummy, dummy, dummy)
     assert rc == abi.OR_E_ARG
+
+
+@pytest.mark.parametrize("nx,ny,nz,n", [(1, 3, 21, 1), (4, 4, 4, 2), (5, 13, 1, 7)])
+def test_noalloc_small_groups_and_cycle_parities(nx, ny, nz, n):
+    """One hexa below, at and one above a CTA's 64 hexas, over odd and even numbers of
+    cycles: the time state's two buffers end a call at either parity."""
+    from oracle.oracle import Oracle
+    f = entry()
+    d = decks.c1_hex_block(nx=nx, ny=ny, nz=nz, law=decks.LAW_JOHNSON_COOK, vz=-10.0)
+    a = Arrays(d)
+    o = Oracle(d, nthreads=1)
+    for k in (n, n + 1):
+        assert a.call(f, k) == 0
+        o.step(k)
+        assert rel(a.D.cpu().numpy(), o.get_nodes()["d"]) < FP64_TOL
+        assert rel(a.V.cpu().numpy(), o.get_nodes()["v"]) < FP64_TOL
+        t = o.time()
+        assert a.t.ncycle == t["ncycle"]
+        assert abs(a.t.dt1 - t["dt1"]) <= FP64_TOL * t["dt2"] and abs(a.t.tt - t["tt"]) <= FP64_TOL * t["tt"]
