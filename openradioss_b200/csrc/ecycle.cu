@@ -507,12 +507,12 @@ cudaError_t launch_k(void (*k)(P...), unsigned grid, unsigned block, size_t smem
 }
 
 template <class R, int T>
-int launch_hex(or_ecycle* h, Impl<R>& m, int parity, bool pdl = false) {
+int launch_hex(or_ecycle* h, Impl<R>& m, int parity, bool pdl = false, int second = 0) {
   if (m.hps.info.empty()) return OR_OK;
   size_t sm = hex_smem<R>(m.hps.nlmax, T, m.hinc_stride);
   const unsigned g = (unsigned)m.hps.info.size();
-  if (m.any_corot) CK(launch_k(hex_patch_kernel<R, T, 1>, g, T, sm, h->stream, pdl, m.hargs(), parity));
-  else CK(launch_k(hex_patch_kernel<R, T, 0>, g, T, sm, h->stream, pdl, m.hargs(), parity));
+  if (m.any_corot) CK(launch_k(hex_patch_kernel<R, T, 1>, g, T, sm, h->stream, pdl, m.hargs(), parity, second));
+  else CK(launch_k(hex_patch_kernel<R, T, 0>, g, T, sm, h->stream, pdl, m.hargs(), parity, second));
   h->launches++;
   return OR_OK;
 }
@@ -593,27 +593,33 @@ cudaError_t set_smem(F* f, int bytes) {
   return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
+// Dynamic shared memory that the patch kernels may be launched with.  The attribute is
+// the process's and not a handle's, so every handle sets the same value: a later, smaller
+// model must not lower what an earlier handle launches with.
+constexpr int MAX_DYN_SMEM = 200 * 1024;
+
 template <class R>
 int set_smem_attrs(or_ecycle* h, Impl<R>& m) {
-  int hs = (int)hex_smem<R>(m.hps.nlmax, h->tile_hex, m.hinc_stride);
-  int ss = (int)shell_smem<R>(m.sps.nlmax, h->tile_shell, m.sinc_stride, 5);   // the largest: the 5-point kernels
-  if (hs > 200 * 1024 || ss > 200 * 1024) return fail(h, OR_E_UNSUPPORTED, "patch shared memory above 200 KB");
-  CK(set_smem(hex_patch_kernel<R, 64, 0>, hs));
-  CK(set_smem(hex_patch_kernel<R, 128, 0>, hs));
-  CK(set_smem(hex_patch_kernel<R, 256, 0>, hs));
-  CK(set_smem(hex_patch_kernel<R, 64, 1>, hs));
-  CK(set_smem(hex_patch_kernel<R, 128, 1>, hs));
-  CK(set_smem(hex_patch_kernel<R, 256, 1>, hs));
-  CK(set_smem(shell_patch_kernel<R, 64, 0, false>, ss));
-  CK(set_smem(shell_patch_kernel<R, 128, 0, false>, ss));
-  CK(set_smem(shell_patch_kernel<R, 256, 0, false>, ss));
-  CK(set_smem(shell_patch_kernel<R, 64, 5, false>, ss));
-  CK(set_smem(shell_patch_kernel<R, 128, 5, false>, ss));
-  CK(set_smem(shell_patch_kernel<R, 256, 5, false>, ss));
+  const size_t hs = hex_smem<R>(m.hps.nlmax, h->tile_hex, m.hinc_stride);
+  const size_t ss = shell_smem<R>(m.sps.nlmax, h->tile_shell, m.sinc_stride, 5);   // the largest: the 5-point kernels
+  if (hs > MAX_DYN_SMEM || ss > MAX_DYN_SMEM) return fail(h, OR_E_UNSUPPORTED, "patch shared memory above 200 KB");
+  auto set = [](auto* f) { return set_smem(f, MAX_DYN_SMEM); };
+  CK(set(hex_patch_kernel<R, 64, 0>));
+  CK(set(hex_patch_kernel<R, 128, 0>));
+  CK(set(hex_patch_kernel<R, 256, 0>));
+  CK(set(hex_patch_kernel<R, 64, 1>));
+  CK(set(hex_patch_kernel<R, 128, 1>));
+  CK(set(hex_patch_kernel<R, 256, 1>));
+  CK(set(shell_patch_kernel<R, 64, 0, false>));
+  CK(set(shell_patch_kernel<R, 128, 0, false>));
+  CK(set(shell_patch_kernel<R, 256, 0, false>));
+  CK(set(shell_patch_kernel<R, 64, 5, false>));
+  CK(set(shell_patch_kernel<R, 128, 5, false>));
+  CK(set(shell_patch_kernel<R, 256, 5, false>));
   if constexpr (sizeof(R) == 4) {
-    CK(set_smem(shell_patch_kernel<R, 64, 5, true>, ss));
-    CK(set_smem(shell_patch_kernel<R, 128, 5, true>, ss));
-    CK(set_smem(shell_patch_kernel<R, 256, 5, true>, ss));
+    CK(set(shell_patch_kernel<R, 64, 5, true>));
+    CK(set(shell_patch_kernel<R, 128, 5, true>));
+    CK(set(shell_patch_kernel<R, 256, 5, true>));
   }
   return OR_OK;
 }
@@ -697,12 +703,12 @@ int persist_build(or_ecycle* h, Impl<R>& m) {
     }
   }
   const size_t smem = persist_smem<R>(ncmax, tile, P, m.sinc_stride, ps.nlmax);
-  if (smem > 200 * 1024) return OR_OK;
+  if (smem > MAX_DYN_SMEM) return OR_OK;
   // one thread per element, and per held node where the CTA holds more nodes than
   // elements (a node phase of one node per thread), in whole TILE groups
   const int T = std::min(PERSIST_THREADS / tile * tile, std::max(P * tile, (ncmax + tile - 1) / tile * tile));
   const PersistFn<R> fn = persist_fn<R>(tile, m.uniform_npt == 5);
-  CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_DYN_SMEM));
   int nb = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, T, smem));
   if (nb < 1 || G > nb * h->nsm) return OR_OK;
@@ -753,15 +759,26 @@ int launch_cycle(or_ecycle* h, Impl<R>& m, int parity, cudaEvent_t* ev) {
   const bool pdl = h->pdl && !ev;
   Trace tr(parity ? "cycle (odd)" : "cycle (even)");
   if ((rc = launch_loads<R>(h, m, parity))) return rc;     // FORCE (resol.F:2847), before the elements
-  rc = h->tile_hex == 64 ? launch_hex<R, 64>(h, m, parity, pdl)
-       : h->tile_hex == 128 ? launch_hex<R, 128>(h, m, parity, pdl) : launch_hex<R, 256>(h, m, parity, pdl);
-  if (rc) return rc;
-  if (ev) CK(cudaEventRecord(ev[1], h->stream));
-  rc = h->tile_shell == 64 ? launch_shell_npt<R, 64>(h, m, parity, pdl)
-       : h->tile_shell == 128 ? launch_shell_npt<R, 128>(h, m, parity, pdl)
-                              : launch_shell_npt<R, 256>(h, m, parity, pdl);
-  if (rc) return rc;
-  if (ev) CK(cudaEventRecord(ev[2], h->stream));
+  auto hexas = [&](int second) {
+    return h->tile_hex == 64 ? launch_hex<R, 64>(h, m, parity, pdl, second)
+           : h->tile_hex == 128 ? launch_hex<R, 128>(h, m, parity, pdl, second)
+                                : launch_hex<R, 256>(h, m, parity, pdl, second);
+  };
+  auto shells = [&]() {
+    return h->tile_shell == 64 ? launch_shell_npt<R, 64>(h, m, parity, pdl)
+           : h->tile_shell == 128 ? launch_shell_npt<R, 128>(h, m, parity, pdl)
+                                  : launch_shell_npt<R, 256>(h, m, parity, pdl);
+  };
+  if (pdl) {
+    // The shells first, the hexas beside them: a skin's shells are about one wave whose
+    // time is one element's chain, and hexas fill the SMs meanwhile.
+    if ((rc = shells()) || (rc = hexas(m.sps.info.empty() ? 0 : 1))) return rc;
+  } else {
+    if ((rc = hexas(0))) return rc;
+    if (ev) CK(cudaEventRecord(ev[1], h->stream));
+    if ((rc = shells())) return rc;
+    if (ev) CK(cudaEventRecord(ev[2], h->stream));
+  }
   rc = launch_link<R>(h, m);
   if (rc) return rc;
   rc = launch_rbody<R>(h, m, parity);

@@ -240,6 +240,12 @@ __host__ __device__ inline size_t halo_buffer_bytes(int nhalo) {
 //  - then pdl_trigger(), so the next kernel may start its own prologue.
 // Because each kernel triggers only after its wait, the grid two kernels back has
 // completed whenever a kernel starts: its prologue may read that grid's output.
+//
+// A mesh of hexas and shells has two element passes in a cycle, which depend on the
+// node pass before them but not on one another.  The second (SECOND below) does not
+// wait at its start: it starts once every CTA of the first has seen the node pass
+// complete, so it may read what the node pass wrote.  It waits at its end, so that
+// its own completion, on which the next node pass waits, includes the first's.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -470,7 +476,7 @@ __host__ __device__ inline size_t hex_smem_bytes(int nl, int tile, int inc_strid
 // run time); CORO = 0 compiles that path out (the register budget of the default)
 template <class R, int TILE, int CORO>
 __global__ void __launch_bounds__(TILE, min_blocks(Occupancy<R>::hex, TILE))
-hex_patch_kernel(HexArgs<R> a, int parity) {
+hex_patch_kernel(HexArgs<R> a, int parity, int second) {
   typedef typename Vec4<R>::T R4;
   constexpr bool split = sizeof(R) == 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -525,7 +531,7 @@ hex_patch_kernel(HexArgs<R> a, int parity) {
   if (tid == 0) { pre_ehour = a.blk_ehour[p]; pre_wpla = a.blk_wpla[p]; }
   // X, V and the cycle's time come from the previous node pass: gathered after the
   // wait, straight into shared memory
-  pdl_wait();
+  if (!second) pdl_wait();
   pdl_trigger();
   for (int j = tid; j < NLM; j += TILE) {
     const int g = a.patch_nodes[p * NLM + j];
@@ -979,6 +985,7 @@ hex_patch_kernel(HexArgs<R> a, int parity) {
       a.blk_wpla[p] = pre_wpla + w;
     }
   }
+  if (second) pdl_wait();
 }
 
 
