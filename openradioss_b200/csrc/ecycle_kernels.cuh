@@ -2105,6 +2105,34 @@ node_io_kernel(int kind, int to_device, double* __restrict__ stage, int n, int s
   }
 }
 
+// Up to four nodal arrays of a part at once, in the caller's layout, written straight to
+// mapped host memory (null: not wanted).  A CTA passes each array through shared memory,
+// so that a warp's stores to the host are 256 consecutive bytes.
+constexpr int NODES_OUT_TILE = 128;
+template <class R>
+__global__ void __launch_bounds__(NODES_OUT_TILE)
+nodes_out_kernel(double* x, double* d, double* v, double* vr, int n, int s, const double4* __restrict__ X,
+                 const double* __restrict__ DX, const double* __restrict__ DY, const double* __restrict__ DZ,
+                 const typename Vec4<R>::T* __restrict__ V, const typename Vec4<R>::T* __restrict__ VR) {
+  __shared__ double row[4][3 * NODES_OUT_TILE];
+  const int i0 = blockIdx.x * NODES_OUT_TILE, t = threadIdx.x, g = s + i0 + t;
+  const int count = n - i0 < NODES_OUT_TILE ? n - i0 : NODES_OUT_TILE;
+  if (t < count) {
+    if (x) { const double4 q = X[g]; row[0][3 * t] = q.x; row[0][3 * t + 1] = q.y; row[0][3 * t + 2] = q.z; }
+    if (d) { row[1][3 * t] = DX[g]; row[1][3 * t + 1] = DY[g]; row[1][3 * t + 2] = DZ[g]; }
+    if (v) { const typename Vec4<R>::T q = V[g]; row[2][3 * t] = q.x; row[2][3 * t + 1] = q.y; row[2][3 * t + 2] = q.z; }
+    if (vr) { const typename Vec4<R>::T q = VR[g]; row[3][3 * t] = q.x; row[3][3 * t + 1] = q.y; row[3][3 * t + 2] = q.z; }
+  }
+  __syncthreads();
+  double* const out[4] = {x, d, v, vr};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (!out[k]) continue;
+    double* q = out[k] + 3 * (size_t)i0;
+    for (int j = t; j < 3 * count; j += NODES_OUT_TILE) q[j] = row[k][j];
+  }
+}
+
 // ===========================================================================
 // rigid links (RLINK1, rlink1.F): per link (one block), MASS = sum MS and
 // AX = sum MS*A over its nodes after ACCELE and BCS10 (the node kernel's
