@@ -168,10 +168,8 @@ struct AdjShellArgs {
 };
 
 // Threads per CTA and resident CTAs per SM of the reverse shell kernel (its
-// register budget: 65536 / (threads x CTAs) per thread).  64 x 5 (204 registers)
-// puts a 40,000-shell plate in one wave of 148 SMs, where 128 x 2 at 255
-// registers left a 6 % tail wave: the C5 adjoint 92-93 -> 88.4 ms on B200
-// (96 x 3: 88.6 ms); the gradients are bitwise the same.
+// register budget: 65536 / (threads x CTAs) per thread).  64 x 5 holds a 40,000-shell plate in one wave of 148 SMs; ten warps
+// share four schedulers, so the compiler's budget is 168 registers.
 #ifndef ORB_ADJ_SHELL_THREADS
 #define ORB_ADJ_SHELL_THREADS 64
 #endif
@@ -180,66 +178,102 @@ struct AdjShellArgs {
 #endif
 constexpr int ADJ_SHELL_THREADS = ORB_ADJ_SHELL_THREADS;
 
-template <int NP>
+// The points of element e, read and written in place in the component-major arrays
+struct AdjPointIO {
+  const AdjShellArgs& a;
+  int e;
+  __device__ __forceinline__ void sig(int ip, double* S) const {
+#pragma unroll
+    for (int c = 0; c < 5; ++c) S[c] = a.sig[(ip * 5 + c) * a.nelpad + e];
+  }
+  __device__ __forceinline__ double pla(int ip) const { return a.pla[ip * a.nelpad + e]; }
+  __device__ __forceinline__ void put_sig(int, const double*) const {}
+  __device__ __forceinline__ void put_pla(int, double) const {}
+  __device__ __forceinline__ void bsig(int ip, double* S) const {
+#pragma unroll
+    for (int c = 0; c < 5; ++c) S[c] = a.lsig[(ip * 5 + c) * a.nelpad + e];
+  }
+  __device__ __forceinline__ double bpla(int ip) const { return a.lpla[ip * a.nelpad + e]; }
+  __device__ __forceinline__ void put_bsig(int ip, const double* S) const {
+#pragma unroll
+    for (int c = 0; c < 5; ++c) a.lsig[(ip * 5 + c) * a.nelpad + e] = S[c];
+  }
+  __device__ __forceinline__ void put_bpla(int ip, double p) const { a.lpla[ip * a.nelpad + e] = p; }
+  // volatile, so that the compiler reads the nodes again instead of keeping (and spilling)
+  // what the forward read
+  __device__ __forceinline__ static void again(const double4* q, double* o) {
+    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(o[0]), "=d"(o[1]) : "l"(q));
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(o[2]) : "l"(reinterpret_cast<const double*>(q) + 2));
+  }
+  __device__ __forceinline__ int node(int k) const {
+    int n;
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(n) : "l"(reinterpret_cast<const int*>(a.enodes + e) + k));
+    return n;
+  }
+  template <class In> __device__ __forceinline__ void velocity(const In&, int k, double* v, double* vr) const {
+    const int n = node(k);
+    again(a.Vn + n, v);
+    again(a.VRn + n, vr);
+  }
+  template <class In> __device__ __forceinline__ void coordinates(const In&, double (*x)[3]) const {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) again(a.Xn + node(k), x[k]);
+  }
+};
+
+// One thread per element.  The integration points stream from global memory, once in the
+// recomputed forward and once in the reverse, and no array is indexed by point: with the
+// points' state, adjoints and tape in arrays the kernel moved 11.3 KB per element through
+// local memory.  With the node reads repeated where the reverse needs them again, 100 cycles
+// of the 200x200 plate's adjoint took 16.2 ms against 19.1 (B200).
 __global__ void __launch_bounds__(ADJ_SHELL_THREADS, ORB_ADJ_SHELL_CTAS) adj_shell_kernel(AdjShellArgs a) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= a.nelpad) return;
   const int gi = a.egroup[e];
   if (gi < 0) return;
-  const AdjGroup G = a.groups[gi];
+  const AdjGroup& G = a.groups[gi];
   orb_adj::ShellParams P = G.P;
   P.degen = a.degen[e];
-  const int npt = P.npt < NP ? P.npt : NP;
   const int nelpad = a.nelpad;
   const int4 nd = a.enodes[e];
   const int node[4] = {nd.x, nd.y, nd.z, nd.w};
-  orb_adj::ShellIn<NP> in;
-  orb_adj::ShellOut<NP> ob;
+  orb_adj::ShellIn<1> in, ib;
+  orb_adj::ShellOut<1> ob, out;
+#pragma unroll
   for (int k = 0; k < 4; ++k) {
     const double4 x = a.Xn[node[k]], v = a.Vn[node[k]], r = a.VRn[node[k]];
     in.x[k][0] = x.x; in.x[k][1] = x.y; in.x[k][2] = x.z;
     in.v[k][0] = v.x; in.v[k][1] = v.y; in.v[k][2] = v.z;
     in.vr[k][0] = r.x; in.vr[k][1] = r.y; in.vr[k][2] = r.z;
-    const double4 f = a.lamF[node[k]], m = a.lamM[node[k]];
-    ob.f[k][0] = f.x; ob.f[k][1] = f.y; ob.f[k][2] = f.z;
-    ob.m[k][0] = m.x; ob.m[k][1] = m.y; ob.m[k][2] = m.z;
-  }
-  for (int ip = 0; ip < NP; ++ip) {
-    for (int c = 0; c < 5; ++c) {
-      in.sig[ip][c] = ip < npt ? a.sig[(ip * 5 + c) * nelpad + e] : 0.0;
-      ob.sig[ip][c] = ip < npt ? a.lsig[(ip * 5 + c) * nelpad + e] : 0.0;
-    }
-    in.pla[ip] = ip < npt ? a.pla[ip * nelpad + e] : 0.0;
-    ob.pla[ip] = ip < npt ? a.lpla[ip * nelpad + e] : 0.0;
   }
   in.thk = a.thk[e];
   in.thke = a.thke[e];
+#pragma unroll
   for (int q = 0; q < 3; ++q) { in.hourg[q] = a.hourg[q * nelpad + e]; ob.hourg[q] = a.lhourg[q * nelpad + e]; }
   in.ca = G.has_jca ? a.jca[e] : G.jc_a;
   in.dt1 = a.tcur[G.part].dt2;
   ob.thk = a.lthk[e];
   ob.wpla = a.w_plastic;
-  orb_adj::ShellTape<NP> t;
-  orb_adj::ShellOut<NP> out;
-  orb_adj::shell_forward<NP>(P, a.zw, in, out, t);
-  orb_adj::ShellIn<NP> ib;
-  for (int k = 0; k < 4; ++k)
+  orb_adj::ShellTape<1> t;
+  AdjPointIO io{a, e};
+  orb_adj::shell_forward_io(P, a.zw, in, out, t, io);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int n = io.node(k);
+    io.again(a.lamF + n, ob.f[k]);
+    io.again(a.lamM + n, ob.m[k]);
+#pragma unroll
     for (int c = 0; c < 3; ++c) { ib.x[k][c] = 0.0; ib.v[k][c] = 0.0; ib.vr[k][c] = 0.0; }
-  for (int ip = 0; ip < NP; ++ip) {
-    for (int c = 0; c < 5; ++c) ib.sig[ip][c] = 0.0;
-    ib.pla[ip] = 0.0;
   }
   ib.thk = ib.thke = ib.ca = ib.dt1 = 0.0;
   ib.hourg[0] = ib.hourg[1] = ib.hourg[2] = 0.0;
-  orb_adj::shell_reverse<NP>(P, a.zw, in, t, ob, ib);
-  for (int ip = 0; ip < npt; ++ip) {
-    for (int c = 0; c < 5; ++c) a.lsig[(ip * 5 + c) * nelpad + e] = ib.sig[ip][c];
-    a.lpla[ip * nelpad + e] = ib.pla[ip];
-  }
+  orb_adj::shell_reverse_io(P, a.zw, in, t, ob, ib, io);
   a.lthk[e] = ib.thk;
+#pragma unroll
   for (int q = 0; q < 3; ++q) a.lhourg[q * nelpad + e] = ib.hourg[q];
   a.dA[e] += ib.ca;
   a.dthke[e] += ib.thke;
+#pragma unroll
   for (int k = 0; k < 4; ++k) {
     a.cX[4 * e + k] = make_double4(ib.x[k][0], ib.x[k][1], ib.x[k][2], 0.0);
     a.cV[4 * e + k] = make_double4(ib.v[k][0], ib.v[k][1], ib.v[k][2], 0.0);

@@ -1932,9 +1932,8 @@ double adj_plastic_work(or_ecycle* h) {
   return s;
 }
 
-template <int NP>
 int launch_adj_shell(or_ecycle* h, const AdjShellArgs& a) {
-  adj_shell_kernel<NP><<<(unsigned)((a.nelpad + ADJ_SHELL_THREADS - 1) / ADJ_SHELL_THREADS), ADJ_SHELL_THREADS, 0,
+  adj_shell_kernel<<<(unsigned)((a.nelpad + ADJ_SHELL_THREADS - 1) / ADJ_SHELL_THREADS), ADJ_SHELL_THREADS, 0,
                          h->stream>>>(a);
   CK(cudaGetLastError());
   h->launches++;
@@ -2041,8 +2040,7 @@ int adjoint_impl(or_ecycle* h, int N, const or_adjoint_response* r, or_ecycle_ti
       sa.lsig = w.lsig.p; sa.lpla = w.lpla.p; sa.lthk = w.lthk.p; sa.lhourg = w.lhourg.p; sa.dA = w.dA.p;
       sa.dthke = w.dthke.p; sa.cX = w.cX.p; sa.cV = w.cV.p; sa.cR = w.cR.p; sa.zw = m.zw.p;
       sa.w_plastic = r->w_plastic; sa.nelpad = nelpad;
-      rc = m.uniform_npt == 5 ? launch_adj_shell<5>(h, sa) : launch_adj_shell<10>(h, sa);
-      if (rc) return rc;
+      if ((rc = launch_adj_shell(h, sa))) return rc;
       AdjPostArgs pa;
       pa.ofs = w.csr_ofs.p; pa.ent = w.csr_ent.p; pa.cX = w.cX.p; pa.cV = w.cV.p; pa.cR = w.cR.p;
       pa.lamX = w.lamX.p; pa.lamV = w.lamV.p; pa.lamVR = w.lamVR.p; pa.nnodpad = nn;

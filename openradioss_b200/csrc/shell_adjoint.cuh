@@ -54,6 +54,10 @@ struct ShellOut {
   double thk, hourg[3], wpla;
 };
 
+// The tape holds nothing per integration point: the reverse forms each point's forward
+// again (shell_point) from its old stress and plastic strain, which it asks the caller
+// for point by point.  A kernel then keeps no array that it indexes by point, which would
+// lie in local memory.
 template <int NP>
 struct ShellTape {
   double d21[3], d31[3], d41[3], d32[3], d34[3];
@@ -66,9 +70,6 @@ struct ShellTape {
   double VZ13, VZ24, t2a, t1a, t1b, t2b, t3a, t3b, VX13, VX24, VY13, VY24;
   double RX13, RX24, RXAV, RY13, RY24, RYAV;
   double Er[8], E[8], FAC1;   // EXX EYY EXY EYZ EXZ KXX KYY KXY, raw and scaled by DT1/AREA
-  double ZT[NP], THKLYL[NP], DXX[NP], DYY[NP], DXY[NP], ST[NP][3], SVM[NP], YLD[NP], RR[NP];
-  double DPLA[NP], EZZp[NP], EZZ[NP], SN[NP][5];
-  int plastic[NP], yclamp[NP], dpla_pos[NP];
   double FOR[5], MOM[3], THKN;
   double px1v, px2v, py1v, py2v, GAMA[4], T2A, H1Q, H2Q, H3Q, TD, HH1, HH2, B12;
   double A1c, A3c, A5c, A7c, A8c;
@@ -103,11 +104,65 @@ ORB_HD void v_normalize_rev(const double n[3], double nu, const double nb[3], do
 }
 
 // ---------------------------------------------------------------------------
-// forward
+// one integration point, MULAWC's layer (mulawc.F90:596-1100, 2603-2620)
 // ---------------------------------------------------------------------------
-template <int NP>
-ORB_HD void shell_forward(const ShellParams& P, const float* zw, const ShellIn<NP>& in, ShellOut<NP>& out,
-                          ShellTape<NP>& t) {
+struct ShellPoint {
+  double THKLYL, ZT, ST[3], SN[5], SVM, YLD, RR, DPLA, EZZp, EZZ, PLA;
+  bool plastic, yclamp, dpla_pos;
+};
+template <class Tape>
+ORB_HD void shell_point(const ShellParams& P, const Tape& t, const double CA, const double z0, const double wf,
+                        const double SO[5], const double PLA0, ShellPoint& q) {
+  const double NU = P.nu, GG = P.shear, YM = P.young;
+  q.THKLYL = wf * t.THK0;
+  q.ZT = z0 * t.THK0;
+  const double DXX = t.E[0] + q.ZT * t.E[5], DYY = t.E[1] + q.ZT * t.E[6], DXY = t.E[2] + q.ZT * t.E[7];
+  q.plastic = q.yclamp = q.dpla_pos = false;
+  q.DPLA = 0.0; q.EZZp = 0.0; q.SVM = 0.0; q.YLD = 0.0; q.RR = 1.0; q.PLA = PLA0;
+  if (P.law == 1) {
+    // SIGEPS01C (sigeps01c.F:130-146)
+    q.SN[0] = SO[0] + P.a11 * DXX + P.a12 * DYY;
+    q.SN[1] = SO[1] + P.a12 * DXX + P.a11 * DYY;
+    q.SN[2] = SO[2] + GG * DXY;
+    q.SN[3] = SO[3] + t.GS * t.E[3];
+    q.SN[4] = SO[4] + t.GS * t.E[4];
+    q.ST[0] = q.SN[0]; q.ST[1] = q.SN[1]; q.ST[2] = q.SN[2];
+    q.EZZ = -NU * (DXX + DYY) / (1.0 - NU);
+    return;
+  }
+  // SIGEPS02C -> M2CPLR, IPLA = 0 (m2cplr.F:96-230)
+  const double A1 = YM / (1.0 - NU * NU), A2 = A1 * NU;
+  q.SN[0] = SO[0] + A1 * DXX + A2 * DYY;
+  q.SN[1] = SO[1] + A2 * DXX + A1 * DYY;
+  q.SN[2] = SO[2] + GG * DXY;
+  q.SN[3] = SO[3] + t.GS * t.E[3];
+  q.SN[4] = SO[4] + t.GS * t.E[4];
+  q.ST[0] = q.SN[0]; q.ST[1] = q.SN[1]; q.ST[2] = q.SN[2];
+  double YLD = PLA0 == 0.0 ? CA : CA + P.jc_b * exp(P.jc_n * log(PLA0));
+  q.yclamp = YLD > P.sigmax;
+  YLD = fmin(YLD, P.sigmax);
+  const double SVM = sqrt(q.SN[0] * q.SN[0] + q.SN[1] * q.SN[1] - q.SN[0] * q.SN[1] + 3.0 * q.SN[2] * q.SN[2]);
+  const double RR = fmin(1.0, YLD / (SVM + A_EM15));
+  if (RR < 1.0) {
+    q.plastic = true;
+    q.SN[0] *= RR; q.SN[1] *= RR; q.SN[2] *= RR;
+    const double d = (SVM - YLD) / YM;
+    q.dpla_pos = d > 0.0;
+    q.DPLA = fmax(0.0, d);
+    q.EZZp = q.DPLA * (0.5 * (q.SN[0] + q.SN[1])) / YLD;
+    q.PLA = PLA0 + q.DPLA;
+  }
+  double EZZ = -(DXX + DYY) * NU - (1.0 - 2.0 * NU) * q.EZZp;   // sigeps02c.F:215-224
+  q.EZZ = EZZ / (1.0 - NU);
+  q.SVM = SVM; q.YLD = YLD; q.RR = RR;
+}
+
+// ---------------------------------------------------------------------------
+// forward.  io: old state of point ip by io.sig(ip, SO) and io.pla(ip), new state to
+// io.put_sig(ip, SN), io.put_pla(ip, PLA)
+// ---------------------------------------------------------------------------
+template <class In, class Out, class Tape, class IO>
+ORB_HD void shell_forward_io(const ShellParams& P, const float* zw, const In& in, Out& out, Tape& t, IO& io) {
   const double DT1 = in.dt1;
   for (int c = 0; c < 3; ++c) {
     t.d21[c] = in.x[1][c] - in.x[0][c];
@@ -169,10 +224,10 @@ ORB_HD void shell_forward(const ShellParams& P, const float* zw, const ShellIn<N
   // CCOEF3 (ccoef3.F:66-160)
   t.THK0 = P.ithk > 0 ? in.thk : in.thke;
   t.THK02 = t.THK0 * t.THK0;
-  const double NU = P.nu, GG = P.shear, YM = P.young;
+  const double NU = P.nu, YM = P.young;
   const int npt = P.npt;
   const double SHF = npt == 1 ? 0.0 : P.shf;
-  t.GS = GG * SHF;
+  t.GS = P.shear * SHF;
   // CDEFO3, IHBE <= 1 (cdefo3.F:84-131)
   for (int k = 0; k < 4; ++k) {
     t.VXl[k] = v_dot(t.e1n, in.v[k]);
@@ -214,7 +269,6 @@ ORB_HD void shell_forward(const ShellParams& P, const float* zw, const ShellIn<N
   // CSTRA3 (cstra3.F:91-101)
   t.FAC1 = DT1 / t.AREA;
   for (int i = 0; i < 8; ++i) t.E[i] = t.Er[i] * t.FAC1;
-  EXX = t.E[0]; EYY = t.E[1]; EXY = t.E[2]; EYZ = t.E[3]; EXZ = t.E[4]; KXX = t.E[5]; KYY = t.E[6]; KXY = t.E[7];
   // MULAWC layer loop (mulawc.F90:596-1100, 2603-2620)
   const float* Z0 = zw + (npt - 1) * 33;
   const float* WF = Z0 + 11;
@@ -222,61 +276,19 @@ ORB_HD void shell_forward(const ShellParams& P, const float* zw, const ShellIn<N
   for (int c = 0; c < 5; ++c) t.FOR[c] = 0.0;
   for (int c = 0; c < 3; ++c) t.MOM[c] = 0.0;
   t.THKN = in.thk;
-  const double CA = in.ca, CB = P.jc_b, CN = P.jc_n, YMAX = P.sigmax;
   double wpla = 0.0;
-  for (int ip = 0; ip < npt && ip < NP; ++ip) {
+  for (int ip = 0; ip < npt; ++ip) {
     const double wf = (double)WF[ip], wm = (double)WM[ip];
-    const double* SO = in.sig[ip];
-    double* SN = t.SN[ip];
-    t.THKLYL[ip] = wf * t.THK0;
-    t.ZT[ip] = (double)Z0[ip] * t.THK0;
-    const double DXX = EXX + t.ZT[ip] * KXX, DYY = EYY + t.ZT[ip] * KYY, DXY = EXY + t.ZT[ip] * KXY;
-    t.DXX[ip] = DXX; t.DYY[ip] = DYY; t.DXY[ip] = DXY;
-    double EZZ = 0.0, PLA = in.pla[ip];
-    t.plastic[ip] = 0; t.yclamp[ip] = 0; t.dpla_pos[ip] = 0;
-    t.DPLA[ip] = 0.0; t.EZZp[ip] = 0.0; t.SVM[ip] = 0.0; t.YLD[ip] = 0.0; t.RR[ip] = 1.0;
-    if (P.law == 1) {
-      // SIGEPS01C (sigeps01c.F:130-146)
-      SN[0] = SO[0] + P.a11 * DXX + P.a12 * DYY;
-      SN[1] = SO[1] + P.a12 * DXX + P.a11 * DYY;
-      SN[2] = SO[2] + GG * DXY;
-      SN[3] = SO[3] + t.GS * EYZ;
-      SN[4] = SO[4] + t.GS * EXZ;
-      EZZ = -NU * (DXX + DYY) / (1.0 - NU);
-    } else {
-      // SIGEPS02C -> M2CPLR, IPLA = 0 (m2cplr.F:96-230)
-      const double A1 = YM / (1.0 - NU * NU), A2 = A1 * NU;
-      SN[0] = SO[0] + A1 * DXX + A2 * DYY;
-      SN[1] = SO[1] + A2 * DXX + A1 * DYY;
-      SN[2] = SO[2] + GG * DXY;
-      SN[3] = SO[3] + t.GS * EYZ;
-      SN[4] = SO[4] + t.GS * EXZ;
-      t.ST[ip][0] = SN[0]; t.ST[ip][1] = SN[1]; t.ST[ip][2] = SN[2];
-      double YLD = PLA == 0.0 ? CA : CA + CB * exp(CN * log(PLA));
-      t.yclamp[ip] = YLD > YMAX;
-      YLD = fmin(YLD, YMAX);
-      const double SVM = sqrt(SN[0] * SN[0] + SN[1] * SN[1] - SN[0] * SN[1] + 3.0 * SN[2] * SN[2]);
-      const double RR = fmin(1.0, YLD / (SVM + A_EM15));
-      double DPLA = 0.0, EZZp = 0.0;
-      if (RR < 1.0) {
-        t.plastic[ip] = 1;
-        SN[0] *= RR; SN[1] *= RR; SN[2] *= RR;
-        const double q = (SVM - YLD) / YM;
-        t.dpla_pos[ip] = q > 0.0;
-        DPLA = fmax(0.0, q);
-        EZZp = DPLA * (0.5 * (SN[0] + SN[1])) / YLD;
-        PLA = PLA + DPLA;
-      }
-      EZZ = -(DXX + DYY) * NU - (1.0 - 2.0 * NU) * EZZp;   // sigeps02c.F:215-224
-      EZZ = EZZ / (1.0 - NU);
-      wpla += YLD * DPLA * t.AREA * t.THKLYL[ip];
-      t.SVM[ip] = SVM; t.YLD[ip] = YLD; t.RR[ip] = RR; t.DPLA[ip] = DPLA; t.EZZp[ip] = EZZp;
-    }
-    t.EZZ[ip] = EZZ;
-    t.THKN = t.THKN + EZZ * t.THKLYL[ip];
-    for (int c = 0; c < 5; ++c) { out.sig[ip][c] = SN[c]; t.FOR[c] = t.FOR[c] + wf * SN[c]; }
-    for (int c = 0; c < 3; ++c) t.MOM[c] = t.MOM[c] + wm * SN[c];
-    out.pla[ip] = PLA;
+    double SO[5];
+    io.sig(ip, SO);
+    ShellPoint q;
+    shell_point(P, t, in.ca, (double)Z0[ip], wf, SO, io.pla(ip), q);
+    wpla += q.YLD * q.DPLA * t.AREA * q.THKLYL;
+    t.THKN = t.THKN + q.EZZ * q.THKLYL;
+    for (int c = 0; c < 5; ++c) t.FOR[c] = t.FOR[c] + wf * q.SN[c];
+    for (int c = 0; c < 3; ++c) t.MOM[c] = t.MOM[c] + wm * q.SN[c];
+    io.put_sig(ip, q.SN);
+    io.put_pla(ip, q.PLA);
   }
   out.wpla = wpla;
   out.thk = t.THKN > A_EM30 ? t.THKN : A_EM30;
@@ -356,11 +368,15 @@ ORB_HD void shell_forward(const ShellParams& P, const float* zw, const ShellIn<N
 }
 
 // ---------------------------------------------------------------------------
-// reverse: ob = adjoints of the outputs, ib = adjoints of the inputs (accumulated)
+// reverse: ob = adjoints of the outputs, ib = adjoints of the inputs (accumulated).  io:
+// old state of point ip by io.sig, io.pla; adjoints of its new state by io.bsig(ip, bS),
+// io.bpla(ip); adjoints of its old state to io.put_bsig(ip, bS), io.put_bpla(ip, b).  The
+// corner velocities and coordinates come from io again near the end, where they are next
+// needed: 36 values and the differences formed from them are not held across the layers.
 // ---------------------------------------------------------------------------
-template <int NP>
-ORB_HD void shell_reverse(const ShellParams& P, const float* zw, const ShellIn<NP>& in, const ShellTape<NP>& t,
-                          const ShellOut<NP>& ob, ShellIn<NP>& ib) {
+template <class In, class Out, class Tape, class IO>
+ORB_HD void shell_reverse_io(const ShellParams& P, const float* zw, const In& in, const Tape& t, const Out& ob, In& ib,
+                             IO& io) {
   const double DT1 = in.dt1;
   const double NU = P.nu, GG = P.shear, YM = P.young;
   const int npt = P.npt;
@@ -515,51 +531,49 @@ ORB_HD void shell_reverse(const ShellParams& P, const float* zw, const ShellIn<N
     const float* WM = Z0 + 22;
     const double CB = P.jc_b, CN = P.jc_n;
     const double bwpla = ob.wpla;
-    for (int ip = 0; ip < npt && ip < NP; ++ip) {
+    for (int ip = 0; ip < npt; ++ip) {
       const double wf = (double)WF[ip], wm = (double)WM[ip];
-      double bSN[5];
-      for (int c = 0; c < 5; ++c) bSN[c] = ob.sig[ip][c] + wf * bFOR[c];
+      double bSN[5], SO[5];
+      io.sig(ip, SO);
+      const double PLA0 = io.pla(ip), bPLAo = io.bpla(ip);
+      io.bsig(ip, bSN);
+      ShellPoint q;
+      shell_point(P, t, in.ca, (double)Z0[ip], wf, SO, PLA0, q);
+      for (int c = 0; c < 5; ++c) bSN[c] += wf * bFOR[c];
       for (int c = 0; c < 3; ++c) bSN[c] += wm * bMOM[c];
-      double bEZZ = bTHKN * t.THKLYL[ip];
-      double bTHKLYL = bTHKN * t.EZZ[ip];
-      double bDXX = 0, bDYY = 0, bDXY = 0;
+      const double bEZZ = bTHKN * q.THKLYL;
+      double bTHKLYL = bTHKN * q.EZZ;
+      double bDXX = 0, bDYY = 0, bDXY = 0, bPLA = bPLAo;
+      double bST[3] = {bSN[0], bSN[1], bSN[2]};
+      bDXX += -NU / (1.0 - NU) * bEZZ; bDYY += -NU / (1.0 - NU) * bEZZ;
       if (P.law == 1) {
-        bDXX += -NU / (1.0 - NU) * bEZZ; bDYY += -NU / (1.0 - NU) * bEZZ;
-        for (int c = 0; c < 5; ++c) ib.sig[ip][c] += bSN[c];
         bDXX += P.a11 * bSN[0] + P.a12 * bSN[1];
         bDYY += P.a12 * bSN[0] + P.a11 * bSN[1];
         bDXY += GG * bSN[2];
-        bE[3] += t.GS * bSN[3];
-        bE[4] += t.GS * bSN[4];
-        ib.pla[ip] += ob.pla[ip];
       } else {
         const double A1 = YM / (1.0 - NU * NU), A2 = A1 * NU;
-        const double YLD = t.YLD[ip], DPLA = t.DPLA[ip], SVM = t.SVM[ip], RR = t.RR[ip];
+        const double YLD = q.YLD, DPLA = q.DPLA, SVM = q.SVM, RR = q.RR;
         // wpla += YLD*DPLA*AREA*THKLYL
-        double bYLD = bwpla * DPLA * t.AREA * t.THKLYL[ip];
-        double bDPLA = bwpla * YLD * t.AREA * t.THKLYL[ip];
-        bAREA += bwpla * YLD * DPLA * t.THKLYL[ip];
+        double bYLD = bwpla * DPLA * t.AREA * q.THKLYL;
+        double bDPLA = bwpla * YLD * t.AREA * q.THKLYL;
+        bAREA += bwpla * YLD * DPLA * q.THKLYL;
         bTHKLYL += bwpla * YLD * DPLA * t.AREA;
         // EZZ = (-(DXX+DYY)*NU - (1-2NU)*EZZp) / (1-NU)
-        bDXX += -NU / (1.0 - NU) * bEZZ; bDYY += -NU / (1.0 - NU) * bEZZ;
         const double bEZZp = -(1.0 - 2.0 * NU) / (1.0 - NU) * bEZZ;
         // PLA_out = PLA_in + DPLA
-        ib.pla[ip] += ob.pla[ip];
-        double bST[3] = {bSN[0], bSN[1], bSN[2]};
-        if (t.plastic[ip]) {
-          bDPLA += ob.pla[ip];
+        if (q.plastic) {
+          bDPLA += bPLAo;
           // EZZp = DPLA*0.5*(SN0+SN1)/YLD, SN scaled
-          const double SN0 = t.SN[ip][0], SN1 = t.SN[ip][1];
-          bDPLA += bEZZp * 0.5 * (SN0 + SN1) / YLD;
+          bDPLA += bEZZp * 0.5 * (q.SN[0] + q.SN[1]) / YLD;
           const double bs01 = bEZZp * DPLA * 0.5 / YLD;
           double bSNs[3] = {bSN[0] + bs01, bSN[1] + bs01, bSN[2]};
-          bYLD += -bEZZp * t.EZZp[ip] / YLD;
+          bYLD += -bEZZp * q.EZZp / YLD;
           // DPLA = max(0, (SVM - YLD)/YM)
           double bSVM = 0.0;
-          if (t.dpla_pos[ip]) { bSVM += bDPLA / YM; bYLD -= bDPLA / YM; }
+          if (q.dpla_pos) { bSVM += bDPLA / YM; bYLD -= bDPLA / YM; }
           // SN[i] = RR*ST[i], i < 3
           double bRR = 0.0;
-          for (int i = 0; i < 3; ++i) { bRR += bSNs[i] * t.ST[ip][i]; bST[i] = bSNs[i] * RR; }
+          for (int i = 0; i < 3; ++i) { bRR += bSNs[i] * q.ST[i]; bST[i] = bSNs[i] * RR; }
           // RR = YLD/(SVM + EM15)
           const double den = SVM + A_EM15;
           bYLD += bRR / den;
@@ -567,32 +581,30 @@ ORB_HD void shell_reverse(const ShellParams& P, const float* zw, const ShellIn<N
           // SVM = sqrt(S0^2 + S1^2 - S0 S1 + 3 S2^2) of the trial stress
           if (SVM > 0.0) {
             const double bQ = bSVM / (2.0 * SVM);
-            const double S0 = t.ST[ip][0], S1 = t.ST[ip][1], S2 = t.ST[ip][2];
-            bST[0] += bQ * (2.0 * S0 - S1);
-            bST[1] += bQ * (2.0 * S1 - S0);
-            bST[2] += bQ * 6.0 * S2;
+            bST[0] += bQ * (2.0 * q.ST[0] - q.ST[1]);
+            bST[1] += bQ * (2.0 * q.ST[1] - q.ST[0]);
+            bST[2] += bQ * 6.0 * q.ST[2];
           }
         }
         // YLD = min(CA + CB*PLA^CN, YMAX), CA when PLA == 0
-        if (!t.yclamp[ip]) {
+        if (!q.yclamp) {
           ib.ca += bYLD;
-          const double PLA = in.pla[ip];
-          if (PLA > 0.0) ib.pla[ip] += bYLD * CB * CN * exp((CN - 1.0) * log(PLA));
+          if (PLA0 > 0.0) bPLA += bYLD * CB * CN * exp((CN - 1.0) * log(PLA0));
         }
         // trial stress
-        for (int c = 0; c < 3; ++c) ib.sig[ip][c] += bST[c];
-        ib.sig[ip][3] += bSN[3];
-        ib.sig[ip][4] += bSN[4];
         bDXX += A1 * bST[0] + A2 * bST[1];
         bDYY += A2 * bST[0] + A1 * bST[1];
         bDXY += GG * bST[2];
-        bE[3] += t.GS * bSN[3];
-        bE[4] += t.GS * bSN[4];
       }
+      bE[3] += t.GS * bSN[3];
+      bE[4] += t.GS * bSN[4];
+      bSN[0] = bST[0]; bSN[1] = bST[1]; bSN[2] = bST[2];
+      io.put_bsig(ip, bSN);
+      io.put_bpla(ip, bPLA);
       // DXX = EXX + ZT*KXX ...
-      bE[0] += bDXX; bE[5] += t.ZT[ip] * bDXX;
-      bE[1] += bDYY; bE[6] += t.ZT[ip] * bDYY;
-      bE[2] += bDXY; bE[7] += t.ZT[ip] * bDXY;
+      bE[0] += bDXX; bE[5] += q.ZT * bDXX;
+      bE[1] += bDYY; bE[6] += q.ZT * bDYY;
+      bE[2] += bDXY; bE[7] += q.ZT * bDXY;
       const double bZT = bDXX * t.E[5] + bDYY * t.E[6] + bDXY * t.E[7];
       bTHK0 += (double)Z0[ip] * bZT + wf * bTHKLYL;
     }
@@ -656,14 +668,17 @@ ORB_HD void shell_reverse(const ShellParams& P, const float* zw, const ShellIn<N
     bVZl[0] += bVZ13; bVZl[2] -= bVZ13; bVZl[1] += bVZ24; bVZl[3] -= bVZ24;
   }
   // local velocities: VXl = e1n.v, VYl = e2n.v, VZl = e3n.v, RXl = e1n.vr, RYl = e2n.vr
-  for (int k = 0; k < 4; ++k)
+  for (int k = 0; k < 4; ++k) {
+    double v[3], vr[3];
+    io.velocity(in, k, v, vr);
     for (int c = 0; c < 3; ++c) {
-      be1n[c] += bVXl[k] * in.v[k][c] + bRXl[k] * in.vr[k][c];
-      be2n[c] += bVYl[k] * in.v[k][c] + bRYl[k] * in.vr[k][c];
-      be3n[c] += bVZl[k] * in.v[k][c];
+      be1n[c] += bVXl[k] * v[c] + bRXl[k] * vr[c];
+      be2n[c] += bVYl[k] * v[c] + bRYl[k] * vr[c];
+      be3n[c] += bVZl[k] * v[c];
       ib.v[k][c] += bVXl[k] * t.e1n[c] + bVYl[k] * t.e2n[c] + bVZl[k] * t.e3n[c];
       ib.vr[k][c] += bRXl[k] * t.e1n[c] + bRYl[k] * t.e2n[c];
     }
+  }
   // ---- CCOEF3: THK0, THK02 ----
   bTHK0 += 2.0 * t.THK0 * bTHK02;
   if (P.ithk > 0) ib.thk += bTHK0; else ib.thke += bTHK0;
@@ -683,9 +698,14 @@ ORB_HD void shell_reverse(const ShellParams& P, const float* zw, const ShellIn<N
   bY3 += 0.5 * bPX2;
   bX3 -= 0.5 * bPY2;
   double bd21[3], bd31[3], bd41[3], bd32[3] = {0, 0, 0}, bd34[3] = {0, 0, 0};
+  double x[4][3], e1[3], e2[3];
+  io.coordinates(in, x);
   for (int c = 0; c < 3; ++c) {
-    be1n[c] += bX2 * t.d21[c] + bX3 * t.d31[c] + bX4 * t.d41[c];
-    be2n[c] += bY2 * t.d21[c] + bY3 * t.d31[c] + bY4 * t.d41[c];
+    const double d21 = x[1][c] - x[0][c], d31 = x[2][c] - x[0][c], d41 = x[3][c] - x[0][c];
+    e1[c] = d21 + (x[2][c] - x[3][c]);
+    e2[c] = (x[2][c] - x[1][c]) + d41;
+    be1n[c] += bX2 * d21 + bX3 * d31 + bX4 * d41;
+    be2n[c] += bY2 * d21 + bY3 * d31 + bY4 * d41;
     bd21[c] = bX2 * t.e1n[c] + bY2 * t.e2n[c];
     bd31[c] = bX3 * t.e1n[c] + bY3 * t.e2n[c];
     bd41[c] = bX4 * t.e1n[c] + bY4 * t.e2n[c];
@@ -703,11 +723,11 @@ ORB_HD void shell_reverse(const ShellParams& P, const float* zw, const ShellIn<N
     // e1p = q2 e1 + e2 x e3 ; q2 = |e2|^2
     double be1[3], be2[3] = {0, 0, 0};
     for (int c = 0; c < 3; ++c) be1[c] = be1p[c] * t.q2;
-    const double bq2 = v_dot(be1p, t.e1);
-    v_cross_rev(t.e2, t.e3, be1p, be2, be3);
-    for (int c = 0; c < 3; ++c) be2[c] += 2.0 * bq2 * t.e2[c];
+    const double bq2 = v_dot(be1p, e1);
+    v_cross_rev(e2, t.e3, be1p, be2, be3);
+    for (int c = 0; c < 3; ++c) be2[c] += 2.0 * bq2 * e2[c];
     // e3 = e1 x e2
-    v_cross_rev(t.e1, t.e2, be3, be1, be2);
+    v_cross_rev(e1, e2, be3, be1, be2);
     for (int c = 0; c < 3; ++c) {
       bd21[c] += be1[c]; bd34[c] += be1[c];
       bd32[c] += be2[c]; bd41[c] += be2[c];
@@ -722,17 +742,17 @@ ORB_HD void shell_reverse(const ShellParams& P, const float* zw, const ShellIn<N
     double be1[3] = {be1p[0], be1p[1], be1p[2]}, be2[3] = {0, 0, 0};
     const double bs = v_dot(be1p, t.c23);
     const double bc23[3] = {be1p[0] * t.s, be1p[1] * t.s, be1p[2] * t.s};
-    v_cross_rev(t.e2, t.e3n, bc23, be2, be3n);
+    v_cross_rev(e2, t.e3n, bc23, be2, be3n);
     // s = sqrt(q1/q2)
     if (t.s > 0.0) {
       const double bq1 = bs / (2.0 * t.s * t.q2);
       const double bq2 = -bs * t.q1 / (2.0 * t.s * t.q2 * t.q2);
-      for (int c = 0; c < 3; ++c) { be1[c] += 2.0 * bq1 * t.e1[c]; be2[c] += 2.0 * bq2 * t.e2[c]; }
+      for (int c = 0; c < 3; ++c) { be1[c] += 2.0 * bq1 * e1[c]; be2[c] += 2.0 * bq2 * e2[c]; }
     }
     // e3n = e3 / |e3| ; e3 = e1 x e2
     double be3[3] = {0, 0, 0};
     v_normalize_rev(t.e3n, t.n3, be3n, be3);
-    v_cross_rev(t.e1, t.e2, be3, be1, be2);
+    v_cross_rev(e1, e2, be3, be1, be2);
     // e1 = d21 + d34 ; e2 = d32 + d41
     for (int c = 0; c < 3; ++c) {
       bd21[c] += be1[c]; bd34[c] += be1[c];
@@ -746,6 +766,43 @@ ORB_HD void shell_reverse(const ShellParams& P, const float* zw, const ShellIn<N
     ib.x[2][c] += bd32[c]; ib.x[1][c] -= bd32[c];
     ib.x[2][c] += bd34[c]; ib.x[3][c] -= bd34[c];
   }
+}
+
+// ---------------------------------------------------------------------------
+// the same over whole arrays (ShellIn, ShellOut): adjoints accumulate in ib
+// ---------------------------------------------------------------------------
+template <int NP>
+struct ShellArrays {
+  const ShellIn<NP>& in;
+  ShellOut<NP>* out;
+  const ShellOut<NP>* ob;
+  ShellIn<NP>* ib;
+  ORB_HD void sig(int ip, double* S) const { for (int c = 0; c < 5; ++c) S[c] = in.sig[ip][c]; }
+  ORB_HD double pla(int ip) const { return in.pla[ip]; }
+  ORB_HD void put_sig(int ip, const double* S) const { for (int c = 0; c < 5; ++c) out->sig[ip][c] = S[c]; }
+  ORB_HD void put_pla(int ip, double p) const { out->pla[ip] = p; }
+  ORB_HD void bsig(int ip, double* S) const { for (int c = 0; c < 5; ++c) S[c] = ob->sig[ip][c]; }
+  ORB_HD double bpla(int ip) const { return ob->pla[ip]; }
+  ORB_HD void put_bsig(int ip, const double* S) const { for (int c = 0; c < 5; ++c) ib->sig[ip][c] += S[c]; }
+  ORB_HD void put_bpla(int ip, double p) const { ib->pla[ip] += p; }
+  ORB_HD void velocity(const ShellIn<NP>& s, int k, double* v, double* vr) const {
+    for (int c = 0; c < 3; ++c) { v[c] = s.v[k][c]; vr[c] = s.vr[k][c]; }
+  }
+  ORB_HD void coordinates(const ShellIn<NP>& s, double (*x)[3]) const {
+    for (int k = 0; k < 4; ++k) for (int c = 0; c < 3; ++c) x[k][c] = s.x[k][c];
+  }
+};
+template <int NP>
+ORB_HD void shell_forward(const ShellParams& P, const float* zw, const ShellIn<NP>& in, ShellOut<NP>& out,
+                          ShellTape<NP>& t) {
+  ShellArrays<NP> io{in, &out, nullptr, nullptr};
+  shell_forward_io(P, zw, in, out, t, io);
+}
+template <int NP>
+ORB_HD void shell_reverse(const ShellParams& P, const float* zw, const ShellIn<NP>& in, const ShellTape<NP>& t,
+                          const ShellOut<NP>& ob, ShellIn<NP>& ib) {
+  ShellArrays<NP> io{in, nullptr, &ob, &ib};
+  shell_reverse_io(P, zw, in, t, ob, ib, io);
 }
 
 }  // namespace orb_adj
