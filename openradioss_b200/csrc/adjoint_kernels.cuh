@@ -16,6 +16,10 @@
 //
 // No float atomics: every sum has a fixed order, so the gradient is bitwise
 // reproducible.
+//
+// The three run under the cycle kernels' programmatic launch protocol (pdl_wait, then
+// pdl_trigger): each starts while its predecessor ends, and adj_shell_kernel forms the
+// element forward, which needs the stored state only, ahead of its wait.
 #pragma once
 #include "ecycle_kernels.cuh"
 #include "shell_adjoint.cuh"
@@ -72,7 +76,40 @@ __device__ inline void adj_bcs_skew(int lcod, const double* sk, double b[3]) {
   }
 }
 
+// State fields copied by one launch, to or from one buffer: a chunk of ADJ_CHUNK bytes per
+// CTA, field after field.  A cycle's start state is seven arrays; copied one by one they
+// took longer to launch than to move.
+constexpr int ADJ_FIELDS = 16, ADJ_CHUNK = 256 * 4 * 16;
+struct AdjCopy {
+  const unsigned char* src[ADJ_FIELDS];
+  unsigned char* dst[ADJ_FIELDS];
+  unsigned long long bytes[ADJ_FIELDS];   // multiples of 8
+  int chunk0[ADJ_FIELDS + 1];             // first chunk of each field
+  int n;
+};
+__global__ void __launch_bounds__(256) adj_copy_kernel(const __grid_constant__ AdjCopy a) {
+  int f = 0;
+  while (f + 1 < a.n && (int)blockIdx.x >= a.chunk0[f + 1]) ++f;
+  const unsigned long long o = (unsigned long long)(blockIdx.x - a.chunk0[f]) * ADJ_CHUNK;
+  const unsigned long long end = a.bytes[f];
+  uint4 v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const unsigned long long q = o + (threadIdx.x + 256 * i) * 16ull;
+    if (q + 16 <= end) v[i] = *reinterpret_cast<const uint4*>(a.src[f] + q);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const unsigned long long q = o + (threadIdx.x + 256 * i) * 16ull;
+    if (q + 16 <= end) *reinterpret_cast<uint4*>(a.dst[f] + q) = v[i];
+    else if (q < end) *reinterpret_cast<unsigned long long*>(a.dst[f] + q) =
+                          *reinterpret_cast<const unsigned long long*>(a.src[f] + q);
+  }
+}
+
 __global__ void __launch_bounds__(128) adj_node_pre_kernel(AdjNodeArgs a) {
+  pdl_wait();
+  pdl_trigger();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= a.nnodpad) return;
   const int part = a.tile_part[n / a.node_tile];
@@ -228,9 +265,12 @@ struct AdjPointIO {
 // of the 200x200 plate's adjoint took 16.2 ms against 19.1 (B200).
 __global__ void __launch_bounds__(ADJ_SHELL_THREADS, ORB_ADJ_SHELL_CTAS) adj_shell_kernel(AdjShellArgs a) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= a.nelpad) return;
-  const int gi = a.egroup[e];
-  if (gi < 0) return;
+  const int gi = e < a.nelpad ? a.egroup[e] : -1;
+  if (gi < 0) {
+    pdl_wait();
+    pdl_trigger();
+    return;
+  }
   const AdjGroup& G = a.groups[gi];
   orb_adj::ShellParams P = G.P;
   P.degen = a.degen[e];
@@ -249,14 +289,18 @@ __global__ void __launch_bounds__(ADJ_SHELL_THREADS, ORB_ADJ_SHELL_CTAS) adj_she
   in.thk = a.thk[e];
   in.thke = a.thke[e];
 #pragma unroll
-  for (int q = 0; q < 3; ++q) { in.hourg[q] = a.hourg[q * nelpad + e]; ob.hourg[q] = a.lhourg[q * nelpad + e]; }
+  for (int q = 0; q < 3; ++q) in.hourg[q] = a.hourg[q * nelpad + e];
   in.ca = G.has_jca ? a.jca[e] : G.jc_a;
   in.dt1 = a.tcur[G.part].dt2;
-  ob.thk = a.lthk[e];
-  ob.wpla = a.w_plastic;
   orb_adj::ShellTape<1> t;
   AdjPointIO io{a, e};
   orb_adj::shell_forward_io(P, a.zw, in, out, t, io);
+  pdl_wait();       // lamF, lamM of the node kernel before
+  pdl_trigger();
+#pragma unroll
+  for (int q = 0; q < 3; ++q) ob.hourg[q] = a.lhourg[q * nelpad + e];
+  ob.thk = a.lthk[e];
+  ob.wpla = a.w_plastic;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int n = io.node(k);
@@ -295,8 +339,9 @@ struct AdjPostArgs {
 
 __global__ void __launch_bounds__(128) adj_node_post_kernel(AdjPostArgs a) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= a.nnodpad) return;
-  const int k0 = a.ofs[n], k1 = a.ofs[n + 1];
+  const int k0 = n < a.nnodpad ? a.ofs[n] : 0, k1 = n < a.nnodpad ? a.ofs[n + 1] : 0;
+  pdl_wait();
+  pdl_trigger();
   if (k1 == k0) return;
   double4 x = a.lamX[n], v = a.lamV[n], r = a.lamVR[n];
   for (int k = k0; k < k1; ++k) {

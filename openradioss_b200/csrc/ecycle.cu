@@ -130,6 +130,7 @@ struct or_ecycle {
   int nsm = 148;                      // multiprocessors of the device
   long long graph_launches = 0;       // kernel launches in one replay of graph_exec
   cudaEvent_t done_ev = nullptr;      // end of the work a call queued (wait_queued)
+  void* tlog = nullptr;               // adjoint forward sweep: where the cycle's time state is logged
   bool late = false;                  // a bounded wait expired: the work may still be running
 };
 
@@ -453,6 +454,7 @@ struct Impl {
     a.rb_role = nrb ? rb_role.p : nullptr;
     a.rotmask = any_rot ? rotmask.p : nullptr;
     a.rot_sparse = rot_sparse;
+    a.tlog = (PartTime*)h->tlog;
     return a;
   }
   void free_all() {
@@ -1806,15 +1808,28 @@ size_t layout_fields(std::vector<AdjField>& f) {
   return off;
 }
 
-int adj_save(or_ecycle* h, const std::vector<AdjField>& f, unsigned char* buf) {
-  for (const auto& x : f)
-    if (x.bytes) CK(cudaMemcpyAsync(buf + x.off, x.p, x.bytes, cudaMemcpyDeviceToDevice, h->stream));
+// The fields to (save) or from the buffer, by one kernel
+int adj_copy(or_ecycle* h, const std::vector<AdjField>& f, unsigned char* buf, bool save) {
+  AdjCopy a{};
+  int chunks = 0;
+  for (const auto& x : f) {
+    if (!x.bytes) continue;
+    if (a.n == ADJ_FIELDS || x.bytes % 8) return fail(h, OR_E_STATE, "adjoint: state fields");
+    a.src[a.n] = save ? (const unsigned char*)x.p : buf + x.off;
+    a.dst[a.n] = save ? buf + x.off : (unsigned char*)x.p;
+    a.bytes[a.n] = x.bytes;
+    a.chunk0[a.n++] = chunks;
+    chunks += (int)((x.bytes + ADJ_CHUNK - 1) / ADJ_CHUNK);
+  }
+  a.chunk0[a.n] = chunks;
+  adj_copy_kernel<<<(unsigned)chunks, 256, 0, h->stream>>>(a);
+  CK(cudaGetLastError());
+  h->launches++;
   return OR_OK;
 }
+int adj_save(or_ecycle* h, const std::vector<AdjField>& f, unsigned char* buf) { return adj_copy(h, f, buf, true); }
 int adj_restore(or_ecycle* h, const std::vector<AdjField>& f, const unsigned char* buf) {
-  for (const auto& x : f)
-    if (x.bytes) CK(cudaMemcpyAsync(x.p, buf + x.off, x.bytes, cudaMemcpyDeviceToDevice, h->stream));
-  return OR_OK;
+  return adj_copy(h, f, const_cast<unsigned char*>(buf), false);
 }
 
 // device tables and buffers of the adjoint, sized for ncycles / checkpoint
@@ -1933,9 +1948,8 @@ double adj_plastic_work(or_ecycle* h) {
 }
 
 int launch_adj_shell(or_ecycle* h, const AdjShellArgs& a) {
-  adj_shell_kernel<<<(unsigned)((a.nelpad + ADJ_SHELL_THREADS - 1) / ADJ_SHELL_THREADS), ADJ_SHELL_THREADS, 0,
-                         h->stream>>>(a);
-  CK(cudaGetLastError());
+  CK(launch_k(adj_shell_kernel, (unsigned)((a.nelpad + ADJ_SHELL_THREADS - 1) / ADJ_SHELL_THREADS), ADJ_SHELL_THREADS,
+              0, h->stream, h->pdl, a));
   h->launches++;
   return OR_OK;
 }
@@ -1965,9 +1979,10 @@ int adjoint_impl(or_ecycle* h, int N, const or_adjoint_response* r, or_ecycle_ti
   CK(cudaMemsetAsync(m.err.p, 0, sizeof(ErrorWord), h->stream));
   for (int c = 0; c < N; ++c) {
     if (c % K == 0 && (rc = adj_save(h, w.full, w.ckpt.p + (size_t)(c / K) * w.full_bytes))) return rc;
-    if ((rc = launch_cycle<double>(h, m, c & 1, nullptr))) return rc;
-    CK(cudaMemcpyAsync(w.tlog.p + (size_t)(c + 1) * np, m.time.p + ((c + 1) & 1) * np, np * sizeof(PartTime),
-                       cudaMemcpyDeviceToDevice, h->stream));
+    h->tlog = w.tlog.p + (size_t)(c + 1) * np;
+    rc = launch_cycle<double>(h, m, c & 1, nullptr);
+    h->tlog = nullptr;
+    if (rc) return rc;
   }
   if ((rc = adj_save(h, w.full, w.fin.p))) return rc;
   if ((rc = adj_check_error(h, m))) return rc;
@@ -2029,8 +2044,7 @@ int adjoint_impl(or_ecycle* h, int N, const or_adjoint_response* r, or_ecycle_ti
       na.lamF = w.lamF.p; na.lamM = w.lamM.p; na.dms = w.dms.p; na.din = w.din.p;
       na.nnodpad = nn; na.node_tile = NODE_TILE;
       na.skew_of = m.skew_of.p; na.skews = m.skw.p;
-      adj_node_pre_kernel<<<nb_node, 128, 0, h->stream>>>(na);
-      CK(cudaGetLastError());
+      CK(launch_k(adj_node_pre_kernel, nb_node, 128, 0, h->stream, h->pdl, na));
       AdjShellArgs sa;
       sa.groups = w.groups.p; sa.egroup = w.egroup.p; sa.enodes = w.enodes.p; sa.degen = m.sdegen.p;
       sa.Xn = na.Xn; sa.Vn = na.Vn; sa.VRn = na.VRn;
@@ -2044,8 +2058,7 @@ int adjoint_impl(or_ecycle* h, int N, const or_adjoint_response* r, or_ecycle_ti
       AdjPostArgs pa;
       pa.ofs = w.csr_ofs.p; pa.ent = w.csr_ent.p; pa.cX = w.cX.p; pa.cV = w.cV.p; pa.cR = w.cR.p;
       pa.lamX = w.lamX.p; pa.lamV = w.lamV.p; pa.lamVR = w.lamVR.p; pa.nnodpad = nn;
-      adj_node_post_kernel<<<nb_node, 128, 0, h->stream>>>(pa);
-      CK(cudaGetLastError());
+      CK(launch_k(adj_node_post_kernel, nb_node, 128, 0, h->stream, h->pdl, pa));
       h->launches += 3;
     }
   }

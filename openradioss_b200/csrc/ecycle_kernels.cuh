@@ -212,6 +212,7 @@ struct NodeArgs {
   // read for every node ahead of the bit, which keeps the latency chain of a
   // one-wave pass short.
   int rot_sparse;
+  PartTime* tlog;             // null, or where the new time state goes too (part by part)
 };
 
 // Whether node n carries rotations in the node pass (NodeArgs::rotmask).
@@ -1974,6 +1975,7 @@ __device__ __forceinline__ void node_pass(NodeArgs<R> a, int parity) {
         t1.tt = t0.tt + DT2; t1.dt2 = DT2; t1.dt2old = DT2; t1.dt1 = DT1; t1.dt12 = DT12;
         t1.ncycle = t0.ncycle + 1; t1.ityptst = ityp; t1.neltst = nelt; t1.pad = 0;
         a.time[(1 - parity) * a.nparts + part] = t1;
+        if (a.tlog) a.tlog[part] = t1;
         PartAcc r; r.dtkey = ~0ull; r.dtbits = ~0ull;
         a.acc[(1 - parity) * a.nparts + part] = r;
       }
