@@ -322,7 +322,7 @@ int  or_ecycle_launch_count(or_ecycle* h, long long* n);
 int  or_ecycle_stream(or_ecycle* h, void** stream);
 /* Bytes of device memory held by the handle. */
 int  or_ecycle_device_bytes(or_ecycle* h, long long* bytes);
-/* Whether or_ecycle_step runs the handle's cycles in the persistent form: one
+/* Whether or_ecycle_step runs a shell mesh's cycles in the persistent form: one
    cooperative launch per call in which each CTA (one per SM) keeps its patches'
    element state in registers and their nodes in shared memory, with one grid
    barrier per cycle.  Chosen at finalize for one part of shell groups with no
@@ -333,6 +333,9 @@ int  or_ecycle_device_bytes(or_ecycle* h, long long* bytes);
    (the library built with -fmad=false); with FMA contraction the compiler may
    fuse a multiply-add in one kernel and not in the other, and the two agree to
    rounding.  ctas, threads: its launch shape (0 when off; either may be NULL).
+   One part of hexa groups that fits likewise runs in a persistent form of its own,
+   under the same conditions and switches; it is not reported here (on = 0), and
+   agrees with the per-phase kernels to rounding.
    No counterpart in the reference. */
 int  or_ecycle_persistent_info(or_ecycle* h, int* on, int* ctas, int* threads);
 

@@ -11,7 +11,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 SRC = [os.path.join(HERE, "csrc", "ecycle.cu"), os.path.join(HERE, "csrc", "ecycle_noalloc.cu")]
 DEPS = SRC + [os.path.join(HERE, "csrc", "ecycle_kernels.cuh"), os.path.join(HERE, "csrc", "persistent_kernel.cuh"),
-              os.path.join(HERE, "csrc", "shell_adjoint.cuh"), os.path.join(HERE, "csrc", "adjoint_kernels.cuh"),
+              os.path.join(HERE, "csrc", "hex_element.cuh"), os.path.join(HERE, "csrc", "shell_adjoint.cuh"), os.path.join(HERE, "csrc", "adjoint_kernels.cuh"),
               os.path.join(HERE, "..", "include", "or_ecycle.h")]
 OUT = os.path.join(HERE, "libor_ecycle.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
@@ -27,7 +27,7 @@ FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std
 # oracle (built with -ffp-contract=off).  Used only by the test that separates the
 # effect of FMA contraction from that of the assembly order.
 OUT_NOFMA = os.path.join(HERE, "libor_ecycle_nofma.so")
-FLAGS_NOFMA = [f for f in FLAGS if f != "--use_fast_math"] + ["-fmad=false"]
+FLAGS_NOFMA = [f for f in FLAGS if f != "--use_fast_math"] + ["-fmad=false", "-DORB_IEEE"]
 
 
 def needs_build(out=OUT):

@@ -388,6 +388,7 @@ struct Impl {
   DBuf<double> sehour, swpla;
   DBuf<float> zw;
   int maxnpt = 1;
+  int same_npt = 0;          // points of every shell group, 0 when they differ
   int uniform_npt = 0;       // 5 when every shell group has 5 points, IHBE 1 and IPLA 0 (the kernels
                              // specialised for that form), else 0 (the general kernels)
   // domain decomposition: halo nodes of this rank's part
@@ -414,7 +415,9 @@ struct Impl {
     int T = 0;                 // threads per CTA
     int stall_cta = -1;        // test hook, OR_ECYCLE_TEST_STALL_CTA
     size_t smem = 0;
-    DBuf<int> node_ofs, node_glob; DBuf<unsigned char> owner; DBuf<uint2> pconn;
+    int nlist = 0;             // words of a CTA's corner lists, at most
+    int npt = 0;               // points whose state stays on the chip (PersistShell), 0: in memory
+    DBuf<int> node_ofs, node_glob, node_nshared, list_ofs, list; DBuf<unsigned char> owner; DBuf<unsigned short> pconn;
     DBuf<R4> fslot2, mslot2; DBuf<PartAcc> acc3; DBuf<double> ek, ekr; DBuf<unsigned> sync;
   } per;
 
@@ -474,11 +477,12 @@ struct Impl {
     dfree(linkd); dfree(link_nodes); dfree(link_of); dfree(link_mean); dfree(stage);
     dfree(rbd); dfree(rb_nodes); dfree(rby); dfree(rb_role); dfree(rb_ek); dfree(rb_ekr);
     dfree(loadd); dfree(funcd); dfree(funcx); dfree(funcy); dfree(wacc); dfree(wpend); dfree(skw); dfree(skew_of);
-    dfree(per.node_ofs); dfree(per.node_glob); dfree(per.owner); dfree(per.pconn); dfree(per.fslot2);
+    dfree(per.node_ofs); dfree(per.node_glob); dfree(per.node_nshared); dfree(per.list_ofs); dfree(per.list); dfree(per.owner); dfree(per.pconn); dfree(per.fslot2);
     dfree(per.mslot2); dfree(per.acc3); dfree(per.ek); dfree(per.ekr); dfree(per.sync);
   }
   PersistArgs pargs() {
     PersistArgs a;
+    a.node_nshared = per.node_nshared.p; a.list_ofs = per.list_ofs.p; a.list = per.list.p; a.nlist = per.nlist;
     a.node_ofs = per.node_ofs.p; a.node_glob = per.node_glob.p; a.owner = per.owner.p; a.pconn = per.pconn.p;
     a.fslot2 = per.fslot2.p; a.mslot2 = per.mslot2.p; a.acc3 = per.acc3.p; a.ek_node = per.ek.p;
     a.ekr_node = per.ekr.p; a.sync = per.sync.p; a.patches_per_cta = per.P; a.ncmax = per.ncmax;
@@ -613,7 +617,7 @@ cudaError_t set_smem(F* f, int bytes) {
 // Dynamic shared memory that the patch kernels may be launched with.  The attribute is
 // the process's and not a handle's, so every handle sets the same value: a later, smaller
 // model must not lower what an earlier handle launches with.
-constexpr int MAX_DYN_SMEM = 200 * 1024;
+constexpr int MAX_DYN_SMEM = 200 * 1024, PERSIST_MAX_SMEM = 224 * 1024;
 
 template <class R>
 int set_smem_attrs(or_ecycle* h, Impl<R>& m) {
@@ -644,19 +648,37 @@ int set_smem_attrs(or_ecycle* h, Impl<R>& m) {
 // ----------------------------------------------------------------------------
 // persistent launch: eligibility, layout, launch
 // ----------------------------------------------------------------------------
+// The kernel of a handle, for a launch of `threads`.  Shells: one for 5 points of Ishell 1
+// with the radial return; for 3 or 5 points of any formulation, their state in registers
+// too; for anything else with the points' state in memory.  22,801 shells of 3 points with
+// the Newton return in FP64 took 16.4 us a cycle from memory, 12.7 so.
+template <class R, int TILE, int MAXT>
+const void* persist_fn_tile(const Impl<R>& m, bool shells, int npt) {
+#define ORB_FN(...) (const void*)cycle_persistent_kernel<__VA_ARGS__, R, MAXT>
+  if (!shells) return m.any_corot ? ORB_FN(PersistHexa<R, 64, 1>) : ORB_FN(PersistHexa<R, 64, 0>);
+  if (npt == 5 && m.uniform_npt == 5) return ORB_FN(PersistShell<R, TILE, 5, false>);
+  if (npt == 5) return ORB_FN(PersistShell<R, TILE, 5, true>);
+  if (npt == 3) return ORB_FN(PersistShell<R, TILE, 3, true>);
+  return ORB_FN(PersistShell<R, TILE, 0, true>);
+#undef ORB_FN
+}
 template <class R>
-using PersistFn = void (*)(ShellArgs<R>, NodeArgs<R>, PersistArgs, int, int, const float*);
-
-template <class R>
-PersistFn<R> persist_fn(int tile, bool npt5) {
-  if (tile == 64) return npt5 ? shell_persistent_kernel<R, 64, 5> : shell_persistent_kernel<R, 64, 0>;
-  if (tile == 128) return npt5 ? shell_persistent_kernel<R, 128, 5> : shell_persistent_kernel<R, 128, 0>;
-  return npt5 ? shell_persistent_kernel<R, 256, 5> : shell_persistent_kernel<R, 256, 0>;
+const void* persist_fn(const or_ecycle* h, const Impl<R>& m, int threads, int npt) {
+  const bool shells = h->hex.empty();
+  const int tile = shells ? h->tile_shell : h->tile_hex;
+  if constexpr (sizeof(R) == 8) {
+    if (persist_maxt(threads, true) == 256)
+      return tile == 64 ? persist_fn_tile<R, 64, 256>(m, shells, npt)
+             : tile == 128 ? persist_fn_tile<R, 128, 256>(m, shells, npt) : persist_fn_tile<R, 256, 256>(m, shells, npt);
+  }
+  return tile == 64 ? persist_fn_tile<R, 64, PERSIST_THREADS>(m, shells, npt)
+         : tile == 128 ? persist_fn_tile<R, 128, PERSIST_THREADS>(m, shells, npt)
+                       : persist_fn_tile<R, 256, PERSIST_THREADS>(m, shells, npt);
 }
 
 // Sets up the persistent launch when the handle qualifies: step() through a graph
-// (cfg.graph != 0), one part, shell groups only, no rigid links and no /CLOAD or
-// /PLOAD loads (the group pressure is fine), cfg.persistent not negative and
+// (cfg.graph != 0), one part, shell groups only or hexa groups only, no rigid links and no
+// /CLOAD or /PLOAD loads (the group pressure is fine), cfg.persistent not negative and
 // OR_ECYCLE_PERSISTENT not 0, and the
 // patches fit one cooperative wave of at most PERSIST_THREADS threads per CTA.
 // Each CTA takes P consecutive patches (Morton order keeps them compact) and holds
@@ -668,14 +690,18 @@ int persist_build(or_ecycle* h, Impl<R>& m) {
   if (h->cfg.persistent < 0) return OR_OK;
   if (const char* s = std::getenv("OR_ECYCLE_PERSISTENT"))
     if (std::atoi(s) == 0) return OR_OK;
-  if (!h->cfg.graph || m.nparts != 1 || !h->hex.empty() || h->shell.empty() || !h->links.empty() || m.nload ||
-      !h->rbodies.empty())
+  const bool shells = h->hex.empty();
+  if (!h->cfg.graph || m.nparts != 1 || (shells ? h->shell.empty() : !h->shell.empty()) || !h->links.empty() ||
+      m.nload || !h->rbodies.empty())
     return OR_OK;
-  const PatchSet& ps = m.sps;
-  const int tile = h->tile_shell;
+  const PatchSet& ps = shells ? m.sps : m.hps;
+  const int tile = shells ? h->tile_shell : h->tile_hex;
+  const int K = shells ? 4 : 8, NT = shells ? tile : tile / Pack<R>::N;      // corners, threads of a patch
+  if (!shells && tile != 64) return OR_OK;       // what the library picks for meshes of this size
+  const int corner_r = 24 * tile, node_r = shells ? 8 : 5;                    // Kind::CORNER_R, NODE_R
   const int npatch = (int)ps.info.size();
-  const int P = std::max((npatch + h->nsm - 1) / h->nsm, (128 + tile - 1) / tile);
-  if (P * tile > PERSIST_THREADS) return OR_OK;
+  const int P = std::max((npatch + h->nsm - 1) / h->nsm, shells ? (128 + tile - 1) / tile : 1);
+  if (P * NT > PERSIST_THREADS) return OR_OK;
   const int G = (npatch + P - 1) / P;
   std::vector<std::vector<int>> lists(G);
   std::vector<char> held(m.nnodpad, 0);
@@ -689,13 +715,19 @@ int persist_build(or_ecycle* h, Impl<R>& m) {
   const HPart& Pt = h->parts[0];
   for (int i = 0, k = 0; i < Pt.numnod; ++i)
     if (!held[Pt.node_start + i]) lists[(k++) % G].push_back(Pt.node_start + i);
-  std::vector<int> ofs(G + 1, 0), glob;
+  std::vector<int> holders(m.nnodpad, 0);
+  for (int c = 0; c < G; ++c)
+    for (int g : lists[c]) holders[g]++;
+  std::vector<int> ofs(G + 1, 0), glob, nshared(G, 0);
   std::vector<unsigned char> own;
   std::vector<int> first(m.nnodpad, -1);
   int ncmax = 0;
+  // a CTA's nodes: those other CTAs hold too, then its own, both in ascending order
+  auto before = [&](int a, int b) { return (holders[a] > 1) != (holders[b] > 1) ? holders[a] > 1 : a < b; };
   for (int c = 0; c < G; ++c) {
-    std::sort(lists[c].begin(), lists[c].end());
+    std::sort(lists[c].begin(), lists[c].end(), before);
     ncmax = std::max(ncmax, (int)lists[c].size());
+    for (int g : lists[c]) nshared[c] += holders[g] > 1;
     for (int g : lists[c]) {
       glob.push_back(g);
       own.push_back(first[g] < 0 ? 1 : 0);
@@ -704,42 +736,79 @@ int persist_build(or_ecycle* h, Impl<R>& m) {
     ofs[c + 1] = (int)glob.size();
   }
   if (ncmax > 65535) return OR_OK;
-  std::vector<uint2> pconn((size_t)ps.nelpad, make_uint2(0, 0));
+  std::vector<unsigned short> pconn((size_t)ps.nelpad * K, 0);
   for (int c = 0; c < G; ++c) {
     const std::vector<int>& L = lists[c];
     for (int p = c * P; p < std::min(npatch, (c + 1) * P); ++p) {
       const PatchInfo& pi = ps.info[p];
-      for (int t = 0; t < pi.nel; ++t) {
-        unsigned l[4];
-        for (int k = 0; k < 4; ++k) {
-          const int g = ps.nodes[pi.node_ofs + (ps.local[(size_t)(pi.elem0 + t) * 4 + k] & LOCAL_MASK)];
-          l[k] = (unsigned)(std::lower_bound(L.begin(), L.end(), g) - L.begin());
+      for (int t = 0; t < pi.nel; ++t)
+        for (int k = 0; k < K; ++k) {
+          const size_t q = (size_t)(pi.elem0 + t) * K + k;
+          const int g = ps.nodes[pi.node_ofs + (ps.local[q] & LOCAL_MASK)];
+          pconn[q] = (unsigned short)(std::lower_bound(L.begin(), L.end(), g, before) - L.begin());
         }
-        pconn[(size_t)pi.elem0 + t] = make_uint2(l[0] | l[1] << 16, l[2] | l[3] << 16);
-      }
     }
   }
-  const size_t smem = persist_smem<R>(ncmax, tile, P, m.sinc_stride, ps.nlmax);
-  if (smem > MAX_DYN_SMEM) return OR_OK;
-  // one thread per element, and per held node where the CTA holds more nodes than
-  // elements (a node phase of one node per thread), in whole TILE groups
-  const int T = std::min(PERSIST_THREADS / tile * tile, std::max(P * tile, (ncmax + tile - 1) / tile * tile));
-  const PersistFn<R> fn = persist_fn<R>(tile, m.uniform_npt == 5);
-  CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_DYN_SMEM));
+  // corner lists of the held nodes: per patch of the CTA its slot and corners (the patch
+  // lists are visited in ascending patch order, their corners ascend)
+  std::vector<int> list_ofs, words;
+  int nlist = 0;
+  for (int c = 0; c < G; ++c) {
+    const std::vector<int>& L = lists[c];
+    std::vector<std::vector<int>> of(L.size());
+    for (int p = c * P; p < std::min(npatch, (c + 1) * P); ++p) {
+      const PatchInfo& pi = ps.info[p];
+      std::vector<std::vector<int>> corners(pi.nloc);
+      for (int t = 0; t < pi.nel; ++t)
+        for (int k = 0; k < K; ++k)        // Kind::offset
+          corners[ps.local[(size_t)(pi.elem0 + t) * K + k] & LOCAL_MASK].push_back(
+              (p - c * P) * (shells ? 12 : 24) * tile + k * tile + t);
+      for (int j = 0; j < pi.nloc; ++j) {
+        const int g = ps.nodes[pi.node_ofs + j], slot = ps.slots[pi.node_ofs + j];
+        std::vector<int>& o = of[std::lower_bound(L.begin(), L.end(), g, before) - L.begin()];
+        if (corners[j].size() > 0xff || slot >= 1 << 23) return OR_OK;
+        o.push_back(slot << 8 | (int)corners[j].size());
+        o.insert(o.end(), corners[j].begin(), corners[j].end());
+      }
+    }
+    const int w0 = (int)words.size();
+    for (auto& o : of) {
+      list_ofs.push_back((int)words.size());
+      words.insert(words.end(), o.begin(), o.end());
+    }
+    nlist = std::max(nlist, (int)words.size() - w0);
+  }
+  list_ofs.push_back((int)words.size());
+  // the points of the shell kernel that keeps their state on the chip (PersistShell); in
+  // FP64 it lies in shared memory, and where that does not fit it stays in global memory
+  int npt = shells && (m.same_npt == 5 || m.same_npt == 3) ? m.same_npt : 0;
+  size_t smem = persist_smem<R>(node_r, corner_r + (sizeof(R) == 8 ? 6 * npt * tile : 0), ncmax, P, nlist);
+  if (npt && sizeof(R) == 8 && smem > PERSIST_MAX_SMEM) {
+    npt = 0;
+    smem = persist_smem<R>(node_r, corner_r, ncmax, P, nlist);
+  }
+  if (smem > PERSIST_MAX_SMEM) return OR_OK;
+  // one thread per element and a warp more, and one per held node where the CTA holds more
+  // nodes than that (node phases of one node per thread), in whole TILE groups
+  const int want = std::max(P * NT + 32, ncmax), unit = shells ? tile : 128;
+  const int T = std::min(PERSIST_THREADS / unit * unit, (want + unit - 1) / unit * unit);
+  const void* fn = persist_fn<R>(h, m, T, npt);
+  CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, PERSIST_MAX_SMEM));
   int nb = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, T, smem));
   if (nb < 1 || G > nb * h->nsm) return OR_OK;
   int rc;
   if ((rc = dput(h, q.node_ofs, ofs)) || (rc = dput(h, q.node_glob, glob)) || (rc = dput(h, q.owner, own)) ||
       (rc = dput(h, q.pconn, pconn)) || (rc = dalloc(h, q.fslot2, (size_t)m.nslot)) ||
-      (rc = dalloc(h, q.mslot2, (size_t)m.nslot)) || (rc = dalloc(h, q.acc3, 3)) || (rc = dalloc(h, q.sync, 2)) ||
+      (rc = dalloc(h, q.mslot2, shells ? (size_t)m.nslot : 0)) || (rc = dalloc(h, q.acc3, 3)) || (rc = dalloc(h, q.sync, SYNC_WORDS)) ||
+      (rc = dput(h, q.node_nshared, nshared)) || (rc = dput(h, q.list_ofs, list_ofs)) || (rc = dput(h, q.list, words)) ||
       (rc = dput(h, q.ek, std::vector<double>(m.nnodpad, 0.0))) ||
       (rc = dput(h, q.ekr, std::vector<double>(m.nnodpad, 0.0))))
     return rc;
   q.stall_cta = -1;
   if (const char* st = std::getenv("OR_ECYCLE_TEST_STALL_CTA")) q.stall_cta = std::atoi(st);
   q.on = true;
-  q.G = G; q.P = P; q.T = T; q.ncmax = ncmax; q.smem = smem;
+  q.G = G; q.P = P; q.T = T; q.ncmax = ncmax; q.nlist = nlist; q.npt = npt; q.smem = smem;
   return OR_OK;
 }
 
@@ -747,17 +816,18 @@ int persist_build(or_ecycle* h, Impl<R>& m) {
 template <class R>
 int launch_persistent(or_ecycle* h, Impl<R>& m, int ncycles, int parity0) {
   auto& q = m.per;
-  CK(cudaMemsetAsync(q.sync.p, 0, 2 * sizeof(unsigned), h->stream));
+  CK(cudaMemsetAsync(q.sync.p, 0, SYNC_WORDS * sizeof(unsigned), h->stream));
   CK(cudaMemsetAsync(q.acc3.p, 0xff, 3 * sizeof(PartAcc), h->stream));
   ShellArgs<R> sa = m.sargs();
+  HexArgs<R> ha = m.hargs();
   NodeArgs<R> na = m.nargs(h);
   PersistArgs pa = m.pargs();
   const float* zw = m.zw.p;
-  void* args[] = {&sa, &na, &pa, &ncycles, &parity0, &zw};
-  const PersistFn<R> fn = persist_fn<R>(h->tile_shell, m.uniform_npt == 5);
+  void* args[] = {h->hex.empty() ? (void*)&sa : (void*)&ha, &na, &pa, &ncycles, &parity0, &zw};
+  const void* fn = persist_fn<R>(h, m, q.T, q.npt);
   Trace tr("persistent cycles");
   const cudaError_t e =
-      cudaLaunchCooperativeKernel((const void*)fn, dim3(q.G), dim3(q.T), args, q.smem, h->stream);
+      cudaLaunchCooperativeKernel(fn, dim3(q.G), dim3(q.T), args, q.smem, h->stream);
   if (e == cudaErrorCooperativeLaunchTooLarge) {   // the wave no longer fits (another context holds SMs):
     cudaGetLastError();                             // the per-phase kernels take over for good
     q.on = false;
@@ -1107,6 +1177,9 @@ int finalize_impl(or_ecycle* h) {
       desc.push_back(d);
       m.maxnpt = std::max(m.maxnpt, g.prop.npt);
     }
+    m.same_npt = h->shell[0].prop.npt;
+    for (auto& g : h->shell)
+      if (g.prop.npt != m.same_npt) m.same_npt = 0;
     m.uniform_npt = h->shell[0].prop.npt == 5 ? 5 : 0;
     for (auto& g : h->shell)
       if (g.prop.npt != 5 || shell_ihbe(g.prop.ishell, g.prop.npt) != 1 || g.prop.ipla != 0) m.uniform_npt = 0;
@@ -1425,8 +1498,10 @@ double* pinned_device_ptr(double* host, size_t bytes) {
 
 // Nodes that one kernel writes straight into the caller's pinned arrays, instead of a
 // kernel and a copy through the staging buffer per array: three arrays of 1,403 nodes 45 -> 20 us,
-// of 40,401 nodes 96 -> 74 us.
-constexpr int DIRECT_NODES = 1 << 17;
+// of 40,401 nodes 95 -> 73 us, two of 134,064 148 -> 140 us.  From there on the link's rate
+// decides (262,701 nodes 257 us either way), and at 2 M nodes the copy engine is ahead (1778
+// against 1886 us).
+constexpr int DIRECT_NODES = 1 << 18;
 
 template <class R>
 int get_nodes_impl(or_ecycle* h, int part, double* x, double* d, double* v, double* vr) {
@@ -2642,10 +2717,10 @@ int or_ecycle_persistent_info(or_ecycle* h, int* on, int* ctas, int* threads) {
   int g = 0, t = 0, o = 0;
   if (h->cfg.precision == OR_PREC_SPLIT) {
     const auto& q = ((Impl<float>*)h->impl)->per;
-    o = q.on; g = q.G; t = q.T;
+    o = q.on && h->hex.empty(); g = q.G; t = q.T;
   } else {
     const auto& q = ((Impl<double>*)h->impl)->per;
-    o = q.on; g = q.G; t = q.T;
+    o = q.on && h->hex.empty(); g = q.G; t = q.T;
   }
   *on = o;
   if (ctas) *ctas = o ? g : 0;

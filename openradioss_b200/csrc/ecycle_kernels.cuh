@@ -16,6 +16,7 @@
 // patch partials instead of element corners).
 #pragma once
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 namespace orb {
@@ -411,6 +412,13 @@ __device__ __forceinline__ void mbar_init(unsigned long long* bar) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
+// an mbarrier of `count` arrivals, and one arrival
+__device__ __forceinline__ void mbar_init_n(unsigned long long* bar, unsigned count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 // the arrival, announcing the bytes the bulk copies below will deliver
 __device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
@@ -444,11 +452,11 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // read this GPU's own memory and complete in microseconds
 constexpr int STAGE_WAIT_TRIES = 1 << 22;
 
-// minimum of a 64-bit unsigned value over the warp, from two 32-bit hardware
-// reductions (high words, then the low words of the lanes holding the high minimum)
-__device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v) {
-  const unsigned hi = __reduce_min_sync(0xffffffffu, (unsigned)(v >> 32));
-  const unsigned lo = __reduce_min_sync(0xffffffffu, (unsigned)(v >> 32) == hi ? (unsigned)v : 0xffffffffu);
+// minimum of a 64-bit unsigned value over the warp's lanes of `lanes`, from two 32-bit
+// hardware reductions (high words, then the low words of the lanes holding the high minimum)
+__device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v, unsigned lanes = 0xffffffffu) {
+  const unsigned hi = __reduce_min_sync(lanes, (unsigned)(v >> 32));
+  const unsigned lo = __reduce_min_sync(lanes, (unsigned)(v >> 32) == hi ? (unsigned)v : 0xffffffffu);
   return ((unsigned long long)hi << 32) | lo;
 }
 
@@ -1094,13 +1102,14 @@ __device__ __forceinline__ void shell_load_state(const ShellArgs<R>& a, int e, S
 }
 
 // Writes back the state that shell_element<KEEP = true> kept in registers.
-template <class R, int NPT>
+template <class R, int NPT, bool IP = true>
 __device__ __forceinline__ void shell_store_state(const ShellArgs<R>& a, int e, const ShellState<R, NPT>& st) {
   static_assert(NPT > 0, "kept state needs a fixed number of integration points");
   const int nelpad = a.nelpad;
   a.thk[e] = st.thk;
   a.hourg[0 * nelpad + e] = st.h[0]; a.hourg[1 * nelpad + e] = st.h[1]; a.hourg[2 * nelpad + e] = st.h[2];
   a.eint[0 * nelpad + e] = st.e[0]; a.eint[1 * nelpad + e] = st.e[1];
+  if (!IP) return;
 #pragma unroll
   for (int ip = 0; ip < NPT; ++ip) {
 #pragma unroll
@@ -1116,18 +1125,26 @@ __device__ __forceinline__ void shell_store_state(const ShellArgs<R>& a, int e, 
 // moments out in global axes with CUPDT3P signs.  KEEP = false writes the new
 // state to memory at index e, as each quantity is formed; KEEP = true leaves it
 // in st (for a caller that keeps the state in registers across cycles).  STAGED
-// (with NPT > 0, KEEP false): the old integration-point state is read from shared
+// (with NPT > 0): the old integration-point state is read from shared
 // planes, stress component c of point ip at sip[(ip * 5 + c) * sstride] and the
-// plastic strain of point ip at sip[(NPT * 5 + ip) * sstride], instead of from st.
-template <class R, int NPT, bool KEEP, bool STAGED = false>
+// plastic strain of point ip at sip[(NPT * 5 + ip) * sstride], instead of from st; with
+// KEEP the new one goes back there.
+// GEN: the group's formulation (Ishell) and plastic return (Iplas) decide at run time;
+// without it they are Ishell 1 and the radial return.  The element's time step depends on
+// its geometry alone (CDLEN3): early(key, bits), if given, is called as soon as it is known,
+// by every thread that runs the element.  Without it CDT3 stays where the reference has it:
+// its branch ends a basic block, across which the compiler fuses no multiply-add, so that
+// moving it would change the rounding of the patch kernels.
+struct NoEarly {};
+template <class R, int NPT, bool KEEP, bool STAGED = false, bool GEN = NPT == 0, class Early = NoEarly>
 __device__ __forceinline__ void shell_element(const ShellArgs<R>& a, const int e, const ShellGroupDesc& gd,
                                               const R DT1, const float* __restrict__ zw, const double* sx,
                                               const double* sy, const double* sz, const R* sv, const int NLM,
                                               const int (&lc)[4], ShellState<R, NPT>& st, R (&Fg)[3][4],
                                               R (&Mg)[3][4], unsigned long long& mykey, unsigned long long& mybits,
-                                              double& my_ehou, double& my_wpla, const R* sip = nullptr,
-                                              const int sstride = 0) {
-  static_assert(!STAGED || (NPT > 0 && !KEEP), "staged state: fixed points, written to memory");
+                                              double& my_ehou, double& my_wpla, R* sip = nullptr,
+                                              const int sstride = 0, const Early& early = Early()) {
+  static_assert(!STAGED || NPT > 0, "staged state: fixed points");
   static_assert(!KEEP || NPT > 0, "kept state needs a fixed number of integration points");
   const int nelpad = a.nelpad;
   const R OFF = R(1);
@@ -1215,6 +1232,15 @@ __device__ __forceinline__ void shell_element(const ShellArgs<R>& a, const int e
     if (DTHOUR < ALDT) ALDT = DTHOUR;
     ALDT = ssqrt(ALDT);
   }
+  // ---- CDT3 (cdt3.F:110-115, 203-214) ----
+  constexpr bool HAS_EARLY = !std::is_same<Early, NoEarly>::value;
+  if constexpr (HAS_EARLY) {
+    const R DT = R(gd.dtfac) * ALDT / SSP;
+    if ((double)DT <= gd.dtmin) raise_error(a.err, 5, st.eid);
+    mykey = dt_key((double)DT, 3, st.eid);
+    mybits = (unsigned long long)__double_as_longlong((double)DT);
+    early(mykey, mybits);
+  }
   // ---- CDEFO3 (cdefo3.F:84-220): IHBE <= 1, 2 and 4 ----
   R VXl[4], VYl[4], VZl[4], RXl[4], RYl[4];
 #pragma unroll
@@ -1227,10 +1253,10 @@ __device__ __forceinline__ void shell_element(const ShellArgs<R>& a, const int e
     RXl[k] = E1X * rx + E1Y * ry + E1Z * rz;
     RYl[k] = E2X * rx + E2Y * ry + E2Z * rz;
   }
-  // NPT = 5 kernels are launched only when every group is Ishell 1 (IHBE 1) with
-  // M2CPLR's radial return (IPLA 0): the other branches compile out of them
-  const int IHBE = NPT == 5 ? 1 : gd.ihbe;
-  const int IPLA = NPT == 5 ? 0 : gd.ipla;
+  // without GEN every group is Ishell 1 (IHBE 1) with M2CPLR's radial return (IPLA 0):
+  // the other branches compile out
+  const int IHBE = GEN ? gd.ihbe : 1;
+  const int IPLA = GEN ? gd.ipla : 0;
   R EXX, EYY, EXY, EXZ, EYZ, KXX, KYY, KXY;
   {
     const R VZ13 = VZl[0] - VZl[2], VZ24 = VZl[1] - VZl[3];
@@ -1369,12 +1395,14 @@ __device__ __forceinline__ void shell_element(const ShellArgs<R>& a, const int e
           DPLA = OFF * fmax(R(0), (SVM - YLD) / YM);
           EZZ = DPLA * (R(0.5) * (SN[0] + SN[1])) / YLD;
           PLA = PLA + DPLA;
-          if (KEEP) st.pla[NPT > 0 ? ip : 0] = PLA;
+          if (KEEP && STAGED) sip[((NPT > 0 ? NPT : 1) * 5 + ip) * sstride] = PLA;
+          else if (KEEP) st.pla[NPT > 0 ? ip : 0] = PLA;
           else a.pla[ip * nelpad + e] = PLA;
         }
       } else {
         if (m2cplr_iterative<R>(IPLA, SN, PLA, YLD, DPLA, EZZ, CA, CB, CN, YMAX, YM, NU, GG, OFF)) {
-          if (KEEP) st.pla[NPT > 0 ? ip : 0] = PLA;
+          if (KEEP && STAGED) sip[((NPT > 0 ? NPT : 1) * 5 + ip) * sstride] = PLA;
+          else if (KEEP) st.pla[NPT > 0 ? ip : 0] = PLA;
           else a.pla[ip * nelpad + e] = PLA;
         }
       }
@@ -1384,7 +1412,10 @@ __device__ __forceinline__ void shell_element(const ShellArgs<R>& a, const int e
       if (DPLA != R(0)) wpla += (double)YLD * (double)DPLA * (double)AREA * (double)THKLYL;
     }
     THKN = THKN + EZZ * THKLYL * OFF;
-    if (KEEP) {
+    if (KEEP && STAGED) {
+#pragma unroll
+      for (int c = 0; c < 5; ++c) sip[(ip * 5 + c) * sstride] = SN[c];
+    } else if (KEEP) {
 #pragma unroll
       for (int c = 0; c < 5; ++c) st.sig[NPT > 0 ? ip : 0][c] = SN[c];
     } else {
@@ -1548,8 +1579,7 @@ __device__ __forceinline__ void shell_element(const ShellArgs<R>& a, const int e
     if (KEEP) { st.h[0] = hour1; st.h[1] = hour2; st.h[2] = hour3; }
     else { a.hourg[0 * nelpad + e] = hour1; a.hourg[1 * nelpad + e] = hour2; a.hourg[2 * nelpad + e] = hour3; }
   }
-  // ---- CDT3 (cdt3.F:110-115, 203-214) ----
-  {
+  if constexpr (!HAS_EARLY) {
     const R DT = R(gd.dtfac) * ALDT / SSP;
     if ((double)DT <= gd.dtmin) raise_error(a.err, 5, st.eid);
     mykey = dt_key((double)DT, 3, st.eid);

@@ -1,56 +1,75 @@
-// persistent_kernel.cuh -- the whole explicit cycle of a shell mesh in one launch.
+// persistent_kernel.cuh -- the whole explicit cycle of a small mesh in one launch.
 //
-// For a mesh whose element and nodal state fit on the chip (one part of BT
-// shells, C2-sized), shell_persistent_kernel runs all the cycles of a step in a
-// single cooperative launch of one CTA per SM:
+// For a mesh whose element and nodal state fit on the chip (one part of BT shells or of
+// hexas), cycle_persistent_kernel runs all the cycles of a step in a
+// single cooperative launch of one CTA per SM.  Every CTA keeps its patches' element
+// state in registers and all the nodes they touch in shared memory; a node that several
+// CTAs hold is updated identically by each of them.  A cycle:
 //
-//   per cycle   element phase   every CTA computes its patches (the same patches,
-//                               element arithmetic and incidence-list sums as
-//                               shell_patch_kernel) from nodal state it keeps in
-//                               shared memory and element state it keeps in
-//                               registers, writes the patch partial sums to the
-//                               node-major slot skyline and min-reduces the time step
-//               grid barrier    (one per cycle)
-//               node phase      every CTA updates all the nodes its patches touch
-//                               (ASSPAR4 over the skyline slots in patch order, the
-//                               dt logic, ACCELE, BCS10, VELOCITY, DEPLA: the same
-//                               node_update as the node pass), so a node shared by
-//                               several CTAs is updated identically by each of them
+//   element phase   the patches' elements, corner forces to shared memory.  The time step
+//                   of an element is known before its forces (a shell's from its geometry
+//                   alone): each warp hands in its minimum as soon as it has it, and one
+//                   thread (of a warp without elements, where there is one) sends the CTA's
+//                   minimum to the grid, counts the CTA as arrived and waits for the others,
+//                   all while the elements' arithmetic goes on.
+//   shared nodes    partial sums, patch by patch, of the nodes other CTAs hold too, to the
+//                   node-major slot skyline; the CTA arrives at the grid's second counter
+//   own nodes       all other nodes: patch partials summed from shared memory in the same
+//                   order, then the dt logic, ACCELE, BCS10, VELOCITY, DEPLA (node_update
+//                   of the node pass).  They need nothing from other CTAs but the time step,
+//                   so their update runs while the shared nodes' slots travel.
+//   shared nodes    wait for the second counter, ASSPAR4 over the slots, node update
 //
-// Only the skyline slots and the time-step reduction cross between SMs (through
+// With one grid barrier between all elements and all nodes, and every patch partial
+// through L2, the 200x200 split plate took 7.5 us a cycle, now 7.0, and 10,000 shells with
+// the Newton return 8.8, now 6.2.  Hexas took two launches a cycle: 4,000 in FP64 9.9 us, now
+// 7.3; 28,952 in the split form 12.6, now 9.1.  What is left is latency: an element's chain
+// (3.2 us of the split plate's cycle), the assembly from shared memory, two L2 round trips.
+//
+// Only the shared nodes' slots and the time-step reduction cross between SMs (through
 // L2).  The slots are double-buffered by cycle parity and the reduction is
-// triple-buffered, so one barrier per cycle orders every reuse.  The result is
-// bit for bit the result of the patch and node kernels: the same operations in
-// the same order.  After the last cycle each node's owner (the lowest CTA that
+// triple-buffered: a CTA reaches the reuse of a buffer only after a counter that every
+// reader has passed.  For shells the result is that of the patch and node kernels: the
+// same operations in the same order (for hexas see hex_element.cuh).  After the last cycle each node's owner (the lowest CTA that
 // holds it) writes it back, the element state is written back, and the kinetic
 // energy is summed per node tile exactly as the node pass sums it.
 //
-// The barrier is a monotonic arrival counter polled with a time limit: past the
-// limit a CTA sets an abort flag and the OR_E_TIMEOUT error word, and every CTA
-// leaves at its next barrier, so the launch always ends.
+// The counters are monotonic and polled with a time limit: past the limit a CTA sets an
+// abort flag and the OR_E_TIMEOUT error word, and every CTA leaves at its next wait, so
+// the launch always ends.
 #pragma once
 #include "ecycle_kernels.cuh"
+#include "hex_element.cuh"
 
 namespace orb {
 
-// host-built layout of the persistent launch (one part, shell groups only)
+// host-built layout of the persistent launch (one part, shell groups or hexa groups only)
 struct PersistArgs {
   const int* node_ofs;        // G + 1: CTA c holds nodes node_ofs[c] .. node_ofs[c+1]-1 of the lists below
-  const int* node_glob;       // padded global node number of each held node, ascending within a CTA
+  const int* node_glob;       // padded global node number of each held node: a CTA's shared nodes, then its own
+  const int* node_nshared;    // G: how many of them are shared with other CTAs
   const unsigned char* owner; // 1 where the CTA is the lowest that holds the node
-  const uint2* pconn;         // per padded shell element: 4 x uint16 CTA-local node indices
+  const unsigned short* pconn;  // per padded element: its 4 or 8 corners' CTA-local node indices
+  // Corner lists: held node i of the lists above has the words list[list_ofs[i]] ..
+  // list[list_ofs[i+1]-1].  For each patch of the CTA that touches it, in ascending order:
+  // slot << 8 | count, then the count corners in ascending (element, corner) order, each
+  // as the offset of its first value among the CTA's corner forces.
+  const int* list_ofs;
+  const int* list;
   void* fslot2;               // second slot buffers (odd cycles); the handle's fslot / mslot serve even ones
   void* mslot2;
   PartAcc* acc3;              // triple-buffered time-step reduction
   double* ek_node;            // last cycle's kinetic energy of every node (owners write)
   double* ekr_node;
-  unsigned* sync;             // [0] arrival counter, [1] abort flag
+  unsigned* sync;             // [0] time-step counter, [1] abort flag, [SYNC_SLOTS] slot counter
   int patches_per_cta;        // P
   int ncmax;                  // node capacity of a CTA (stride of the shared planes)
+  int nlist;                  // list capacity of a CTA
   int ntiles_node;            // node tiles of NODE tile size 128 (kinetic energy partials)
   int stall_cta;              // test hook (OR_ECYCLE_TEST_STALL_CTA): this CTA does not arrive at the
-                              // first cycle's barrier, so the others' bounded waits run out; -1 off
+                              // first cycle's counter, so the others' bounded waits run out; -1 off
 };
+constexpr int SYNC_SLOTS = 32, SYNC_WORDS = 64;      // the two counters on lines of their own
 
 // L2-coherent loads and stores (bypassing L1) of the data other SMs write during
 // the launch: the slot skyline and the reduction
@@ -66,38 +85,31 @@ __device__ __forceinline__ void st_cg(double4* p, double4 v) {
   __stcg(reinterpret_cast<double2*>(p) + 1, make_double2(v.z, v.w));
 }
 
-// one grid-wide barrier: arrive, then poll the counter until every CTA arrived at
-// this barrier; true when the launch must end (a CTA gave up waiting)
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ bool grid_barrier(unsigned* sync, unsigned target, ErrorWord* err, int* s_abort,
-                                             bool arrive = true) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();                          // release: this CTA's slot writes and reductions
-    if (arrive) atomicAdd(&sync[0], 1u);
-    const long long t0 = clock64();
-    int ab = 0;
-    for (;;) {
-      const unsigned v = ld_acquire(&sync[0]);  // acquire: every CTA's writes before its arrival
-      if (v >= target) break;
-      if (__ldcg(&sync[1])) { ab = 1; break; }
-      if (clock64() - t0 > (1ll << 31)) {           // about a second at the SM clock
-        atomicExch(&sync[1], 1u);
-        raise_error(err, 7, (int)blockIdx.x);
-        ab = 1;
-        break;
-      }
-      __nanosleep(32);
+// One thread's part of a grid-wide counter.  Arrive: release what the CTA wrote before.
+__device__ __forceinline__ void grid_arrive(unsigned* count) {
+  __threadfence();
+  atomicAdd(count, 1u);
+}
+// Wait until `target` arrivals were counted; true when the launch must end (a CTA gave up)
+__device__ __forceinline__ bool grid_wait(unsigned* count, unsigned target, unsigned* abort, ErrorWord* err) {
+  const long long t0 = clock64();
+  for (;;) {
+    if (ld_acquire(count) >= target) return false;  // acquire: every CTA's writes before its arrival
+    if (__ldcg(abort)) break;
+    if (clock64() - t0 > (1ll << 31)) {             // about a second at the SM clock
+      atomicExch(abort, 1u);
+      raise_error(err, 7, (int)blockIdx.x);
+      break;
     }
-    if (ab) __threadfence();
-    *s_abort = ab;
+    __nanosleep(20);
   }
-  __syncthreads();
-  return *s_abort != 0;
+  __threadfence();
+  return true;
 }
 
 // pairs of reals for the corner-force planes of the persistent kernel
@@ -107,80 +119,248 @@ template <> struct Vec2<double> { typedef double2 T; };
 __device__ __forceinline__ float2 mk2(float a, float b) { return make_float2(a, b); }
 __device__ __forceinline__ double2 mk2(double a, double b) { return make_double2(a, b); }
 
-// the dt-key / dt-bits min and the two energy sums of a group of TILE threads
-// (threads g*TILE .. g*TILE+TILE-1), with the operation order of block_reduce
-template <int TILE>
-__device__ inline void group_reduce(unsigned long long& key, unsigned long long& bits, double& s0, double& s1,
-                                    unsigned long long* skey, unsigned long long* sbits, double* ss0, double* ss1) {
-  const int lt = threadIdx.x % TILE;
+// the two energy sums of a group of NT threads (threads g*NT .. g*NT+NT-1), with the
+// operation order of block_reduce
+template <int NT>
+__device__ inline void group_sums(double& s0, double& s1, double* ss0, double* ss1) {
+  const int lt = threadIdx.x % NT;
   const int lane = lt & 31, warp = lt >> 5;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    unsigned long long k2 = __shfl_xor_sync(0xffffffffu, key, o);
-    unsigned long long b2 = __shfl_xor_sync(0xffffffffu, bits, o);
-    key = k2 < key ? k2 : key;
-    bits = b2 < bits ? b2 : bits;
     s0 += __shfl_xor_sync(0xffffffffu, s0, o);
     s1 += __shfl_xor_sync(0xffffffffu, s1, o);
   }
-  if (lane == 0) { skey[warp] = key; sbits[warp] = bits; ss0[warp] = s0; ss1[warp] = s1; }
+  if (lane == 0) { ss0[warp] = s0; ss1[warp] = s1; }
   __syncthreads();
   if (warp == 0) {
-    constexpr int NW = TILE / 32;
-    key = lane < NW ? skey[lane] : ~0ull;
-    bits = lane < NW ? sbits[lane] : ~0ull;
+    constexpr int NW = NT / 32;
     s0 = lane < NW ? ss0[lane] : 0.0;
     s1 = lane < NW ? ss1[lane] : 0.0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-      unsigned long long k2 = __shfl_xor_sync(0xffffffffu, key, o);
-      unsigned long long b2 = __shfl_xor_sync(0xffffffffu, bits, o);
-      key = k2 < key ? k2 : key;
-      bits = b2 < bits ? b2 : bits;
       s0 += __shfl_xor_sync(0xffffffffu, s0, o);
       s1 += __shfl_xor_sync(0xffffffffu, s1, o);
     }
   }
 }
 
-// Threads per CTA: at least P patches x TILE elements (one per element), raised to
-// cover the CTA's held nodes (one per node in the node phase) and at most
-// PERSIST_THREADS; one CTA per SM (the register budget of the shell element at that
-// many threads).  Threads beyond the P patches work in the node phase only.
+// Threads per CTA: at least one per element (per pair of hexas in the split form), raised
+// to cover the CTA's held nodes (one per node in the node phases) and a warp without
+// elements, and at most PERSIST_THREADS; one CTA per SM.  The threads beyond the elements'
+// work on the time step and the nodes only.  MAXT is the thread count that a kernel's
+// register budget is for: PERSIST_THREADS (168 registers), or 256 (255), where FP64
+// elements spill less.
 constexpr int PERSIST_THREADS = 384;
-// reduction scratch is laid out for every TILE group of PERSIST_THREADS threads
-__host__ __device__ constexpr int persist_groups(int tile) { return (PERSIST_THREADS + tile - 1) / tile; }
+constexpr int persist_maxt(int threads, bool fp64) { return fp64 && threads <= 256 ? 256 : PERSIST_THREADS; }
 
+// ---- the elements of a thread -------------------------------------------------
+// Kind: NODE_R, reals per held node beside the coordinates; C, force components per
+// corner; TILE elements and NT threads per patch; CORNER_R, reals of corner forces per
+// patch, and STATE_R, of element state kept in shared memory.  element() evaluates the thread's elements into the corner forces, corner() reads
+// one corner back.
+
+// one shell; corner forces and moments as three planes of pairs (fx fy | fz mx | my mz),
+// corner k of element t at pair k * TILE + t.  In FP64 the integration points' state (60
+// registers for 5 points) is kept in shared planes instead of registers, which spilled:
+// the 200x200 plate 18.9 -> 16.1 us a cycle together with the single node update below.
+template <class R, int TILE_, int NPT, bool GEN>
+struct PersistShell {
+  typedef ShellArgs<R> Args;
+  typedef typename Vec2<R>::T R2;
+  static constexpr bool KEEP = NPT > 0, PLANES = KEEP && sizeof(R) == 8;
+  static constexpr int TILE = TILE_, NT = TILE, C = 6, NODE_R = 8, CORNER_R = 24 * TILE,
+                       STATE_R = PLANES ? 6 * NPT * TILE : 0;
+  ShellState<R, NPT> st;
+  int lc[4], e, lt;
+  ShellGroupDesc gd;
+  const float* zw;
+  R* sc;                        // the patch's corner forces
+  R* sp;                        // PLANES: this thread's entry of the patch's state planes
+  __device__ __forceinline__ bool load(const Args& a, const PersistArgs& pa, const float* z, int p, bool has, int t, R* c,
+                                       R* state) {
+    zw = z; sc = c; sp = state + t; lt = t; e = (has ? p : 0) * TILE + t;
+    if (KEEP) shell_load_state<R, NPT, !PLANES>(a, e, st);
+    if constexpr (PLANES) {
+      if (has) {
+#pragma unroll 5
+        for (int q = 0; q < 5 * NPT; ++q) sp[q * TILE] = a.sig[q * a.nelpad + e];
+#pragma unroll
+        for (int ip = 0; ip < NPT; ++ip) sp[(5 * NPT + ip) * TILE] = a.pla[ip * a.nelpad + e];
+      }
+    }
+    const uint2 w = reinterpret_cast<const uint2*>(pa.pconn)[e];
+    lc[0] = w.x & 0xffffu; lc[1] = w.x >> 16; lc[2] = w.y & 0xffffu; lc[3] = w.y >> 16;
+    gd = a.groups[has ? a.patch[p].group : 0];
+    return has && t < a.patch[p].nel;
+  }
+  template <class Early>
+  __device__ __forceinline__ void element(const Args& a, const R DT1, const double* sx, const double* sy,
+                                          const double* sz, const R* sv, const int NC, const Early& early,
+                                          double& ehou, double& wpla) {
+    R Fg[3][4], Mg[3][4];
+    unsigned long long key = ~0ull, bits = ~0ull;
+    double h = 0.0, w = 0.0;
+    if (!KEEP) shell_load_state<R, NPT>(a, e, st);
+    shell_element<R, NPT, KEEP, PLANES, GEN>(a, e, gd, DT1, zw, sx, sy, sz, sv, NC, lc, st, Fg, Mg, key, bits, h, w, sp,
+                                             TILE, early);
+    R2* q = reinterpret_cast<R2*>(sc);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      q[(0 * 4 + k) * TILE + lt] = mk2(Fg[0][k], Fg[1][k]);
+      q[(1 * 4 + k) * TILE + lt] = mk2(Fg[2][k], Mg[0][k]);
+      q[(2 * 4 + k) * TILE + lt] = mk2(Mg[1][k], Mg[2][k]);
+    }
+    ehou += h;
+    wpla += w;
+  }
+  static __host__ __device__ int offset(int sub, int t, int k) { return sub * 12 * TILE + k * TILE + t; }
+  static __device__ __forceinline__ void corner(const R* all, int o, R (&f)[C]) {
+    const R2* q = reinterpret_cast<const R2*>(all);
+    const R2 p0 = q[o], p1 = q[4 * TILE + o], p2 = q[8 * TILE + o];
+    f[0] += p0.x; f[1] += p0.y; f[2] += p1.x; f[3] += p1.y; f[4] += p2.x; f[5] += p2.y;
+  }
+  __device__ __forceinline__ void store(const Args& a, bool has) const {
+    if (!has) return;
+    if constexpr (KEEP) shell_store_state<R, NPT, !PLANES>(a, e, st);
+    if constexpr (PLANES) {
+#pragma unroll 5
+      for (int q = 0; q < 5 * NPT; ++q) a.sig[q * a.nelpad + e] = sp[q * TILE];
+#pragma unroll
+      for (int ip = 0; ip < NPT; ++ip) a.pla[ip * a.nelpad + e] = sp[(5 * NPT + ip) * TILE];
+    }
+  }
+};
+
+// N hexas (hex_element.cuh); corner forces in three planes of TILE x 8, corner k of
+// element t at k * TILE + t
+template <class R, int TILE_, int CORO>
+struct PersistHexa {
+  typedef HexArgs<R> Args;
+  typedef Pack<R> K;
+  typedef typename K::W W;
+  typedef typename Vec4<R>::T R4;
+  static constexpr int N = K::N, TILE = TILE_, NT = TILE / N, C = 3, NODE_R = 5, CORNER_R = 24 * TILE, STATE_R = 0;
+  W sig_[6], eint_, rho_, qvis_, vol0_, pla_, epsd_;
+  double v0_[N];
+  int eid_[N], lc[N][8], e, t0;
+  bool act[N];
+  HexGroupDesc gd;
+  R* sc;
+  __device__ __forceinline__ bool load(const Args& a, const PersistArgs& pa, const float*, int p, bool has, int t, R* c,
+                                       R*) {
+    sc = c; t0 = N * t; e = (has ? p : 0) * TILE + t0;
+    const int nel = has ? a.patch[p].nel : 0;
+    auto ld = [&](const R* q) { return K::map([&](int i) { return q[e + i]; }); };
+#pragma unroll
+    for (int k = 0; k < 6; ++k) sig_[k] = ld(a.sig + (size_t)k * a.nelpad);
+    eint_ = ld(a.eint); rho_ = ld(a.rho); qvis_ = ld(a.qvis); vol0_ = ld(a.vol0); pla_ = ld(a.pla); epsd_ = ld(a.epsd);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      act[i] = t0 + i < nel;
+      eid_[i] = a.elem_id[e + i];
+      v0_[i] = a.vol0dp[e + i];
+      const uint4 w = reinterpret_cast<const uint4*>(pa.pconn)[e + i];
+      const unsigned q[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+      for (int k = 0; k < 8; ++k) lc[i][k] = (q[k / 2] >> (16 * (k & 1))) & 0xffffu;
+    }
+    gd = a.groups[has ? a.patch[p].group : 0];
+    return act[0];
+  }
+  // what hex_element asks for
+  template <class Early>
+  struct IO {
+    PersistHexa& h;
+    const double *sx, *sy, *sz;
+    const R* sv;
+    const int NC;
+    const Early& hand_in;
+    __device__ __forceinline__ void x(int i, int k, double (&o)[3]) const {
+      const int l = h.lc[i][k];
+      o[0] = sx[l]; o[1] = sy[l]; o[2] = sz[l];
+    }
+    __device__ __forceinline__ void v(int i, int k, R (&o)[3]) const {
+      const int l = h.lc[i][k];
+      o[0] = sv[l]; o[1] = sv[NC + l]; o[2] = sv[2 * NC + l];
+    }
+    __device__ __forceinline__ int eid(int i) const { return h.eid_[i]; }
+    __device__ __forceinline__ double vol0dp(int i) const { return h.v0_[i]; }
+    __device__ __forceinline__ W sig(int c) const { return h.sig_[c]; }
+    __device__ __forceinline__ W eint() const { return h.eint_; }
+    __device__ __forceinline__ W rho() const { return h.rho_; }
+    __device__ __forceinline__ W qvis() const { return h.qvis_; }
+    __device__ __forceinline__ W vol0() const { return h.vol0_; }
+    __device__ __forceinline__ W pla() const { return h.pla_; }
+    __device__ __forceinline__ void put_sig(int c, W a) const { h.sig_[c] = a; }
+    __device__ __forceinline__ void put_eint(W a) const { h.eint_ = a; }
+    __device__ __forceinline__ void put_rho(W a) const { h.rho_ = a; }
+    __device__ __forceinline__ void put_qvis(W a) const { h.qvis_ = a; }
+    __device__ __forceinline__ void put_pla(W a) const { h.pla_ = a; }
+    __device__ __forceinline__ void put_epsd(W a) const { h.epsd_ = a; }
+    __device__ __forceinline__ void early(unsigned long long k, unsigned long long b) const { hand_in(k, b); }
+    __device__ __forceinline__ void corner(int k, const W (&f)[3]) const {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        R* q = h.sc + (8 * c + k) * TILE + h.t0;
+        if constexpr (N == 2) *reinterpret_cast<float2*>(q) = make_float2(f2_get(f[c], 0), f2_get(f[c], 1));
+        else *q = f[c];
+      }
+    }
+  };
+  template <class Early>
+  __device__ __forceinline__ void element(const Args& a, const R DT1, const double* sx, const double* sy,
+                                          const double* sz, const R* sv, const int NC, const Early& early,
+                                          double& ehou, double& wpla) {
+    IO<Early> io{*this, sx, sy, sz, sv, NC, early};
+    hex_element<R, CORO>(gd, act, DT1, io, a.err, ehou, wpla);
+  }
+  static __host__ __device__ int offset(int sub, int t, int k) { return sub * 24 * TILE + k * TILE + t; }
+  static __device__ __forceinline__ void corner(const R* all, int o, R (&f)[C]) {
+    f[0] += all[o]; f[1] += all[8 * TILE + o]; f[2] += all[16 * TILE + o];
+  }
+  __device__ __forceinline__ void store(const Args& a, bool has) const {
+    if (!has) return;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      if (!act[i]) continue;
+#pragma unroll
+      for (int c = 0; c < 6; ++c) a.sig[(size_t)c * a.nelpad + e + i] = K::get(sig_[c], i);
+      a.eint[e + i] = K::get(eint_, i);
+      a.rho[e + i] = K::get(rho_, i);
+      a.qvis[e + i] = K::get(qvis_, i);
+      a.pla[e + i] = K::get(pla_, i);
+      a.epsd[e + i] = K::get(epsd_, i);
+    }
+  }
+};
+
+// Shared memory: node planes x y z dx dy dz (FP64) and NODE_R of R (velocities, mass, with
+// rotations also those and the inertia), global index (int), owner and code (bytes); per
+// patch its corner forces and state planes; per held node its list range and slot range (int2); the lists
 template <class R>
-__host__ __device__ inline size_t persist_smem(int ncmax, int tile, int P, int inc_stride, int nlmax) {
-  // node planes: x y z dx dy dz (FP64), vx vy vz rx ry rz ms in (R), global index
-  // (int), owner and code (bytes); per patch: 24 corner planes of TILE (R), the
-  // incidence lists (uint16), reduction scratch, the slot of each patch node (int);
-  // per held node its slot range (int2)
-  const size_t nodes = (size_t)ncmax * (6 * sizeof(double) + 8 * sizeof(R) + sizeof(int) + 2);
-  const size_t nodes_al = (nodes + 15) / 16 * 16;
-  const size_t corners = (size_t)P * 24 * tile * sizeof(R);
-  const size_t inc = ((size_t)P * inc_stride * 2 + 15) / 16 * 16;
-  const size_t red = (size_t)persist_groups(tile) * (tile / 32) * 32;
-  const size_t slots = ((size_t)P * nlmax * sizeof(int) + 15) / 16 * 16;
-  const size_t ranges = (size_t)ncmax * sizeof(int2);
-  return nodes_al + corners + inc + red + slots + ranges;
+inline size_t persist_smem(int node_r, int patch_r, int ncmax, int P, int nlist) {
+  const size_t nodes = (size_t)ncmax * (6 * sizeof(double) + node_r * sizeof(R) + sizeof(int) + 2);
+  return (nodes + 15) / 16 * 16 + (size_t)P * patch_r * sizeof(R) +      // patch_r: CORNER_R + STATE_R
+         2 * (size_t)ncmax * sizeof(int2) + (size_t)nlist * sizeof(int);
 }
 
-template <class R, int TILE, int NPT>
-__global__ void __launch_bounds__(PERSIST_THREADS, 1)
-shell_persistent_kernel(ShellArgs<R> a, NodeArgs<R> na, PersistArgs pa, int ncycles, int parity0,
+template <class Kind, class R, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1)
+cycle_persistent_kernel(typename Kind::Args a, NodeArgs<R> na, PersistArgs pa, int ncycles, int parity0,
                         const float* __restrict__ zw) {
   typedef typename Vec4<R>::T R4;
-  constexpr bool KEEP = NPT > 0;
+  constexpr int NT = Kind::NT, C = Kind::C;
+  constexpr bool ROT = C == 6;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_abort;
   __shared__ double s_e0[PERSIST_THREADS / 32], s_e1[PERSIST_THREADS / 32];
   __shared__ unsigned long long s_dt[2];        // the CTA's dt key and dt bits minimum of a cycle
+  __shared__ PartAcc s_acc;                     // the grid's
+  __shared__ __align__(8) unsigned long long s_dtbar;
   const int tid = threadIdx.x;
   const int cta = blockIdx.x, G = gridDim.x;
   const int P = pa.patches_per_cta, NC = pa.ncmax;
-  const int sub = tid / TILE, lt = tid % TILE;
+  const int sub = tid / NT, lt = tid % NT;
   // ---- shared layout ----
   double* sx = reinterpret_cast<double*>(smem_raw);
   double* sy = sx + NC;
@@ -188,199 +368,207 @@ shell_persistent_kernel(ShellArgs<R> a, NodeArgs<R> na, PersistArgs pa, int ncyc
   double* sdx = sz + NC;
   double* sdy = sdx + NC;
   double* sdz = sdy + NC;
-  R* sv = reinterpret_cast<R*>(sdz + NC);      // vx vy vz rx ry rz: 6 planes of NC
-  R* sms = sv + 6 * NC;
-  R* sin_ = sms + NC;
-  int* sglob = reinterpret_cast<int*>(sin_ + NC);
+  R* sv = reinterpret_cast<R*>(sdz + NC);      // vx vy vz [rx ry rz] planes of NC
+  R* sms = sv + C * NC;
+  R* sin_ = sms + NC;                          // ROT: inertia; else the spare fifth plane
+  int* sglob = reinterpret_cast<int*>(sv + (size_t)Kind::NODE_R * NC);
   unsigned char* sown = reinterpret_cast<unsigned char*>(sglob + NC);
   unsigned char* scode = sown + NC;
-  const size_t nodes = (size_t)NC * (6 * sizeof(double) + 8 * sizeof(R) + sizeof(int) + 2);
-  unsigned char* after_nodes = smem_raw + (nodes + 15) / 16 * 16;
-  R* sc_all = reinterpret_cast<R*>(after_nodes);                  // P x 24 x TILE
-  unsigned short* sinc_all = reinterpret_cast<unsigned short*>(sc_all + (size_t)P * 24 * TILE);
-  unsigned char* red_base = reinterpret_cast<unsigned char*>(sinc_all) + ((size_t)P * a.inc_stride * 2 + 15) / 16 * 16;
-  constexpr int NW = TILE / 32;
-  unsigned long long* s_key = reinterpret_cast<unsigned long long*>(red_base) + sub * 4 * NW;
-  unsigned long long* s_bits = s_key + NW;
-  double* s_s0 = reinterpret_cast<double*>(s_bits + NW);
-  double* s_s1 = s_s0 + NW;
-  R* sc = sc_all + (size_t)sub * 24 * TILE;
-  unsigned short* sinc = sinc_all + (size_t)sub * a.inc_stride;
-  // slot numbers of the patch nodes and slot ranges of the held nodes, read once
-  // here instead of from global memory in every cycle
-  int* sslot_all = reinterpret_cast<int*>(red_base + (size_t)persist_groups(TILE) * NW * 32);
-  int* sslot = sslot_all + (size_t)sub * a.nlmax;
-  int2* srange = reinterpret_cast<int2*>(reinterpret_cast<unsigned char*>(sslot_all) +
-                                         ((size_t)P * a.nlmax * sizeof(int) + 15) / 16 * 16);
+  const size_t nodes = (size_t)NC * (6 * sizeof(double) + Kind::NODE_R * sizeof(R) + sizeof(int) + 2);
+  R* sc_all = reinterpret_cast<R*>(smem_raw + (nodes + 15) / 16 * 16);     // corner forces, patch after patch
+  R* sp_all = sc_all + (size_t)P * Kind::CORNER_R;                         // state planes, patch after patch
+  int2* slist = reinterpret_cast<int2*>(sp_all + (size_t)P * Kind::STATE_R);   // list ranges
+  int2* srange = slist + NC;                                                   // slot ranges
+  int* swords = reinterpret_cast<int*>(srange + NC);
 
-  // ---- this CTA's patch and element ----
+  // ---- this CTA's patch and elements ----
   const int p = cta * P + sub;
   const bool has_patch = sub < P && p < a.npatch;
-  const int e = (has_patch ? p : 0) * TILE + lt;
-  PatchInfo pi{};
-  if (has_patch) pi = a.patch[p];
-  const bool active = has_patch && lt < pi.nel;
-  const int NLM = a.nlmax;
-  // ---- stage the held nodes, the incidence lists, the element state ----
+  Kind el;
+  const bool active = el.load(a, pa, zw, p, has_patch, lt, sc_all + (size_t)sub * Kind::CORNER_R,
+                              sp_all + (size_t)sub * Kind::STATE_R);
+  const unsigned lanes = __ballot_sync(0xffffffffu, active);      // of this warp, with elements
+  // ---- stage the held nodes and their lists ----
   const int n0 = pa.node_ofs[cta], nn = pa.node_ofs[cta + 1] - n0;
+  const int nsh = pa.node_nshared[cta];
+  const int w0 = pa.list_ofs[n0], nw = pa.list_ofs[n0 + nn] - w0;
   for (int i = tid; i < nn; i += blockDim.x) {
     const int g = pa.node_glob[n0 + i];
     const double4 xx = na.X[g];
     const R4 vv = na.V[g];
-    const R4 rr = na.VR[g];
     sx[i] = xx.x; sy[i] = xx.y; sz[i] = xx.z;
     sdx[i] = na.DX[g]; sdy[i] = na.DY[g]; sdz[i] = na.DZ[g];
     sv[0 * NC + i] = vv.x; sv[1 * NC + i] = vv.y; sv[2 * NC + i] = vv.z;
-    sv[3 * NC + i] = rr.x; sv[4 * NC + i] = rr.y; sv[5 * NC + i] = rr.z;
+    if constexpr (ROT) {
+      const R4 rr = na.VR[g];
+      sv[3 * NC + i] = rr.x; sv[4 * NC + i] = rr.y; sv[5 * NC + i] = rr.z;
+      sin_[i] = rr.w;
+    }
     sms[i] = R(xx.w);
-    sin_[i] = rr.w;
     sglob[i] = g;
     sown[i] = pa.owner[n0 + i];
     scode[i] = na.code[g];
     srange[i] = make_int2(na.adsky[g], na.adsky[g + 1]);
+    slist[i] = make_int2(pa.list_ofs[n0 + i] - w0, pa.list_ofs[n0 + i + 1] - w0);
   }
-  if (has_patch) {
-    const unsigned* src = reinterpret_cast<const unsigned*>(a.inc + (size_t)p * a.inc_stride);
-    unsigned* dst = reinterpret_cast<unsigned*>(sinc);
-    for (int i = lt; i < a.inc_stride / 2; i += TILE) dst[i] = src[i];
-    for (int j = lt; j < a.patch[p].nloc; j += TILE) sslot[j] = a.patch_slots[p * a.nlmax + j];
-  }
-  ShellState<R, NPT> st;
-  if (KEEP) shell_load_state<R, NPT>(a, e, st);
-  int lc[4] = {0, 0, 0, 0};
-  {
-    const uint2 w = pa.pconn[e];
-    lc[0] = w.x & 0xffffu; lc[1] = w.x >> 16; lc[2] = w.y & 0xffffu; lc[3] = w.y >> 16;
-  }
-  const ShellGroupDesc gd = a.groups[has_patch ? pi.group : 0];
-  const int nl = has_patch ? pi.nloc : 0;
-  // Energies: each thread adds its element's hourglass energy and plastic work over
+  for (int i = tid; i < nw; i += blockDim.x) swords[i] = pa.list[w0 + i];
+  // the thread that carries the CTA's time step to the grid: of the last warp, idle in the
+  // element phase, or of the first if all have elements
+  const bool courier = tid == ((int)blockDim.x > P * NT ? (int)blockDim.x - 32 : 0);
+  const bool reports = tid < P * NT;               // in a warp that hands in a minimum (an empty one too)
+  // Energies: each thread adds its elements' hourglass energy and plastic work over
   // the launch's cycles; the patch sums them once at the end onto its cumulative
   // partials (the phase kernels sum per cycle, so the two agree to FP64 rounding).
   double cum_ehou_t = 0.0, cum_wpla_t = 0.0;
-  if (tid == 0) { s_dt[0] = ~0ull; s_dt[1] = ~0ull; }
+  if (tid == 0) {
+    s_dt[0] = ~0ull; s_dt[1] = ~0ull;
+    s_abort = 0;
+    mbar_init_n(&s_dtbar, (unsigned)(P * NT / 32));
+  }
   PartTime t = na.time[parity0];
   R4* fs[2] = {a.fslot, reinterpret_cast<R4*>(pa.fslot2)};
-  R4* ms_[2] = {a.mslot, reinterpret_cast<R4*>(pa.mslot2)};
+  R4* ms_[2] = {const_cast<R4*>(na.mslot), reinterpret_cast<R4*>(pa.mslot2)};
+  unsigned* const abort = pa.sync + 1;
+  unsigned* const slot_count = pa.sync + SYNC_SLOTS;
   __syncthreads();
+
+  // one patch's partial of a node: its corners from word w on; returns its slot
+  auto partial = [&](int& w, R (&f)[C]) {
+    const int head = swords[w++];
+#pragma unroll
+    for (int q = 0; q < C; ++q) f[q] = R(0);
+    const int end = w + (head & 0xff);
+#pragma unroll 4
+    for (; w < end; ++w) Kind::corner(sc_all, swords[w], f);
+    return head >> 8;
+  };
 
   for (int c = 0; c < ncycles; ++c) {
     R4* fslot = fs[c & 1];
     R4* mslot = ms_[c & 1];
     // ---------------- element phase ----------------
-    const R DT1 = R(t.dt2);
-    R Fg[3][4], Mg[3][4];
-    unsigned long long mykey = ~0ull, mybits = ~0ull;
-    double my_ehou = 0.0, my_wpla = 0.0;
     if (active) {
-      if (!KEEP) shell_load_state<R, NPT>(a, e, st);
-      shell_element<R, NPT, KEEP>(a, e, gd, DT1, zw, sx, sy, sz, sv, NC, lc, st, Fg, Mg, mykey, mybits, my_ehou,
-                                  my_wpla);
-      // corner forces and moments as three planes of pairs (fx fy | fz mx | my mz),
-      // corner k of element lt at k * TILE + lt
-      typename Vec2<R>::T* sc2 = reinterpret_cast<typename Vec2<R>::T*>(sc);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        sc2[(0 * 4 + k) * TILE + lt] = mk2(Fg[0][k], Fg[1][k]);
-        sc2[(1 * 4 + k) * TILE + lt] = mk2(Fg[2][k], Mg[0][k]);
-        sc2[(2 * 4 + k) * TILE + lt] = mk2(Mg[1][k], Mg[2][k]);
-      }
-      cum_ehou_t += my_ehou;
-      cum_wpla_t += my_wpla;
+      auto early = [&](unsigned long long key, unsigned long long bits) {
+        const unsigned long long wk = warp_min_u64(key, lanes), wb = warp_min_u64(bits, lanes);
+        if ((tid & 31) == __ffs(lanes) - 1) {
+          atomicMin(&s_dt[0], wk);
+          atomicMin(&s_dt[1], wb);
+          mbar_arrive(&s_dtbar);
+        }
+      };
+      el.element(a, R(t.dt2), sx, sy, sz, sv, NC, early, cum_ehou_t, cum_wpla_t);
+    } else if (reports && lanes == 0 && (tid & 31) == 0) {
+      mbar_arrive(&s_dtbar);             // a warp without elements
     }
-    {   // the CTA's dt minimum: per warp in registers, then one shared atomic per warp
-      const unsigned long long wk = warp_min_u64(mykey), wb = warp_min_u64(mybits);
-      if ((tid & 31) == 0) { atomicMin(&s_dt[0], wk); atomicMin(&s_dt[1], wb); }
-    }
-    __syncthreads();
-    if (tid == 0) {      // to the grid's reduction at once, ahead of the patch sums
+    if (courier) {
+      bool out = !mbar_wait(&s_dtbar, c & 1, STAGE_WAIT_TRIES);
+      if (out) { atomicExch(abort, 1u); raise_error(a.err, 7, cta); }
       PartAcc* acc = &pa.acc3[c % 3];
       atomicMin(&acc->dtkey, s_dt[0]);
       atomicMin(&acc->dtbits, s_dt[1]);
-      s_dt[0] = ~0ull; s_dt[1] = ~0ull;        // no warp touches them again before the grid barrier
-    }
-    for (int j = lt; j < nl; j += TILE) {
-      R f0 = R(0), f1 = R(0), f2 = R(0), m0 = R(0), m1 = R(0), m2 = R(0);
-      const int i1 = sinc[j + 1];
-      const typename Vec2<R>::T* sc2 = reinterpret_cast<const typename Vec2<R>::T*>(sc);
-#pragma unroll 4
-      for (int i = sinc[j]; i < i1; ++i) {
-        const int o = sinc[NLM + 1 + i];   // corner k of element t: k * TILE + t
-        const typename Vec2<R>::T p0 = sc2[o], p1 = sc2[4 * TILE + o], p2 = sc2[8 * TILE + o];
-        f0 += p0.x; f1 += p0.y; f2 += p1.x;
-        m0 += p1.y; m1 += p2.x; m2 += p2.y;
+      s_dt[0] = ~0ull; s_dt[1] = ~0ull;        // no warp touches them again in this cycle
+      if (!(c == 0 && cta == pa.stall_cta)) grid_arrive(&pa.sync[0]);
+      out = out || grid_wait(&pa.sync[0], (unsigned)(c + 1) * (unsigned)G, abort, a.err);
+      s_acc.dtkey = __ldcg(&acc->dtkey);
+      s_acc.dtbits = __ldcg(&acc->dtbits);
+      if (cta == 0) {      // every CTA arrived here, so all have read the last cycle's: its buffer is cycle c + 2's
+        PartAcc r; r.dtkey = ~0ull; r.dtbits = ~0ull;
+        pa.acc3[(c + 2) % 3] = r;
       }
-      const int s = sslot[j];
-      st_cg(&fslot[s], mk4(f0, f1, f2, R(0)));
-      st_cg(&mslot[s], mk4(m0, m1, m2, R(0)));
+      if (out) s_abort = 1;
     }
-    if (grid_barrier(pa.sync, (unsigned)(c + 1) * (unsigned)G, a.err, &s_abort, !(c == 0 && cta == pa.stall_cta)))
-      return;
-    // ---------------- node phase ----------------
-    // A thread's nodes are i0 = tid + 2 j blockDim.x and i0 + blockDim.x.  The first
-    // two slots of both are loaded before either is summed, and for the first pair
-    // before the cycle's dt reduction is read, so that all these L2 reads are in
-    // flight together.
-    R4 F0[2], F1[2], M0[2], M1[2];
-    int2 rg[2];
-    auto prefetch = [&](int i0) {
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int i = i0 + u * blockDim.x;
-        rg[u] = i < nn ? srange[i] : make_int2(0, 0);
-        F0[u] = F1[u] = M0[u] = M1[u] = mk4(R(0), R(0), R(0), R(0));
-        if (rg[u].y > rg[u].x) { F0[u] = ld_cg(&fslot[rg[u].x]); M0[u] = ld_cg(&mslot[rg[u].x]); }
-        if (rg[u].y > rg[u].x + 1) { F1[u] = ld_cg(&fslot[rg[u].x + 1]); M1[u] = ld_cg(&mslot[rg[u].x + 1]); }
-      }
-    };
-    prefetch(tid);
-    PartAcc ac;
-    ac.dtkey = __ldcg(&pa.acc3[c % 3].dtkey);
-    ac.dtbits = __ldcg(&pa.acc3[c % 3].dtbits);
+    __syncthreads();
+    if (s_abort) return;
+    // ---------------- nodes ----------------
     int ityp, nelt;
     double DT2;
-    cycle_dt(ac, t, na.growth, na.dtmx, na.split, DT2, ityp, nelt);
+    cycle_dt(s_acc, t, na.growth, na.dtmx, na.split, DT2, ityp, nelt);
     const double DTc1 = t.dt2;
     const double DT12 = 0.5 * (DTc1 + DT2);
     const bool last = c == ncycles - 1;
-    for (int i0 = tid; i0 < nn; i0 += 2 * blockDim.x) {
-    if (i0 != tid) prefetch(i0);
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int i = i0 + u * blockDim.x;
-      if (i >= nn) break;
+    auto update = [&](const int i, const R (&f)[C]) {
       const int g = sglob[i];
-      const int k0 = rg[u].x, k1 = rg[u].y;
-      R ax = R(0), ay = R(0), az = R(0), rx = R(0), ry = R(0), rz = R(0);
-      if (k1 > k0) {
-        ax = F0[u].x; ay = F0[u].y; az = F0[u].z;
-        rx = M0[u].x; ry = M0[u].y; rz = M0[u].z;
-      }
-      if (k1 > k0 + 1) {
-        ax += F1[u].x; ay += F1[u].y; az += F1[u].z;
-        rx += M1[u].x; ry += M1[u].y; rz += M1[u].z;
-      }
-      for (int k = k0 + 2; k < k1; ++k) {
-        const R4 f = ld_cg(&fslot[k]);
-        ax += f.x; ay += f.y; az += f.z;
-        const R4 m = ld_cg(&mslot[k]);
-        rx += m.x; ry += m.y; rz += m.z;
-      }
       double px = sx[i], py = sy[i], pz = sz[i], qx = sdx[i], qy = sdy[i], qz = sdz[i];
-      R4 v = mk4(sv[0 * NC + i], sv[1 * NC + i], sv[2 * NC + i], R(0));
-      R4 w = mk4(sv[3 * NC + i], sv[4 * NC + i], sv[5 * NC + i], sin_[i]);
+      R4 v = mk4(sv[0 * NC + i], sv[1 * NC + i], sv[2 * NC + i], R(0)), w = mk4(R(0), R(0), R(0), R(0));
+      R r[3] = {R(0), R(0), R(0)};
+      if constexpr (ROT) {
+        w = mk4(sv[3 * NC + i], sv[4 * NC + i], sv[5 * NC + i], sin_[i]);
+        r[0] = f[3]; r[1] = f[4]; r[2] = f[5];
+      }
       double ek = 0.0, ekr = 0.0;
-      node_update<R>(na, g, scode[i], true, ax, ay, az, rx, ry, rz, sms[i], DTc1, DT2, DT12, px, py, pz, qx, qy, qz,
-                     v, w, ek, ekr, last);        // only the launch's last cycle reports kinetic energy
+      node_update<R>(na, g, scode[i], ROT, f[0], f[1], f[2], r[0], r[1], r[2], sms[i], DTc1, DT2, DT12, px, py, pz, qx,
+                     qy, qz, v, w, ek, ekr, last);        // only the launch's last cycle reports kinetic energy
       sx[i] = px; sy[i] = py; sz[i] = pz; sdx[i] = qx; sdy[i] = qy; sdz[i] = qz;
       sv[0 * NC + i] = v.x; sv[1 * NC + i] = v.y; sv[2 * NC + i] = v.z;
-      sv[3 * NC + i] = w.x; sv[4 * NC + i] = w.y; sv[5 * NC + i] = w.z;
+      if constexpr (ROT) { sv[3 * NC + i] = w.x; sv[4 * NC + i] = w.y; sv[5 * NC + i] = w.z; }
       if (last && sown[i]) { pa.ek_node[g] = ek; pa.ekr_node[g] = ekr; }
+    };
+    // shared nodes: this CTA's patch partials to their slots
+    for (int i = tid; i < nsh; i += blockDim.x) {
+      const int2 lr = slist[i];
+      for (int w = lr.x; w < lr.y;) {
+        R f[C];
+        const int s = partial(w, f);
+        st_cg(&fslot[s], mk4(f[0], f[1], f[2], R(0)));
+        if constexpr (ROT) st_cg(&mslot[s], mk4(f[3], f[4], f[5], R(0)));
+      }
     }
-    }
-    if (cta == 0 && tid == 0) {            // reuse in two cycles: everyone has read it
-      PartAcc r; r.dtkey = ~0ull; r.dtbits = ~0ull;
-      pa.acc3[(c + 2) % 3] = r;
+    __syncthreads();
+    if (tid == 0) grid_arrive(slot_count);
+    // the CTA's own nodes while the shared nodes' slots travel, then those; the own ones by
+    // the threads from the last down, so that the first have the shared ones.  For shells one
+    // loop, so that the node update is in the kernel once: in FP64 they spill less for it.
+    // Hexas do not, and ran 5 % faster with the two phases apart.
+#pragma unroll (ROT ? 1 : 2)
+    for (int shared = 0; shared < 2; ++shared) {
+      if (shared) {
+        if (tid == 0 && grid_wait(slot_count, (unsigned)(c + 1) * (unsigned)G, abort, a.err)) s_abort = 1;
+        __syncthreads();
+        if (s_abort) return;
+      }
+      const int last_node = shared ? nsh - 1 : nn - 1, first_node = shared ? 0 : nsh;
+      const int i0 = shared ? last_node - (nsh - 1 - tid) : last_node - (int)(blockDim.x - 1 - tid);
+      const int dir = shared ? (int)blockDim.x : -(int)blockDim.x;
+      for (int i = i0; i >= first_node && i <= last_node; i += dir) {
+        R f[C];
+#pragma unroll
+        for (int q = 0; q < C; ++q) f[q] = R(0);
+        if (!shared) {
+          const int2 lr = slist[i];
+          for (int w = lr.x; w < lr.y;) {
+            R h[C];
+            const bool first = w == lr.x;
+            partial(w, h);
+#pragma unroll
+            for (int q = 0; q < C; ++q) f[q] = first ? h[q] : f[q] + h[q];
+          }
+        } else {
+          // ASSPAR4: the node's slots in ascending patch order, U read at a time
+          constexpr int U = ROT && sizeof(R) == 8 ? 2 : 4;
+          const int2 rg = srange[i];
+          for (int k = rg.x; k < rg.y; k += U) {
+            R4 F[U], M[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+              if (k + u < rg.y) {
+                F[u] = ld_cg(&fslot[k + u]);
+                if constexpr (ROT) M[u] = ld_cg(&mslot[k + u]);
+              }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              if (k + u >= rg.y) break;
+              const bool first = k + u == rg.x;
+              f[0] = first ? F[u].x : f[0] + F[u].x; f[1] = first ? F[u].y : f[1] + F[u].y;
+              f[2] = first ? F[u].z : f[2] + F[u].z;
+              if constexpr (ROT) {
+                f[3] = first ? M[u].x : f[3] + M[u].x; f[4] = first ? M[u].y : f[4] + M[u].y;
+                f[5] = first ? M[u].z : f[5] + M[u].z;
+              }
+            }
+          }
+        }
+        update(i, f);
+      }
     }
     t.tt = t.tt + DT2; t.dt2 = DT2; t.dt2old = DT2; t.dt1 = DTc1; t.dt12 = DT12;
     t.ncycle = t.ncycle + 1; t.ityptst = ityp; t.neltst = nelt; t.pad = 0;
@@ -394,14 +582,12 @@ shell_persistent_kernel(ShellArgs<R> a, NodeArgs<R> na, PersistArgs pa, int ncyc
     na.X[g] = make_double4(sx[i], sy[i], sz[i], na.X[g].w);
     na.DX[g] = sdx[i]; na.DY[g] = sdy[i]; na.DZ[g] = sdz[i];
     na.V[g] = mk4(sv[0 * NC + i], sv[1 * NC + i], sv[2 * NC + i], R(0));
-    na.VR[g] = mk4(sv[3 * NC + i], sv[4 * NC + i], sv[5 * NC + i], sin_[i]);
+    if constexpr (ROT) na.VR[g] = mk4(sv[3 * NC + i], sv[4 * NC + i], sv[5 * NC + i], sin_[i]);
   }
-  if constexpr (KEEP) {
-    if (has_patch) shell_store_state<R, NPT>(a, e, st);
-  }
-  {
-    unsigned long long k0 = ~0ull, k1 = ~0ull;
-    group_reduce<TILE>(k0, k1, cum_ehou_t, cum_wpla_t, s_key, s_bits, s_s0, s_s1);
+  el.store(a, has_patch);
+  {   // the group's sums, through the corner forces' memory (read for the last time above)
+    double* s_sum = reinterpret_cast<double*>(sc_all) + 2 * (size_t)sub * (NT / 32);
+    group_sums<NT>(cum_ehou_t, cum_wpla_t, s_sum, s_sum + NT / 32);
     if (has_patch && lt == 0) {
       a.blk_ehour[p] = a.blk_ehour[p] + cum_ehou_t;
       a.blk_wpla[p] = a.blk_wpla[p] + cum_wpla_t;
@@ -414,7 +600,13 @@ shell_persistent_kernel(ShellArgs<R> a, NodeArgs<R> na, PersistArgs pa, int ncyc
     a.acc[fin] = r;
   }
   // kinetic energy per node tile of 128, summed as the node pass sums it
-  if (grid_barrier(pa.sync, (unsigned)(ncycles + 1) * (unsigned)G, a.err, &s_abort)) return;
+  __syncthreads();
+  if (tid == 0) {
+    grid_arrive(slot_count);
+    if (grid_wait(slot_count, (unsigned)(ncycles + 1) * (unsigned)G, abort, a.err)) s_abort = 1;
+  }
+  __syncthreads();
+  if (s_abort) return;
   for (int tile = cta; tile < pa.ntiles_node; tile += G) {
     double ek = 0.0, ekr = 0.0;
     if (tid < 128) {
