@@ -492,18 +492,14 @@ struct Impl {
   }
 };
 
-// dynamic shared memory of a patch kernel.  Hexa: the layout of hex_smem_bytes.
-// Shell: for the NPT-point kernels the staged integration-point planes (6 NPT of
-// TILE), then node planes (x, y, z in FP64; velocities and rotational velocities in
-// R), 24 planes of TILE corner forces, the incidence lists.
+// dynamic shared memory of a patch kernel
 template <class R>
 size_t hex_smem(int nl, int tile, int inc_stride) {
   return hex_smem_bytes<R>(nl, tile, inc_stride);
 }
 template <class R>
-size_t shell_smem(int nl, int tile, int inc_stride, int npt = 0) {
-  return (size_t)shell_staged_planes(npt) * tile * sizeof(R) + (size_t)nl * (3 * sizeof(double) + 6 * sizeof(R)) +
-         24 * (size_t)tile * sizeof(R) + 2 * (size_t)inc_stride;
+size_t shell_smem(int nl, int tile, int inc_stride, int staged_npt = 0) {
+  return shell_smem_bytes<R>(nl, tile, inc_stride, staged_npt);
 }
 
 // A cycle kernel launch; with pdl, programmatic stream serialization lets its
@@ -540,9 +536,12 @@ int launch_hex(or_ecycle* h, Impl<R>& m, int parity, bool pdl = false, int secon
 template <class R, int T, int NPT, bool STG>
 int launch_shell(or_ecycle* h, Impl<R>& m, int parity, bool pdl) {
   if (m.sps.info.empty()) return OR_OK;
-  size_t sm = shell_smem<R>(m.sps.nlmax, T, m.sinc_stride, STG ? NPT : 0);
-  CK(launch_k(shell_patch_kernel<R, T, NPT, STG>, (unsigned)m.sps.info.size(), T, sm, h->stream, pdl, m.sargs(),
-              parity, (const float*)m.zw.p));
+  const size_t sm = shell_smem<R>(m.sps.nlmax, T, m.sinc_stride, STG ? NPT : 0);
+  const unsigned g = (unsigned)m.sps.info.size();
+  if constexpr (STG)
+    CK(launch_k(shell_patch_staged_kernel<R, T, NPT>, g, T, sm, h->stream, pdl, m.sargs(), parity, (const float*)m.zw.p));
+  else
+    CK(launch_k(shell_patch_kernel<R, T, NPT>, g, T, sm, h->stream, pdl, m.sargs(), parity, (const float*)m.zw.p));
   h->launches++;
   return OR_OK;
 }
@@ -631,16 +630,16 @@ int set_smem_attrs(or_ecycle* h, Impl<R>& m) {
   CK(set(hex_patch_kernel<R, 64, 1>));
   CK(set(hex_patch_kernel<R, 128, 1>));
   CK(set(hex_patch_kernel<R, 256, 1>));
-  CK(set(shell_patch_kernel<R, 64, 0, false>));
-  CK(set(shell_patch_kernel<R, 128, 0, false>));
-  CK(set(shell_patch_kernel<R, 256, 0, false>));
-  CK(set(shell_patch_kernel<R, 64, 5, false>));
-  CK(set(shell_patch_kernel<R, 128, 5, false>));
-  CK(set(shell_patch_kernel<R, 256, 5, false>));
+  CK(set(shell_patch_kernel<R, 64, 0>));
+  CK(set(shell_patch_kernel<R, 128, 0>));
+  CK(set(shell_patch_kernel<R, 256, 0>));
+  CK(set(shell_patch_kernel<R, 64, 5>));
+  CK(set(shell_patch_kernel<R, 128, 5>));
+  CK(set(shell_patch_kernel<R, 256, 5>));
   if constexpr (sizeof(R) == 4) {
-    CK(set(shell_patch_kernel<R, 64, 5, true>));
-    CK(set(shell_patch_kernel<R, 128, 5, true>));
-    CK(set(shell_patch_kernel<R, 256, 5, true>));
+    CK(set(shell_patch_staged_kernel<R, 64, 5>));
+    CK(set(shell_patch_staged_kernel<R, 128, 5>));
+    CK(set(shell_patch_staged_kernel<R, 256, 5>));
   }
   return OR_OK;
 }

@@ -55,7 +55,7 @@ struct HexGroupDesc {
 };
 static_assert(sizeof(HexGroupDesc) % 16 == 0, "HexGroupDesc is bulk-copied");
 
-struct ShellGroupDesc {
+struct ShellGroupDesc {          // 192 bytes: the staged shell kernel bulk-copies it
   int part, law, nel, npt;
   int ithk, has_jca, ishfram, ipla;   // ipla: M2CPLR return (0 radial, 1 Newton, 2 projection)
   int ihbe, pad;                      // engine IHBE (IPARG(23)): 1, 0, 2 or 4
@@ -63,6 +63,8 @@ struct ShellGroupDesc {
   double hm, hf, hr, shf, pressure, dtfac, dtmin;
   double dn;                          // GEO(17): one-point V-shape hourglass coefficient
 };
+
+static_assert(sizeof(ShellGroupDesc) % 16 == 0, "ShellGroupDesc is bulk-copied");
 
 struct PartDesc {
   int node_start, node_end;  // padded global node range
@@ -1109,17 +1111,45 @@ __device__ __forceinline__ void shell_store_state(const ShellArgs<R>& a, int e, 
   a.thk[e] = st.thk;
   a.hourg[0 * nelpad + e] = st.h[0]; a.hourg[1 * nelpad + e] = st.h[1]; a.hourg[2 * nelpad + e] = st.h[2];
   a.eint[0 * nelpad + e] = st.e[0]; a.eint[1 * nelpad + e] = st.e[1];
-  if (!IP) return;
 #pragma unroll
-  for (int ip = 0; ip < NPT; ++ip) {
+  for (int ip = 0; ip < (IP ? NPT : 0); ++ip) {
 #pragma unroll
     for (int c = 0; c < 5; ++c) a.sig[(ip * 5 + c) * nelpad + e] = st.sig[ip][c];
     a.pla[ip * nelpad + e] = st.pla[ip];
   }
 }
 
-// CCOOR3 (from nodal planes in shared memory: x, y, z in FP64 and vx vy vz rx ry rz
-// in R, stride NLM, corner k at index lc[k]), CNVEC3, CDERI3, CCOEF3, CDLEN3,
+// The nodes of a shell's corners in shared memory: x, y, z in FP64, velocities and
+// rotational velocities in R.  As planes of stride NLM (vx vy vz rx ry rz in sv), or as
+// records that a gather copies whole (positions as (x, y) and z, velocities as R4).
+template <class R>
+struct ShellNodePlanes {
+  const double *sx, *sy, *sz;
+  const R* sv;
+  int NLM;
+  const int (&lc)[4];
+  __device__ __forceinline__ double x(int k) const { return sx[lc[k]]; }
+  __device__ __forceinline__ double y(int k) const { return sy[lc[k]]; }
+  __device__ __forceinline__ double z(int k) const { return sz[lc[k]]; }
+  __device__ __forceinline__ R v(int c, int k) const { return sv[c * NLM + lc[k]]; }     // c: 0..5
+};
+template <class R>
+struct ShellNodeRecords {
+  typedef typename Vec4<R>::T R4;
+  const double2* sxy;
+  const double* sz;
+  const R4 *sv, *sr;
+  const int (&lc)[4];
+  __device__ __forceinline__ double x(int k) const { return sxy[lc[k]].x; }
+  __device__ __forceinline__ double y(int k) const { return sxy[lc[k]].y; }
+  __device__ __forceinline__ double z(int k) const { return sz[lc[k]]; }
+  __device__ __forceinline__ R v(int c, int k) const {
+    const R4 q = (c < 3 ? sv : sr)[lc[k]];
+    return c % 3 == 0 ? q.x : c % 3 == 1 ? q.y : q.z;
+  }
+};
+
+// CCOOR3 (nodes nd of the corners), CNVEC3, CDERI3, CCOEF3, CDLEN3,
 // CDEFO3, CCURV3, CSTRA3, MULAWC (SIGEPS01C / SIGEPS02C -> M2CPLR per
 // integration point), CHVIS3, CDT3, CFINT3, the group pressure; corner forces and
 // moments out in global axes with CUPDT3P signs.  KEEP = false writes the new
@@ -1136,11 +1166,10 @@ __device__ __forceinline__ void shell_store_state(const ShellArgs<R>& a, int e, 
 // its branch ends a basic block, across which the compiler fuses no multiply-add, so that
 // moving it would change the rounding of the patch kernels.
 struct NoEarly {};
-template <class R, int NPT, bool KEEP, bool STAGED = false, bool GEN = NPT == 0, class Early = NoEarly>
+template <class R, int NPT, bool KEEP, bool STAGED = false, bool GEN = NPT == 0, class Early = NoEarly, class Nodes>
 __device__ __forceinline__ void shell_element(const ShellArgs<R>& a, const int e, const ShellGroupDesc& gd,
-                                              const R DT1, const float* __restrict__ zw, const double* sx,
-                                              const double* sy, const double* sz, const R* sv, const int NLM,
-                                              const int (&lc)[4], ShellState<R, NPT>& st, R (&Fg)[3][4],
+                                              const R DT1, const float* __restrict__ zw, const Nodes& nd,
+                                              ShellState<R, NPT>& st, R (&Fg)[3][4],
                                               R (&Mg)[3][4], unsigned long long& mykey, unsigned long long& mybits,
                                               double& my_ehou, double& my_wpla, R* sip = nullptr,
                                               const int sstride = 0, const Early& early = Early()) {
@@ -1149,12 +1178,12 @@ __device__ __forceinline__ void shell_element(const ShellArgs<R>& a, const int e
   const int nelpad = a.nelpad;
   const R OFF = R(1);
   // coordinate differences in FP64, cast to R (CNVEC3 / CDERI3 inputs)
-  const double x1 = sx[lc[0]], y1 = sy[lc[0]], z1 = sz[lc[0]];
-  const R X21 = R(sx[lc[1]] - x1), Y21 = R(sy[lc[1]] - y1), Z21 = R(sz[lc[1]] - z1);
-  const R X31 = R(sx[lc[2]] - x1), Y31 = R(sy[lc[2]] - y1), Z31 = R(sz[lc[2]] - z1);
-  const R X41 = R(sx[lc[3]] - x1), Y41 = R(sy[lc[3]] - y1), Z41 = R(sz[lc[3]] - z1);
-  const R X32 = R(sx[lc[2]] - sx[lc[1]]), Y32 = R(sy[lc[2]] - sy[lc[1]]), Z32 = R(sz[lc[2]] - sz[lc[1]]);
-  const R X34 = R(sx[lc[2]] - sx[lc[3]]), Y34 = R(sy[lc[2]] - sy[lc[3]]), Z34 = R(sz[lc[2]] - sz[lc[3]]);
+  const double x1 = nd.x(0), y1 = nd.y(0), z1 = nd.z(0);
+  const R X21 = R(nd.x(1) - x1), Y21 = R(nd.y(1) - y1), Z21 = R(nd.z(1) - z1);
+  const R X31 = R(nd.x(2) - x1), Y31 = R(nd.y(2) - y1), Z31 = R(nd.z(2) - z1);
+  const R X41 = R(nd.x(3) - x1), Y41 = R(nd.y(3) - y1), Z41 = R(nd.z(3) - z1);
+  const R X32 = R(nd.x(2) - nd.x(1)), Y32 = R(nd.y(2) - nd.y(1)), Z32 = R(nd.z(2) - nd.z(1));
+  const R X34 = R(nd.x(2) - nd.x(3)), Y34 = R(nd.y(2) - nd.y(3)), Z34 = R(nd.z(2) - nd.z(3));
   // ---- CNVEC3, ISHFRAM = 0 (cnvec3.F:66-81) or 2 (cnvec3.F:82-106) ----
   R E1X = X21 + X34, E1Y = Y21 + Y34, E1Z = Z21 + Z34;
   R E2X = X32 + X41, E2Y = Y32 + Y41, E2Z = Z32 + Z41;
@@ -1245,11 +1274,11 @@ __device__ __forceinline__ void shell_element(const ShellArgs<R>& a, const int e
   R VXl[4], VYl[4], VZl[4], RXl[4], RYl[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const R vx = sv[0 * NLM + lc[k]], vy = sv[1 * NLM + lc[k]], vz = sv[2 * NLM + lc[k]];
+    const R vx = nd.v(0, k), vy = nd.v(1, k), vz = nd.v(2, k);
     VXl[k] = E1X * vx + E1Y * vy + E1Z * vz;
     VYl[k] = E2X * vx + E2Y * vy + E2Z * vz;
     VZl[k] = E3X * vx + E3Y * vy + E3Z * vz;
-    const R rx = sv[3 * NLM + lc[k]], ry = sv[4 * NLM + lc[k]], rz = sv[5 * NLM + lc[k]];
+    const R rx = nd.v(3, k), ry = nd.v(4, k), rz = nd.v(5, k);
     RXl[k] = E1X * rx + E1Y * ry + E1Z * rz;
     RYl[k] = E2X * rx + E2Y * ry + E2Z * rz;
   }
@@ -1623,8 +1652,8 @@ __device__ __forceinline__ void shell_element(const ShellArgs<R>& a, const int e
   // the diagonals taken in FP64 and the cross product in R ----
   R PF[3] = {R(0), R(0), R(0)};
   if (gd.pressure != 0.0) {
-    const R ax = R(sx[lc[2]] - x1), ay = R(sy[lc[2]] - y1), az = R(sz[lc[2]] - z1);
-    const R bx = R(sx[lc[3]] - sx[lc[1]]), by = R(sy[lc[3]] - sy[lc[1]]), bz = R(sz[lc[3]] - sz[lc[1]]);
+    const R ax = R(nd.x(2) - x1), ay = R(nd.y(2) - y1), az = R(nd.z(2) - z1);
+    const R bx = R(nd.x(3) - nd.x(1)), by = R(nd.y(3) - nd.y(1)), bz = R(nd.z(3) - nd.z(1));
     const R NX = ay * bz - az * by, NY = az * bx - ax * bz, NZ = ax * by - ay * bx;
     const R AA = -R(gd.pressure) * R(0.125);
     PF[0] = AA * NX; PF[1] = AA * NY; PF[2] = AA * NZ;
@@ -1636,9 +1665,58 @@ __device__ __forceinline__ void shell_element(const ShellArgs<R>& a, const int e
   }
 }
 
-// Shared planes of staged integration-point state of the NPT-point shell patch
-// kernel: 5 stresses and the plastic strain per point (none for the generic kernel).
-__host__ __device__ constexpr int shell_staged_planes(int npt) { return npt > 0 ? 6 * npt : 0; }
+// Dynamic shared memory of the shell patch kernels (R = element precision, nl = nlmax).
+// Without staging: node planes (x, y, z in FP64; velocities and rotational velocities in
+// R), 24 planes of TILE corner forces and moments, the incidence lists.  Staged form, in
+// this order, every block 16-byte aligned:
+//   integration-point planes (5 stresses per point, then the plastic strains)   6 NPT TILE R
+//   conn (uint2)                                                                TILE
+//   24 corner planes of TILE R; planes 0..9 first receive the patch's thk, thke, hourg 1..3,
+//      eint 1..2, jca, elem_id, degen, each thread reading only its own entries before it
+//      writes its own corners there
+//   node x, y (double2) | velocity (R4) | rotational velocity (R4)              NLM each
+//   incidence lists (uint16, inc_stride, a multiple of 8)
+//   node z (double)                                                            NLM
+template <class R>
+__host__ __device__ inline size_t shell_smem_bytes(int nl, int tile, int inc_stride, int staged_npt) {
+  const size_t node = staged_npt ? 16 + 8 * sizeof(R) + 8 : 3 * sizeof(double) + 6 * sizeof(R);
+  return (size_t)(24 + 6 * staged_npt) * tile * sizeof(R) + (staged_npt ? 8 * (size_t)tile : 0) + (size_t)nl * node +
+         2 * (size_t)inc_stride;
+}
+
+// End of a shell patch kernel: each patch node sums its incident corners in ascending
+// (element, corner) order, then the dt minimum and the energy partials.
+template <class R, int TILE>
+__device__ __forceinline__ void shell_patch_end(const ShellArgs<R>& a, const int parity, const int p, const PatchInfo& pi,
+                                                const R* sc, const unsigned short* sinc, const int slot0,
+                                                const int slot1, const double pre_ehour, const double pre_wpla,
+                                                unsigned long long mykey, unsigned long long mybits, double my_ehou,
+                                                double my_wpla) {
+  __shared__ unsigned long long s_key[TILE / 32], s_bits[TILE / 32];
+  __shared__ double s_s0[TILE / 32], s_s1[TILE / 32];
+  const int tid = threadIdx.x, NLM = a.nlmax, nl = pi.nloc;
+  __syncthreads();
+  for (int j = tid; j < nl; j += TILE) {
+    R f0 = R(0), f1 = R(0), f2 = R(0), m0 = R(0), m1 = R(0), m2 = R(0);
+    const int i1 = sinc[j + 1];
+    for (int i = sinc[j]; i < i1; ++i) {
+      const int o = sinc[NLM + 1 + i];     // corner k of element t: k * TILE + t
+      f0 += sc[o]; f1 += sc[4 * TILE + o]; f2 += sc[8 * TILE + o];
+      m0 += sc[12 * TILE + o]; m1 += sc[16 * TILE + o]; m2 += sc[20 * TILE + o];
+    }
+    const int s = j == tid ? slot0 : j == tid + TILE ? slot1 : a.patch_slots[p * NLM + j];
+    a.fslot[s] = mk4(f0, f1, f2, R(0));
+    a.mslot[s] = mk4(m0, m1, m2, R(0));
+  }
+  block_reduce<TILE>(mykey, mybits, my_ehou, my_wpla, s_key, s_bits, s_s0, s_s1);
+  if (tid == 0) {
+    PartAcc* acc = &a.acc[parity * a.nparts + pi.part];
+    atomicMin(&acc->dtkey, mykey);
+    atomicMin(&acc->dtbits, mybits);
+    a.blk_ehour[p] = pre_ehour + my_ehou;
+    a.blk_wpla[p] = pre_wpla + my_wpla;
+  }
+}
 
 // ===========================================================================
 // shell patch kernel
@@ -1646,21 +1724,14 @@ __host__ __device__ constexpr int shell_staged_planes(int npt) { return npt > 0 
 // Per element (thread): CCOOR3, CNVEC3, CDERI3, CCOEF3, CDLEN3, CDEFO3, CCURV3,
 // CSTRA3, MULAWC (SIGEPS01C / SIGEPS02C -> M2CPLR per integration point),
 // CHVIS3, CDT3, CFINT3; forces and moments into shared memory (CUPDT3P signs).
-// NPT > 0: every group of the launch has NPT integration points; their state is
-// loaded up front into registers, or with STG staged in shared memory by bulk
-// copies and read point by point; NPT = 0: generic 1..10 points, read from global
-// memory in the layer loop.
-template <class R, int TILE, int NPT, bool STG>
-__global__ void __launch_bounds__(TILE, min_blocks(STG ? Occupancy<R>::shell_staged : Occupancy<R>::shell, TILE))
+// NPT > 0: every group of the launch has NPT integration points, their state loaded up
+// front into registers; NPT = 0: generic 1..10 points, read from global memory in the
+// layer loop.
+template <class R, int TILE, int NPT>
+__global__ void __launch_bounds__(TILE, min_blocks(Occupancy<R>::shell, TILE))
 shell_patch_kernel(ShellArgs<R> a, int parity, const float* __restrict__ zw) {
   typedef typename Vec4<R>::T R4;
-  // NPT > 0: the patch's integration-point stresses and plastic strains are staged in
-  // NSP shared planes of TILE by bulk copies, read point by point in the layer loop
-  constexpr int NSP = STG ? shell_staged_planes(NPT) : 0;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ unsigned long long s_key[TILE / 32], s_bits[TILE / 32];
-  __shared__ double s_s0[TILE / 32], s_s1[TILE / 32];
-  __shared__ __align__(8) unsigned long long s_bar;
   const int p = blockIdx.x;
   const int tid = threadIdx.x;
   // element index and node-list slots follow from (p, tid) alone (patches padded
@@ -1674,30 +1745,17 @@ shell_patch_kernel(ShellArgs<R> a, int parity, const float* __restrict__ zw) {
   const int slot1 = tid + TILE < NLM ? a.patch_slots[p * NLM + tid + TILE] : -1;
   double pre_ehour = 0.0, pre_wpla = 0.0;
   if (tid == 0) { pre_ehour = a.blk_ehour[p]; pre_wpla = a.blk_wpla[p]; }
-  R* sip = reinterpret_cast<R*>(smem_raw);
-  double* sx = reinterpret_cast<double*>(sip + NSP * TILE);
+  double* sx = reinterpret_cast<double*>(smem_raw);
   double* sy = sx + NLM;
   double* sz = sy + NLM;
   R* sv = reinterpret_cast<R*>(sz + NLM);   // vx vy vz rx ry rz: 6 planes of NLM
   R* sc = sv + 6 * NLM;                     // 24 planes of TILE: component c of corner k at (c*4+k)
   unsigned short* sinc = reinterpret_cast<unsigned short*>(sc + 24 * TILE);
-  const int nelpad = a.nelpad;
   // per-element loads issued before the staging barrier (overlap with the gathers)
   // padding elements (tid >= nel) hold valid state: load unconditionally
-  if (NSP > 0 && tid == 0) {   // written two launches back: issued before the wait
-    mbar_init(&s_bar);
-    const unsigned pl = TILE * sizeof(R);
-    const size_t e0 = (size_t)p * TILE;
-    mbar_expect_tx(&s_bar, NSP * pl);
-#pragma unroll 1
-    for (int q = 0; q < 5 * NPT; ++q) bulk_g2s(sip + q * TILE, a.sig + (size_t)q * nelpad + e0, pl, &s_bar);
-#pragma unroll 1
-    for (int ip = 0; ip < NPT; ++ip)
-      bulk_g2s(sip + (5 * NPT + ip) * TILE, a.pla + (size_t)ip * nelpad + e0, pl, &s_bar);
-  }
   const uint2 cw = a.conn[e];
   ShellState<R, NPT> st;
-  shell_load_state<R, NPT, NSP == 0>(a, e, st);
+  shell_load_state<R, NPT>(a, e, st);
   {
     const unsigned* src = reinterpret_cast<const unsigned*>(a.inc + (size_t)p * a.inc_stride);
     unsigned* dst = reinterpret_cast<unsigned*>(sinc);
@@ -1721,23 +1779,19 @@ shell_patch_kernel(ShellArgs<R> a, int parity, const float* __restrict__ zw) {
   }
   const ShellGroupDesc gd = a.groups[pi.group];
   const bool active = tid < pi.nel;
-  const int nl = pi.nloc;
   const PartTime& tm = a.time[parity * a.nparts + pi.part];
   const R DT1 = R(tm.dt2);
   __syncthreads();
-  if (NSP > 0 && !mbar_wait0(&s_bar, STAGE_WAIT_TRIES)) raise_error(a.err, 7, p);
 
   int lc[4];
-  int color = -1;
   R Fg[3][4], Mg[3][4];
   unsigned long long mykey = ~0ull, mybits = ~0ull;
   double my_ehou = 0.0, my_wpla = 0.0;
   if (active) {
     lc[0] = cw.x & 0xffffu; lc[1] = cw.x >> 16; lc[2] = cw.y & 0xffffu; lc[3] = cw.y >> 16;
-    color = lc[0] >> COLOR_SHIFT;
     lc[0] &= LOCAL_MASK;
-    shell_element<R, NPT, false, (NSP > 0)>(a, e, gd, DT1, zw, sx, sy, sz, sv, NLM, lc, st, Fg, Mg, mykey, mybits,
-                                            my_ehou, my_wpla, sip + tid, TILE);
+    const ShellNodePlanes<R> nd{sx, sy, sz, sv, NLM, lc};
+    shell_element<R, NPT, false>(a, e, gd, DT1, zw, nd, st, Fg, Mg, mykey, mybits, my_ehou, my_wpla);
   }
   // ---- patch assembly: corner forces and moments to shared memory, then each patch
   // node sums its incident corners in ascending (element, corner) order ----
@@ -1751,28 +1805,114 @@ shell_patch_kernel(ShellArgs<R> a, int parity, const float* __restrict__ zw) {
       }
     }
   }
-  (void)color;
-  __syncthreads();
-  for (int j = tid; j < nl; j += TILE) {
-    R f0 = R(0), f1 = R(0), f2 = R(0), m0 = R(0), m1 = R(0), m2 = R(0);
-    const int i1 = sinc[j + 1];
-    for (int i = sinc[j]; i < i1; ++i) {
-      const int o = sinc[NLM + 1 + i];     // corner k of element t: k * TILE + t
-      f0 += sc[o]; f1 += sc[4 * TILE + o]; f2 += sc[8 * TILE + o];
-      m0 += sc[12 * TILE + o]; m1 += sc[16 * TILE + o]; m2 += sc[20 * TILE + o];
-    }
-    const int s = j == tid ? slot0 : j == tid + TILE ? slot1 : a.patch_slots[p * NLM + j];
-    a.fslot[s] = mk4(f0, f1, f2, R(0));
-    a.mslot[s] = mk4(m0, m1, m2, R(0));
-  }
-  block_reduce<TILE>(mykey, mybits, my_ehou, my_wpla, s_key, s_bits, s_s0, s_s1);
+  shell_patch_end<R, TILE>(a, parity, p, pi, sc, sinc, slot0, slot1, pre_ehour, pre_wpla, mykey, mybits, my_ehou, my_wpla);
+}
+
+// The same for patches beyond one wave of the kernel above (NPT points of Ishell 1): the
+// patch's points, the rest of its element state, connectivity, incidence lists and group
+// constants come by bulk copies on an mbarrier, its nodes by asynchronous gathers of whole
+// records, so that no register holds what is in flight and a corner's node is read in four
+// wide loads.  The layer loop reads the points from shared memory one by one.  360,000
+// shells: 59.5 us a pass with the points alone staged and the rest through registers, 55.6 so.
+template <class R, int TILE, int NPT>
+__global__ void __launch_bounds__(TILE, min_blocks(Occupancy<R>::shell_staged, TILE))
+shell_patch_staged_kernel(ShellArgs<R> a, int parity, const float* __restrict__ zw) {
+  typedef typename Vec4<R>::T R4;
+  static_assert(sizeof(R) == 4, "node records are gathered in 16-byte pieces of R4");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(8) unsigned long long s_bar;
+  __shared__ __align__(16) ShellGroupDesc s_gd;
+  const int p = blockIdx.x;
+  const int tid = threadIdx.x;
+  const int NLM = a.nlmax, nelpad = a.nelpad;
+  const size_t e0 = (size_t)p * TILE;
+  const int e = p * TILE + tid;
+  R* sip = reinterpret_cast<R*>(smem_raw);
+  uint2* sconn = reinterpret_cast<uint2*>(sip + 6 * NPT * TILE);
+  R* sc = reinterpret_cast<R*>(sconn + TILE);
+  double2* sxy = reinterpret_cast<double2*>(sc + 24 * TILE);
+  R4* sv = reinterpret_cast<R4*>(sxy + NLM);
+  R4* sr = sv + NLM;
+  unsigned short* sinc = reinterpret_cast<unsigned short*>(sr + NLM);
+  double* sz = reinterpret_cast<double*>(sinc + a.inc_stride);
+  // written two launches back or static: issued before the wait on the previous kernel
   if (tid == 0) {
-    PartAcc* acc = &a.acc[parity * a.nparts + pi.part];
-    atomicMin(&acc->dtkey, mykey);
-    atomicMin(&acc->dtbits, mybits);
-    a.blk_ehour[p] = pre_ehour + my_ehou;
-    a.blk_wpla[p] = pre_wpla + my_wpla;
+    mbar_init(&s_bar);
+    const unsigned pl = TILE * sizeof(R);
+    mbar_expect_tx(&s_bar, (6 * NPT + (a.jca ? 12 : 11)) * pl + 2 * a.inc_stride + (unsigned)sizeof(ShellGroupDesc));
+    auto plane = [&](int q, const void* src) { bulk_g2s(sc + q * TILE, src, pl, &s_bar); };
+    plane(0, a.thk + e0);
+    plane(1, a.thke + e0);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) plane(2 + q, a.hourg + (size_t)q * nelpad + e0);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) plane(5 + q, a.eint + (size_t)q * nelpad + e0);
+    if (a.jca) plane(7, a.jca + e0);
+    plane(8, a.elem_id + e0);
+    plane(9, a.degen + e0);
+    bulk_g2s(sconn, a.conn + e0, 8 * TILE, &s_bar);
+    bulk_g2s(sinc, a.inc + (size_t)p * a.inc_stride, 2 * a.inc_stride, &s_bar);
+#pragma unroll 1
+    for (int q = 0; q < 5 * NPT; ++q) bulk_g2s(sip + q * TILE, a.sig + (size_t)q * nelpad + e0, pl, &s_bar);
+#pragma unroll 1
+    for (int ip = 0; ip < NPT; ++ip)
+      bulk_g2s(sip + (5 * NPT + ip) * TILE, a.pla + (size_t)ip * nelpad + e0, pl, &s_bar);
   }
+  const PatchInfo pi = a.patch[p];
+  if (tid == 0) bulk_g2s(&s_gd, a.groups + pi.group, sizeof(ShellGroupDesc), &s_bar);
+  const int slot0 = tid < NLM ? a.patch_slots[p * NLM + tid] : -1;
+  const int slot1 = tid + TILE < NLM ? a.patch_slots[p * NLM + tid + TILE] : -1;
+  double pre_ehour = 0.0, pre_wpla = 0.0;
+  if (tid == 0) { pre_ehour = a.blk_ehour[p]; pre_wpla = a.blk_wpla[p]; }
+  const int node0 = tid < NLM ? a.patch_nodes[p * NLM + tid] : 0;
+  const int node1 = tid + TILE < NLM ? a.patch_nodes[p * NLM + tid + TILE] : 0;
+  // X, V, VR and the cycle's time come from the previous node pass
+  pdl_wait();
+  pdl_trigger();
+  for (int j = tid; j < NLM; j += TILE) {
+    const int g = j == tid ? node0 : j == tid + TILE ? node1 : a.patch_nodes[p * NLM + j];
+    const double* xg = reinterpret_cast<const double*>(a.X + g);
+    cp_async16(sxy + j, xg);
+    cp_async8(sz + j, xg + 2);
+    cp_async16(sv + j, a.V + g);
+    cp_async16(sr + j, a.VR + g);
+  }
+  const PartTime& tm = a.time[parity * a.nparts + pi.part];
+  const R DT1 = R(tm.dt2);
+  cp_async_wait_all();
+  __syncthreads();   // node gathers of every thread landed; the mbarrier is initialised
+  if (!mbar_wait0(&s_bar, STAGE_WAIT_TRIES)) raise_error(a.err, 7, p);
+
+  unsigned long long mykey = ~0ull, mybits = ~0ull;
+  double my_ehou = 0.0, my_wpla = 0.0;
+  const bool active = tid < pi.nel;
+  R Fg[3][4], Mg[3][4];
+  if (active) {
+    ShellState<R, NPT> st;
+    st.thk = sc[tid]; st.thke = sc[TILE + tid];
+    st.h[0] = sc[2 * TILE + tid]; st.h[1] = sc[3 * TILE + tid]; st.h[2] = sc[4 * TILE + tid];
+    st.e[0] = sc[5 * TILE + tid]; st.e[1] = sc[6 * TILE + tid];
+    st.jca = a.jca ? sc[7 * TILE + tid] : R(0);
+    const uint2 cw = sconn[tid];
+    st.eid = reinterpret_cast<const int*>(sc + 8 * TILE)[tid];
+    st.degen = reinterpret_cast<const int*>(sc + 9 * TILE)[tid];
+    int lc[4];
+    lc[0] = cw.x & LOCAL_MASK; lc[1] = cw.x >> 16; lc[2] = cw.y & 0xffffu; lc[3] = cw.y >> 16;
+    const ShellNodeRecords<R> nd{sxy, sz, sv, sr, lc};
+    shell_element<R, NPT, false, true>(a, e, s_gd, DT1, zw, nd, st, Fg, Mg, mykey, mybits, my_ehou, my_wpla, sip + tid,
+                                       TILE);
+  }
+  if (active) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        sc[(c * 4 + k) * TILE + tid] = Fg[c][k];
+        sc[((c + 3) * 4 + k) * TILE + tid] = Mg[c][k];
+      }
+    }
+  }
+  shell_patch_end<R, TILE>(a, parity, p, pi, sc, sinc, slot0, slot1, pre_ehour, pre_wpla, mykey, mybits, my_ehou, my_wpla);
 }
 
 // ===========================================================================

@@ -201,8 +201,8 @@ struct PersistShell {
     unsigned long long key = ~0ull, bits = ~0ull;
     double h = 0.0, w = 0.0;
     if (!KEEP) shell_load_state<R, NPT>(a, e, st);
-    shell_element<R, NPT, KEEP, PLANES, GEN>(a, e, gd, DT1, zw, sx, sy, sz, sv, NC, lc, st, Fg, Mg, key, bits, h, w, sp,
-                                             TILE, early);
+    const ShellNodePlanes<R> nd{sx, sy, sz, sv, NC, lc};
+    shell_element<R, NPT, KEEP, PLANES, GEN>(a, e, gd, DT1, zw, nd, st, Fg, Mg, key, bits, h, w, sp, TILE, early);
     R2* q = reinterpret_cast<R2*>(sc);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
