@@ -504,9 +504,7 @@ size_t shell_smem(int nl, int tile, int inc_stride, int staged_npt = 0) {
 
 // A cycle kernel launch; with pdl, programmatic stream serialization lets its
 // blocks start before the previous kernel in the stream has finished (the
-// kernels' pdl_wait / pdl_trigger protocol keeps every read ordered).  Only the
-// element and node passes of the regular cycle use it: their alternation is what
-// the protocol relies on.
+// kernels' pdl_wait / pdl_trigger protocol keeps every read ordered).
 template <class... P, class... A>
 cudaError_t launch_k(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, bool pdl,
                      A&&... args) {
@@ -563,31 +561,32 @@ int launch_shell_npt(or_ecycle* h, Impl<R>& m, int parity, bool pdl = false) {
   return launch_shell<R, T, 5, false>(h, m, parity, pdl);
 }
 template <class R>
-int launch_link(or_ecycle* h, Impl<R>& m) {
+int launch_link(or_ecycle* h, Impl<R>& m, bool pdl) {
+  typedef typename Vec4<R>::T R4;
   if (!m.nlinks) return OR_OK;
-  link_kernel<R><<<(unsigned)m.nlinks, LINK_THREADS, 0, h->stream>>>(
-      m.linkd.p, m.link_nodes.p, m.adsky.p, m.fslot.p, m.mslot.p, m.X.p, m.VR.p, m.code.p, m.skew_of.p, m.skw.p,
-      m.link_mean.p);
-  CK(cudaGetLastError());
+  CK(launch_k(link_kernel<R>, (unsigned)m.nlinks, LINK_THREADS, 0, h->stream, pdl, (const LinkDesc*)m.linkd.p,
+              (const int*)m.link_nodes.p, (const int*)m.adsky.p, (const R4*)m.fslot.p, (const R4*)m.mslot.p,
+              (const double4*)m.X.p, (const R4*)m.VR.p, (const unsigned char*)m.code.p, (const int*)m.skew_of.p,
+              (const R*)m.skw.p, m.link_mean.p));
   h->launches++;
   return OR_OK;
 }
 template <class R>
-int launch_rbody(or_ecycle* h, Impl<R>& m, int parity) {
+int launch_rbody(or_ecycle* h, Impl<R>& m, int parity, bool pdl) {
   if (!m.nrb) return OR_OK;
-  rbody_kernel<R><<<(unsigned)m.nrb, RB_THREADS, 0, h->stream>>>(m.nargs(h), parity, m.rbd.p, m.rb_nodes.p, m.rby.p,
-                                                                  m.rb_ek.p, m.rb_ekr.p);
-  CK(cudaGetLastError());
+  CK(launch_k(rbody_kernel<R>, (unsigned)m.nrb, RB_THREADS, 0, h->stream, pdl, m.nargs(h), parity,
+              (const RBodyDesc*)m.rbd.p, (const int*)m.rb_nodes.p, m.rby.p, m.rb_ek.p, m.rb_ekr.p));
   h->launches++;
   return OR_OK;
 }
 template <class R>
-int launch_loads(or_ecycle* h, Impl<R>& m, int parity) {
+int launch_loads(or_ecycle* h, Impl<R>& m, int parity, bool pdl) {
+  typedef typename Vec4<R>::T R4;
   if (!m.nload) return OR_OK;
-  load_kernel<R><<<(unsigned)((m.nload + 127) / 128), 128, 0, h->stream>>>(
-      m.loadd.p, m.nload, m.funcd.p, m.funcx.p, m.funcy.p, m.skw.p, m.time.p, parity, m.nparts, m.X.p, m.V.p, m.VR.p,
-      m.fslot.p, m.mslot.p, m.wacc.p, m.wpend.p);
-  CK(cudaGetLastError());
+  CK(launch_k(load_kernel<R>, (unsigned)((m.nload + 127) / 128), 128, 0, h->stream, pdl, (const LoadDesc*)m.loadd.p,
+              m.nload, (const FuncDesc*)m.funcd.p, (const double*)m.funcx.p, (const double*)m.funcy.p,
+              (const R*)m.skw.p, (const PartTime*)m.time.p, parity, m.nparts, (const double4*)m.X.p, (const R4*)m.V.p,
+              (const R4*)m.VR.p, m.fslot.p, m.mslot.p, m.wacc.p, m.wpend.p));
   h->launches++;
   return OR_OK;
 }
@@ -844,7 +843,7 @@ int launch_cycle(or_ecycle* h, Impl<R>& m, int parity, cudaEvent_t* ev) {
   // per-phase events need the kernels serialised
   const bool pdl = h->pdl && !ev;
   Trace tr(parity ? "cycle (odd)" : "cycle (even)");
-  if ((rc = launch_loads<R>(h, m, parity))) return rc;     // FORCE (resol.F:2847), before the elements
+  if ((rc = launch_loads<R>(h, m, parity, pdl))) return rc;     // FORCE (resol.F:2847), before the elements
   auto hexas = [&](int second) {
     return h->tile_hex == 64 ? launch_hex<R, 64>(h, m, parity, pdl, second)
            : h->tile_hex == 128 ? launch_hex<R, 128>(h, m, parity, pdl, second)
@@ -865,9 +864,9 @@ int launch_cycle(or_ecycle* h, Impl<R>& m, int parity, cudaEvent_t* ev) {
     if ((rc = shells())) return rc;
     if (ev) CK(cudaEventRecord(ev[2], h->stream));
   }
-  rc = launch_link<R>(h, m);
+  rc = launch_link<R>(h, m, pdl);
   if (rc) return rc;
-  rc = launch_rbody<R>(h, m, parity);
+  rc = launch_rbody<R>(h, m, parity, pdl);
   if (rc) return rc;
   rc = launch_node<R>(h, m, parity, pdl);
   if (rc) return rc;

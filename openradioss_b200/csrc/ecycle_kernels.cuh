@@ -234,8 +234,9 @@ __host__ __device__ inline size_t halo_buffer_bytes(int nhalo) {
 // ---------------------------------------------------------------------------
 // helpers
 // ---------------------------------------------------------------------------
-// Programmatic dependent launch.  The cycle's kernels alternate element pass ->
-// node pass, each launched with programmatic stream serialization, so a kernel's
+// Programmatic dependent launch.  The cycle's kernels, element pass -> node pass with loads
+// before and rigid links and bodies between them where the model has any, are each launched
+// with programmatic stream serialization, so a kernel's
 // blocks can start while the previous kernel is still running.  Every kernel
 //  - issues first the loads that do not depend on the previous kernel (data written
 //    two kernels back or earlier, or static),
@@ -2204,12 +2205,13 @@ template <class R>
 __global__ void __launch_bounds__(128)
 load_kernel(const LoadDesc* __restrict__ loads, int nload, const FuncDesc* __restrict__ funcs,
             const double* __restrict__ fx, const double* __restrict__ fy, const R* __restrict__ skews,
-            const PartTime* __restrict__ time, int parity, int nparts, const double4* __restrict__ X,
-            const typename Vec4<R>::T* __restrict__ V, const typename Vec4<R>::T* __restrict__ VR,
-            typename Vec4<R>::T* __restrict__ fslot, typename Vec4<R>::T* __restrict__ mslot,
-            double* __restrict__ wacc, double* __restrict__ wpend) {
+            const PartTime* time, int parity, int nparts, const double4* X, const typename Vec4<R>::T* V,
+            const typename Vec4<R>::T* VR, typename Vec4<R>::T* fslot, typename Vec4<R>::T* mslot, double* wacc,
+            double* wpend) {
   typedef typename Vec4<R>::T R4;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_wait();
+  pdl_trigger();
   if (e >= nload) return;
   const LoadDesc L = loads[e];
   const PartTime t0 = time[parity * nparts + L.part];
@@ -2333,13 +2335,14 @@ constexpr int LINK_THREADS = 128;
 template <class R>
 __global__ void __launch_bounds__(LINK_THREADS)
 link_kernel(const LinkDesc* __restrict__ links, const int* __restrict__ link_nodes, const int* __restrict__ adsky,
-            const typename Vec4<R>::T* __restrict__ fslot, const typename Vec4<R>::T* __restrict__ mslot,
-            const double4* __restrict__ X, const typename Vec4<R>::T* __restrict__ VR,
-            const unsigned char* __restrict__ codes, const int* __restrict__ skew_of, const R* __restrict__ skews,
-            LinkMean* __restrict__ out) {
+            const typename Vec4<R>::T* fslot, const typename Vec4<R>::T* mslot, const double4* X,
+            const typename Vec4<R>::T* VR, const unsigned char* __restrict__ codes, const int* __restrict__ skew_of,
+            const R* __restrict__ skews, LinkMean* out) {
   typedef typename Vec4<R>::T R4;
   __shared__ double s_sum[8][LINK_THREADS / 32];
   const LinkDesc L = links[blockIdx.x];
+  pdl_wait();
+  pdl_trigger();
   double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (L.ic | L.icr) {
     for (int j = threadIdx.x; j < L.count; j += LINK_THREADS) {
@@ -2464,6 +2467,8 @@ rbody_kernel(NodeArgs<R> a, int parity, const RBodyDesc* __restrict__ bodies, co
   __shared__ R s_vm[3];
   __shared__ double s_dt[3];     // DT1, DT2, DT12
   const RBodyDesc B = bodies[blockIdx.x];
+  pdl_wait();
+  pdl_trigger();
   const int M = B.master;
   R* rby = rby_state + 12 * (size_t)blockIdx.x;
   const double4 xm4 = a.X[M];
