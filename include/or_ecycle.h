@@ -334,8 +334,9 @@ int  or_ecycle_device_bytes(or_ecycle* h, long long* bytes);
    fuse a multiply-add in one kernel and not in the other, and the two agree to
    rounding.  ctas, threads: its launch shape (0 when off; either may be NULL).
    One part of hexa groups that fits likewise runs in a persistent form of its own,
-   under the same conditions and switches; it is not reported here (on = 0), and
-   agrees with the per-phase kernels to rounding.
+   under the same conditions and switches; it is not reported here (on = 0).  In
+   FP64 it too performs the per-phase kernels' operations in their order; in the
+   split form the two agree to rounding.
    No counterpart in the reference. */
 int  or_ecycle_persistent_info(or_ecycle* h, int* on, int* ctas, int* threads);
 

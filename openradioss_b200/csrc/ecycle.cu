@@ -653,7 +653,10 @@ int set_smem_attrs(or_ecycle* h, Impl<R>& m) {
 template <class R, int TILE, int MAXT>
 const void* persist_fn_tile(const Impl<R>& m, bool shells, int npt) {
 #define ORB_FN(...) (const void*)cycle_persistent_kernel<__VA_ARGS__, R, MAXT>
-  if (!shells) return m.any_corot ? ORB_FN(PersistHexa<R, 64, 1>) : ORB_FN(PersistHexa<R, 64, 0>);
+  if (!shells) {
+    if constexpr (sizeof(R) == 4) return m.any_corot ? ORB_FN(PersistHexPair<64, 1>) : ORB_FN(PersistHexPair<64, 0>);
+    else return m.any_corot ? ORB_FN(PersistHexa<64, 1>) : ORB_FN(PersistHexa<64, 0>);
+  }
   if (npt == 5 && m.uniform_npt == 5) return ORB_FN(PersistShell<R, TILE, 5, false>);
   if (npt == 5) return ORB_FN(PersistShell<R, TILE, 5, true>);
   if (npt == 3) return ORB_FN(PersistShell<R, TILE, 3, true>);
@@ -694,7 +697,7 @@ int persist_build(or_ecycle* h, Impl<R>& m) {
     return OR_OK;
   const PatchSet& ps = shells ? m.sps : m.hps;
   const int tile = shells ? h->tile_shell : h->tile_hex;
-  const int K = shells ? 4 : 8, NT = shells ? tile : tile / Pack<R>::N;      // corners, threads of a patch
+  const int K = shells ? 4 : 8, NT = shells || sizeof(R) == 8 ? tile : tile / 2;      // corners, threads of a patch
   if (!shells && tile != 64) return OR_OK;       // what the library picks for meshes of this size
   const int corner_r = 24 * tile, node_r = shells ? 8 : 5;                    // Kind::CORNER_R, NODE_R
   const int npatch = (int)ps.info.size();
@@ -758,7 +761,7 @@ int persist_build(or_ecycle* h, Impl<R>& m) {
       const PatchInfo& pi = ps.info[p];
       std::vector<std::vector<int>> corners(pi.nloc);
       for (int t = 0; t < pi.nel; ++t)
-        for (int k = 0; k < K; ++k)        // Kind::offset
+        for (int k = 0; k < K; ++k)        // as Kind::corner reads them
           corners[ps.local[(size_t)(pi.elem0 + t) * K + k] & LOCAL_MASK].push_back(
               (p - c * P) * (shells ? 12 : 24) * tile + k * tile + t);
       for (int j = 0; j < pi.nloc; ++j) {

@@ -497,8 +497,440 @@ __host__ __device__ inline size_t hex_smem_bytes(int nl, int tile, int inc_strid
          (size_t)nl * (16 + 4 * sizeof(R) + 8) + 2 * (size_t)inc_stride;
 }
 
-// Per element (thread): SCOOR3, SDERI3, SDLEN3, SDEFO3, SRHO3, SROTA3, MMAIN ->
-// M1LAW / M2LAW -> MQVISCB, SHVIS3, SFINT3; corner forces into shared memory.
+// SFORC3 of one hexa: SCOOR3, SDERI3, SDLEN3, SDEFO3, SRHO3, SROTA3, MMAIN -> M1LAW / M2LAW
+// -> MQVISCB, SHVIS3, SFINT3.  IO gives the corners' nodes and the state and takes the new
+// state and the corner forces; io.park / io.unpark hold PXH (0..11) and PX, PY, PZ (12..23),
+// needed again only by SFINT3, while the material law runs; io.early(key, bits) hands in the
+// element's time step as soon as it is known.
+template <class R, int CORO, class IO>
+__device__ __forceinline__ void hex_element(const HexGroupDesc& gd, const R DT1, const IO& io, ErrorWord* err,
+                                            unsigned long long& mykey, unsigned long long& mybits, double& my_ehou,
+                                            double& my_wpla) {
+  typedef typename Vec4<R>::T R4;
+  constexpr bool split = sizeof(R) == 4;
+  const int st_eid = io.eid();
+  // ---- SDERI3 in FP64 (sderi3.F:103-149, 264-298): the corner differences of the
+  // pairs 1-7, 2-8, 3-5, 4-6, and the coordinates relative to corner 1 (differences
+  // taken in FP64, then rounded to R: beyond the determinant nothing needs FP64, as in
+  // the reference's -prec=sp build, which forms the inverse Jacobian, the hourglass
+  // vectors and SDLEN3 in my_real) ----
+  double X17, X28, X35, X46, Y17, Y28, Y35, Y46, Z17, Z28, Z35, Z46;
+  R xr[8], yr[8], zr[8];
+  R R11 = R(1), R12 = R(0), R13 = R(0), R21 = R(0), R22 = R(1), R23 = R(0), R31 = R(0), R32 = R(0), R33 = R(1);
+  const bool corot = CORO && gd.jcvt;
+  if (corot) {
+    double XD[8], YD[8], ZD[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      io.x(k, XD[k], YD[k], ZD[k]);
+    }
+    // SRCOOR3 (srcoor3.F, JCVT /= 0, ISORTH = 0): convected frame R = [e1 e2 e3] of
+    // SREPISO3 (FP64 differences, r, s, t in R) and SORTHO3 (three symmetric
+    // corrections, then Gram-Schmidt); coordinates (FP64) and velocities in it
+    const R x17 = R(XD[6] - XD[0]), x28 = R(XD[7] - XD[1]), x35 = R(XD[4] - XD[2]), x46 = R(XD[5] - XD[3]);
+    const R y17 = R(YD[6] - YD[0]), y28 = R(YD[7] - YD[1]), y35 = R(YD[4] - YD[2]), y46 = R(YD[5] - YD[3]);
+    const R z17 = R(ZD[6] - ZD[0]), z28 = R(ZD[7] - ZD[1]), z35 = R(ZD[4] - ZD[2]), z46 = R(ZD[5] - ZD[3]);
+    const R a17 = x17 + x46, a28 = x28 + x35, b17 = y17 + y46, b28 = y28 + y35, c17 = z17 + z46, c28 = z28 + z35;
+    R Ux = x17 + x28 - x35 - x46, Uy = y17 + y28 - y35 - y46, Uz = z17 + z28 - z35 - z46;
+    R Vx = a17 + a28, Vy = b17 + b28, Vz = c17 + c28;
+    R Wx = a17 - a28, Wy = b17 - b28, Wz = c17 - c28;
+    auto unit = [](R& x, R& y, R& z) {
+      R aa = ssqrt(x * x + y * y + z * z);
+      if (aa != R(0)) aa = R(1) / aa;
+      x *= aa; y *= aa; z *= aa;
+    };
+    unit(Ux, Uy, Uz); unit(Vx, Vy, Vz); unit(Wx, Wy, Wz);
+#pragma unroll
+    for (int it = 0; it < 3; ++it) {
+      R e1x = Vy * Wz - Vz * Wy + Ux, e1y = Vz * Wx - Vx * Wz + Uy, e1z = Vx * Wy - Vy * Wx + Uz;
+      R e2x = Wy * Uz - Wz * Uy + Vx, e2y = Wz * Ux - Wx * Uz + Vy, e2z = Wx * Uy - Wy * Ux + Vz;
+      R e3x = Uy * Vz - Uz * Vy + Wx, e3y = Uz * Vx - Ux * Vz + Wy, e3z = Ux * Vy - Uy * Vx + Wz;
+      unit(e1x, e1y, e1z); unit(e2x, e2y, e2z); unit(e3x, e3y, e3z);
+      Ux = e1x; Uy = e1y; Uz = e1z; Vx = e2x; Vy = e2y; Vz = e2z; Wx = e3x; Wy = e3y; Wz = e3z;
+    }
+    R e3x = Uy * Vz - Uz * Vy, e3y = Uz * Vx - Ux * Vz, e3z = Ux * Vy - Uy * Vx;
+    unit(e3x, e3y, e3z);
+    R11 = Ux; R21 = Uy; R31 = Uz;
+    R12 = e3y * Uz - e3z * Uy; R22 = e3z * Ux - e3x * Uz; R32 = e3x * Uy - e3y * Ux;
+    R13 = e3x; R23 = e3y; R33 = e3z;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const double xl = (double)R11 * XD[k] + (double)R21 * YD[k] + (double)R31 * ZD[k];
+      const double yl = (double)R12 * XD[k] + (double)R22 * YD[k] + (double)R32 * ZD[k];
+      const double zl = (double)R13 * XD[k] + (double)R23 * YD[k] + (double)R33 * ZD[k];
+      XD[k] = xl; YD[k] = yl; ZD[k] = zl;
+    }
+    X17 = XD[6] - XD[0]; X28 = XD[7] - XD[1]; X35 = XD[4] - XD[2]; X46 = XD[5] - XD[3];
+    Y17 = YD[6] - YD[0]; Y28 = YD[7] - YD[1]; Y35 = YD[4] - YD[2]; Y46 = YD[5] - YD[3];
+    Z17 = ZD[6] - ZD[0]; Z28 = ZD[7] - ZD[1]; Z35 = ZD[4] - ZD[2]; Z46 = ZD[5] - ZD[3];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) { xr[k] = R(XD[k] - XD[0]); yr[k] = R(YD[k] - YD[0]); zr[k] = R(ZD[k] - ZD[0]); }
+  } else {
+    // corner 1 first, then the pairs, so that at most two corners are held in FP64
+    double x0, y0, z0;
+    io.x(0, x0, y0, z0);
+    xr[0] = R(0); yr[0] = R(0); zr[0] = R(0);
+    auto ld = [&](int k, double& x, double& y, double& z) {
+      io.x(k, x, y, z);
+      xr[k] = R(x - x0); yr[k] = R(y - y0); zr[k] = R(z - z0);
+    };
+    double xk, yk, zk, xm, ym, zm;
+    ld(6, xk, yk, zk);
+    X17 = xk - x0; Y17 = yk - y0; Z17 = zk - z0;
+    ld(1, xm, ym, zm); ld(7, xk, yk, zk);
+    X28 = xk - xm; Y28 = yk - ym; Z28 = zk - zm;
+    ld(2, xm, ym, zm); ld(4, xk, yk, zk);
+    X35 = xk - xm; Y35 = yk - ym; Z35 = zk - zm;
+    ld(3, xm, ym, zm); ld(5, xk, yk, zk);
+    X46 = xk - xm; Y46 = yk - ym; Z46 = zk - zm;
+  }
+  const double J1 = X17 + X28 - X35 - X46, J2 = Y17 + Y28 - Y35 - Y46, J3 = Z17 + Z28 - Z35 - Z46;
+  const double xa = X17 + X46, xb = X28 + X35, ya = Y17 + Y46, yb = Y28 + Y35, za = Z17 + Z46, zb = Z28 + Z35;
+  const double J4 = xa + xb, J5 = ya + yb, J6 = za + zb, J7 = xa - xb, J8 = ya - yb, J9 = za - zb;
+  const double C1 = J5 * J9 - J6 * J8, C4 = J6 * J7 - J4 * J9, C7 = J4 * J8 - J5 * J7;
+  double det = (1.0 / 64.0) * (J1 * C1 + J2 * C4 + J3 * C7);
+  if (!(det > 0.0)) {   // SCHKJABT3: zero or negative volume stops the run
+    raise_error(err, 4, st_eid);
+    det = 1.0;
+  }
+  const R j1 = R(J1), j2 = R(J2), j3 = R(J3), j4 = R(J4), j5 = R(J5), j6 = R(J6), j7 = R(J7), j8 = R(J8), j9 = R(J9);
+  const R dett = R(1.0 / 64.0) / R(det);
+  const R I1 = dett * R(C1), I4 = dett * R(C4), I7 = dett * R(C7);
+  const R I2 = dett * (j3 * j8 - j2 * j9), I5 = dett * (j1 * j9 - j3 * j7), I8 = dett * (j2 * j7 - j1 * j8);
+  const R I3 = dett * (j2 * j6 - j3 * j5), I6 = dett * (j3 * j4 - j1 * j6), I9 = dett * (j1 * j5 - j2 * j4);
+  R PX[4], PY[4], PZ[4];
+  {
+    const R a12 = I1 + I2, a45 = I4 + I5, a78 = I7 + I8;
+    const R b12 = I1 - I2, b45 = I4 - I5, b78 = I7 - I8;
+    PX[0] = -a12 - I3; PY[0] = -a45 - I6; PZ[0] = -a78 - I9;
+    PX[1] = -a12 + I3; PY[1] = -a45 + I6; PZ[1] = -a78 + I9;
+    PX[2] = b12 + I3;  PY[2] = b45 + I6;  PZ[2] = b78 + I9;
+    PX[3] = b12 - I3;  PY[3] = b45 - I6;  PZ[3] = b78 - I9;
+  }
+  // hourglass projections PXiHj (sderi3.F:302-333): modes (+-+-+-+-), (++----++), (+--+-++-);
+  // the mode vectors sum to zero, so relative coordinates give the same products
+  R PXH[4][3];
+  {
+    const R hx1 = xr[0] - xr[1] + xr[2] - xr[3] + xr[4] - xr[5] + xr[6] - xr[7];
+    const R hy1 = yr[0] - yr[1] + yr[2] - yr[3] + yr[4] - yr[5] + yr[6] - yr[7];
+    const R hz1 = zr[0] - zr[1] + zr[2] - zr[3] + zr[4] - zr[5] + zr[6] - zr[7];
+    const R hx2 = xr[0] + xr[1] - xr[2] - xr[3] - xr[4] - xr[5] + xr[6] + xr[7];
+    const R hy2 = yr[0] + yr[1] - yr[2] - yr[3] - yr[4] - yr[5] + yr[6] + yr[7];
+    const R hz2 = zr[0] + zr[1] - zr[2] - zr[3] - zr[4] - zr[5] + zr[6] + zr[7];
+    const R hx3 = xr[0] - xr[1] - xr[2] + xr[3] - xr[4] + xr[5] + xr[6] - xr[7];
+    const R hy3 = yr[0] - yr[1] - yr[2] + yr[3] - yr[4] + yr[5] + yr[6] - yr[7];
+    const R hz3 = zr[0] - zr[1] - zr[2] + zr[3] - zr[4] + zr[5] + zr[6] - zr[7];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      PXH[q][0] = PX[q] * hx1 + PY[q] * hy1 + PZ[q] * hz1;
+      PXH[q][1] = PX[q] * hx2 + PY[q] * hy2 + PZ[q] * hz2;
+      PXH[q][2] = PX[q] * hx3 + PY[q] * hy3 + PZ[q] * hz3;
+    }
+  }
+  const double VOLN_D = det;
+  const R VOLN = R(det);
+  // ---- SDLEN3 / SLEN (sdlen3.F:110-166): 4 V / sqrt(max face (E G - F^2)) ----
+  R AREAM = R(EM20);
+  {
+    const int FC[6][4] = {{0, 1, 2, 3}, {4, 5, 6, 7}, {0, 1, 5, 4}, {1, 2, 6, 5}, {2, 3, 7, 6}, {3, 0, 4, 7}};
+#pragma unroll
+    for (int f = 0; f < 6; ++f) {
+      const R x13 = xr[FC[f][2]] - xr[FC[f][0]], x24 = xr[FC[f][3]] - xr[FC[f][1]];
+      const R y13 = yr[FC[f][2]] - yr[FC[f][0]], y24 = yr[FC[f][3]] - yr[FC[f][1]];
+      const R z13 = zr[FC[f][2]] - zr[FC[f][0]], z24 = zr[FC[f][3]] - zr[FC[f][1]];
+      const R s1 = x13 - x24, t1 = x13 + x24, s2 = y13 - y24, t2 = y13 + y24, s3 = z13 - z24, t3 = z13 + z24;
+      const R E = s1 * s1 + s2 * s2 + s3 * s3, Fm = s1 * t1 + s2 * t2 + s3 * t3, G = t1 * t1 + t2 * t2 + t3 * t3;
+      const R ar = E * G - Fm * Fm;
+      AREAM = ar > AREAM ? ar : AREAM;
+    }
+  }
+  const R DELTAX = R(4) * VOLN / ssqrt(AREAM);
+  // ---- SDEFO3 (sdefo3.F:114-170, JHBE=1) and the hourglass velocity modes of
+  // SHVIS3, from the velocities taken in the corner pairs (1,7) (2,8) (3,5) (4,6)
+  // that share a row of PX: the mode-j sum  sum_k g_jk v_k  with g_jk = s_jk -+ PXH
+  // splits into the sign sum  sum_k s_jk v_k  and  -sum_q PXH[q][j] (v_k1 - v_k2) ----
+  constexpr int sgn[3][8] = {{1, -1, 1, -1, 1, -1, 1, -1}, {1, 1, -1, -1, -1, -1, 1, 1}, {1, -1, -1, 1, -1, 1, 1, -1}};
+  constexpr int h4[8] = {1, -1, 1, -1, -1, 1, -1, 1};
+  constexpr int pk1[4] = {0, 1, 2, 3}, pk2[4] = {6, 7, 4, 5};
+  R DXX = R(0), DYY = R(0), DZZ = R(0), DXY = R(0), DXZ = R(0), DYX = R(0), DYZ = R(0), DZX = R(0), DZY = R(0);
+  R HGX[4] = {R(0), R(0), R(0), R(0)}, HGY[4] = {R(0), R(0), R(0), R(0)}, HGZ[4] = {R(0), R(0), R(0), R(0)};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int k1 = pk1[q], k2 = pk2[q];
+    const R4 v1 = io.v(k1), v2 = io.v(k2);
+    R u1 = v1.x, w1 = v1.y, t1 = v1.z, u2 = v2.x, w2 = v2.y, t2 = v2.z;
+    if (corot) {
+      const R a1 = R11 * u1 + R21 * w1 + R31 * t1, b1 = R12 * u1 + R22 * w1 + R32 * t1, c1 = R13 * u1 + R23 * w1 + R33 * t1;
+      const R a2 = R11 * u2 + R21 * w2 + R31 * t2, b2 = R12 * u2 + R22 * w2 + R32 * t2, c2 = R13 * u2 + R23 * w2 + R33 * t2;
+      u1 = a1; w1 = b1; t1 = c1; u2 = a2; w2 = b2; t2 = c2;
+    }
+    const R dvx = u1 - u2, dvy = w1 - w2, dvz = t1 - t2;
+    DXX += PX[q] * dvx; DYY += PY[q] * dvy; DZZ += PZ[q] * dvz;
+    DXY += PY[q] * dvx; DXZ += PZ[q] * dvx; DYX += PX[q] * dvy;
+    DYZ += PZ[q] * dvy; DZX += PX[q] * dvz; DZY += PY[q] * dvz;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const R s1 = R(sgn[j][k1]), s2 = R(sgn[j][k2]);
+      HGX[j] += s1 * u1 + s2 * u2 - PXH[q][j] * dvx;
+      HGY[j] += s1 * w1 + s2 * w2 - PXH[q][j] * dvy;
+      HGZ[j] += s1 * t1 + s2 * t2 - PXH[q][j] * dvz;
+    }
+    // the 4th mode (+-+--+-+) (shvis3.F:230-232)
+    HGX[3] += R(h4[k1]) * u1 + R(h4[k2]) * u2;
+    HGY[3] += R(h4[k1]) * w1 + R(h4[k2]) * w2;
+    HGZ[3] += R(h4[k1]) * t1 + R(h4[k2]) * t2;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) io.park(3 * q + j, PXH[q][j]);
+  const R DT1D2 = R(0.5) * DT1;
+  const R D4 = DXY + DYX, D5 = DYZ + DZY, D6 = DXZ + DZX;
+  const R WZZ = DT1D2 * (DYX - DXY), WYY = DT1D2 * (DXZ - DZX), WXX = DT1D2 * (DZY - DYZ);
+  // ---- SRHO3 (srho3.F:122-156; FP64 volume ratios in the split form, srho3.F:230-245) ----
+  const R RHO0 = R(gd.rho0);
+  const R rho_old = io.rho();
+  const R VOLO = io.vol0();
+  R DVOL, RHON, AMU;
+  if (split) {
+    const double v0 = io.vol0dp();
+    DVOL = R(VOLN_D - ((double)RHO0 / (double)rho_old) * v0);
+    RHON = R((double)RHO0 * (v0 / VOLN_D));
+    AMU = R(v0 / VOLN_D - 1.0);
+  } else {
+    DVOL = VOLN - (RHO0 / rho_old) * VOLO;
+    RHON = RHO0 * (VOLO / VOLN);
+    AMU = RHON / RHO0 - R(1);
+  }
+  R EINT = io.eint() * VOLO;
+  // ---- SROTA3 Jaumann rotation (srota3.F:81-91) ----
+  const R S1 = io.sig(0), S2 = io.sig(1), S3 = io.sig(2);
+  const R S4 = io.sig(3), S5 = io.sig(4), S6 = io.sig(5);
+  R SG[6];
+  if (corot) {          // SRMALLA3 (srmall3.F): convected-frame stress, not rotated
+    SG[0] = S1; SG[1] = S2; SG[2] = S3; SG[3] = S4; SG[4] = S5; SG[5] = S6;
+  } else {
+    const R q1 = R(2) * S4 * WZZ, q2 = R(2) * S6 * WYY, q3 = R(2) * S5 * WXX;
+    SG[0] = S1 - q1 + q2;
+    SG[1] = S2 + q1 - q3;
+    SG[2] = S3 - q2 + q3;
+    SG[3] = S4 + WZZ * (S1 - S2) + WYY * S5 - WXX * S6;
+    SG[4] = S5 + WXX * (S2 - S3) + WZZ * S6 - WYY * S4;
+    SG[5] = S6 + WYY * (S3 - S1) + WXX * S4 - WZZ * S5;
+  }
+  const R VOL_AVG = VOLN - R(0.5) * DVOL;
+  const R QOLD = io.qvis();
+  const R EPXE = io.pla();
+  // PX, PY, PZ too are needed again only by SFINT3
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    io.park(12 + q, PX[q]);
+    io.park(16 + q, PY[q]);
+    io.park(20 + q, PZ[q]);
+  }
+  // ---- elastic predictor (m1law.F:124-140 / m2law.F:187-200) ----
+  const R OFF = R(1);
+  const R Gs = R(gd.shear) * OFF;
+  const R G1 = DT1 * Gs, G2 = R(2) * G1;
+  const R SSP = ssqrt((R(1.333) * Gs + R(gd.bulk)) / RHO0);
+  {
+    const R P = -R(1.0 / 3.0) * (SG[0] + SG[1] + SG[2]);
+    const R DAV = -R(1.0 / 3.0) * (DXX + DYY + DZZ);
+    SG[0] = SG[0] + P + G2 * (DXX + DAV);
+    SG[1] = SG[1] + P + G2 * (DYY + DAV);
+    SG[2] = SG[2] + P + G2 * (DZZ + DAV);
+    SG[3] = SG[3] + G1 * D4;
+    SG[4] = SG[4] + G1 * D5;
+    SG[5] = SG[5] + G1 * D6;
+  }
+  R DPLA = R(0), SIGY = R(0);
+  if (gd.law == 2) {
+    // ---- M2LAW radial return (m2law.F:197-352), CC=0, FISOKIN=0 ----
+    R AJ2 = R(0.5) * (SG[0] * SG[0] + SG[1] * SG[1] + SG[2] * SG[2]) + SG[3] * SG[3] + SG[4] * SG[4] + SG[5] * SG[5];
+    AJ2 = ssqrt(R(3) * AJ2);
+    {   // MSTRAIN_RATE, ISRATE = 0, total strain rate
+      const R e4 = R(0.5) * D4, e5 = R(0.5) * D5, e6 = R(0.5) * D6;
+      io.put_epsd(ssqrt(DXX * DXX + DYY * DYY + DZZ * DZZ + R(2) * (e4 * e4 + e5 * e5 + e6 * e6)));
+    }
+    const R CA = R(gd.jc_a), CB = R(gd.jc_b), CN = R(gd.jc_n);
+    R AK, QH;
+    if (CN == R(1)) { AK = CA + CB * EPXE; QH = CB; }
+    else if (EPXE > R(0)) {
+      AK = CA + CB * pow_(EPXE, CN);
+      QH = (CN > R(1)) ? CB * CN * pow_(EPXE, CN - R(1)) : CB * CN / pow_(EPXE, R(1) - CN);
+    } else { AK = CA; QH = R(0); }
+    if (R(gd.sigmax) < AK) { AK = R(gd.sigmax); QH = R(0); }
+    SIGY = AK;
+    if (EPXE > R(gd.epsmax)) { AK = R(0); QH = R(0); }
+    R SCALE = AK / (AJ2 > R(EM15) ? AJ2 : R(EM15));
+    SCALE = SCALE < R(1) ? SCALE : R(1);
+    const R den = R(3) * Gs + QH;
+    DPLA = (R(1) - SCALE) * AJ2 / (den > R(EM15) ? den : R(EM15));
+    AK = AK + DPLA * QH;
+    SCALE = AK / (AJ2 > R(EM15) ? AJ2 : R(EM15));
+    SCALE = SCALE < R(1) ? SCALE : R(1);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) SG[c] = SCALE * SG[c];
+    io.put_pla(EPXE + DPLA);
+    SIGY = SIGY > AK ? SIGY : AK;
+  }
+  // ---- MQVISCB (mqviscb.F:139-354) ----
+  R QNEW;
+  const R AL = VOLN > R(0) ? cbrt_(VOLN) : R(0);
+  {
+    const R DD = -DXX - DYY - DZZ;
+    const R AD = DD > R(0) ? DD : R(0);
+    const R QA = R(gd.qa), QB = R(gd.qb);
+    const R QAA = QA * QA * AD;
+    const R QX = QB * SSP + AL * QAA;
+    QNEW = RHON * AD * AL * (QAA * AL + QB * SSP);
+    R SSP_EQ = QX + ssqrt(QX * QX + SSP * SSP);
+    SSP_EQ = SSP_EQ > R(EM20) ? SSP_EQ : R(EM20);
+    const R DTX = R(gd.dtfac) * (DELTAX / SSP_EQ);
+    if ((double)DTX <= gd.dtmin) raise_error(err, 5, st_eid);
+    const double dtd = (double)DTX;
+    mykey = dt_key(dtd, 1, st_eid);
+    mybits = (unsigned long long)__double_as_longlong(dtd);
+    io.early(mykey, mybits);
+  }
+  // ---- pressure and internal energy (m1law.F:172-190 / m2law.F:434-461) ----
+  const R PNEW = R(gd.bulk) * AMU;
+  SG[0] = (SG[0] - PNEW) * OFF; SG[1] = (SG[1] - PNEW) * OFF; SG[2] = (SG[2] - PNEW) * OFF;
+  SG[3] = SG[3] * OFF; SG[4] = SG[4] * OFF; SG[5] = SG[5] * OFF;
+  const R DTA = R(0.5) * DT1;
+  R EINC;
+  if (gd.law == 1) {
+    const R P2 = -(S1 + SG[0] + S2 + SG[1] + S3 + SG[2]) * R(1.0 / 3.0);
+    EINC = VOL_AVG * (DXX * (S1 + SG[0] + P2) + DYY * (S2 + SG[1] + P2) + DZZ * (S3 + SG[2] + P2) +
+                      D4 * (S4 + SG[3]) + D5 * (S5 + SG[4]) + D6 * (S6 + SG[5])) * DTA -
+           R(0.5) * DVOL * (QOLD + QNEW + P2);
+  } else {
+    EINC = VOL_AVG * (DXX * (S1 + SG[0]) + DYY * (S2 + SG[1]) + DZZ * (S3 + SG[2]) +
+                      D4 * (S4 + SG[3]) + D5 * (S5 + SG[4]) + D6 * (S6 + SG[5])) * DTA -
+           R(0.5) * DVOL * (QOLD + QNEW);
+    my_wpla = (double)SIGY * (double)DPLA * (double)VOLN;
+  }
+  const R vdiv = VOLO > R(EM15) ? VOLO : R(EM15);
+  EINT = (EINT + EINC * OFF) / vdiv;
+#pragma unroll
+  for (int c = 0; c < 6; ++c) io.put_sig(c, SG[c]);
+  io.put_eint(EINT);
+  io.put_rho(RHON);
+  io.put_qvis(QNEW);
+  // ---- SHVIS3 Flanagan-Belytschko viscous hourglass (shvis3.F:156-424, JHBE>=1) ----
+  const R CAQ = R(0.25) * OFF * R(gd.qh);
+  R FCL = CAQ * RHON * (AL * AL);   // VOL**TWO_THIRD
+  const R FCQ = FCL * CAQ * R(100);
+  FCL = FCL * SSP;
+  R HX[4], HY[4], HZ[4];
+  {
+    R ehou = R(0);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      HX[j] = HGX[j] * (FCL + fabs(HGX[j]) * FCQ);
+      HY[j] = HGY[j] * (FCL + fabs(HGY[j]) * FCQ);
+      HZ[j] = HGZ[j] * (FCL + fabs(HGZ[j]) * FCQ);
+      ehou += HX[j] * HGX[j] + HY[j] * HGY[j] + HZ[j] * HGZ[j];
+    }
+    my_ehou = (double)(DT1 * ehou);
+  }
+  // ---- SFINT3 (sfint3.F:256-321), antisymmetric pairs 1-7, 2-8, 3-5, 4-6: corner
+  // k1 gets -f_q, corner k2 gets +f_q, added to the hourglass force; the hourglass
+  // force  -sum_j g_jk H_j - h4_k H_4  splits like the mode sums above ----
+  const R s1 = (SG[0] - QNEW) * VOLN, s2 = (SG[1] - QNEW) * VOLN, s3 = (SG[2] - QNEW) * VOLN;
+  const R s4 = SG[3] * VOLN, s5 = SG[4] * VOLN, s6 = SG[5] * VOLN;
+  // all parked values come back before any corner is written
+  R PH[4][3], QX[4], QY[4], QZ[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) PH[q][j] = io.unpark(3 * q + j);
+    QX[q] = io.unpark(12 + q);
+    QY[q] = io.unpark(16 + q);
+    QZ[q] = io.unpark(20 + q);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int k1 = pk1[q], k2 = pk2[q];
+    // common part of the pair: sum_j PXH[q][j] H_j minus the stress term
+    const R ux = PH[q][0] * HX[0] + PH[q][1] * HX[1] + PH[q][2] * HX[2] - (s1 * QX[q] + s4 * QY[q] + s6 * QZ[q]);
+    const R uy = PH[q][0] * HY[0] + PH[q][1] * HY[1] + PH[q][2] * HY[2] - (s2 * QY[q] + s4 * QX[q] + s5 * QZ[q]);
+    const R uz = PH[q][0] * HZ[0] + PH[q][1] * HZ[1] + PH[q][2] * HZ[2] - (s3 * QZ[q] + s6 * QX[q] + s5 * QY[q]);
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+      const int k = side ? k2 : k1;
+      const R sg = side ? R(-1) : R(1);
+      R fx = -R(sgn[0][k]) * HX[0] - R(sgn[1][k]) * HX[1] - R(sgn[2][k]) * HX[2] - R(h4[k]) * HX[3] + sg * ux;
+      R fy = -R(sgn[0][k]) * HY[0] - R(sgn[1][k]) * HY[1] - R(sgn[2][k]) * HY[2] - R(h4[k]) * HY[3] + sg * uy;
+      R fz = -R(sgn[0][k]) * HZ[0] - R(sgn[1][k]) * HZ[1] - R(sgn[2][k]) * HZ[2] - R(h4[k]) * HZ[3] + sg * uz;
+      if (corot) {        // SRROTA3 with R transposed (sforc3.F:1603-1614): back to global axes
+        const R gx = R11 * fx + R12 * fy + R13 * fz;
+        const R gy = R21 * fx + R22 * fy + R23 * fz;
+        const R gz = R31 * fx + R32 * fy + R33 * fz;
+        fx = gx; fy = gy; fz = gz;
+      }
+      io.corner(k, fx, fy, fz);
+    }
+  }
+}
+
+// A thread's hexa in a patch: state staged in shared planes of TILE reals, the new state
+// written to global memory, corner forces and parked values to the shared planes.  A thread
+// reads and writes only its own entries of a plane: it reads its state before it parks over
+// it, and its parked values (volatile, so that the compiler reloads them instead of holding
+// 24 registers across the material law) before it writes corners there.
+template <class R, int TILE>
+struct HexPatchIO {
+  typedef typename Vec4<R>::T R4;
+  const HexArgs<R>& a;
+  R* sc;                        // the corner planes
+  const int* seid;
+  const double* svol0dp;
+  const double2* sxy;
+  const double* sz;
+  const R4* sv;
+  const uint4 cw;
+  const int tid;
+  const size_t e;
+  // local node of corner k (the colour bits of corner 0 masked off)
+  __device__ __forceinline__ int local(int k) const {
+    const unsigned w = k < 2 ? cw.x : k < 4 ? cw.y : k < 6 ? cw.z : cw.w;
+    const int l = (k & 1) ? (int)(w >> 16) : (int)(w & 0xffffu);
+    return k == 0 ? (l & (int)LOCAL_MASK) : l;
+  }
+  __device__ __forceinline__ void x(int k, double& x, double& y, double& z) const {
+    const int l = local(k);
+    const double2 q = sxy[l];
+    x = q.x; y = q.y; z = sz[l];
+  }
+  __device__ __forceinline__ R4 v(int k) const { return sv[local(k)]; }
+  __device__ __forceinline__ int eid() const { return seid[tid]; }
+  __device__ __forceinline__ double vol0dp() const { return svol0dp[tid]; }
+  __device__ __forceinline__ R sig(int c) const { return sc[c * TILE + tid]; }
+  __device__ __forceinline__ R eint() const { return sc[6 * TILE + tid]; }
+  __device__ __forceinline__ R rho() const { return sc[7 * TILE + tid]; }
+  __device__ __forceinline__ R qvis() const { return sc[8 * TILE + tid]; }
+  __device__ __forceinline__ R vol0() const { return sc[9 * TILE + tid]; }
+  __device__ __forceinline__ R pla() const { return sc[10 * TILE + tid]; }
+  __device__ __forceinline__ void put_sig(int c, R v) const { __stcs(a.sig + c * a.nelpad + e, v); }
+  __device__ __forceinline__ void put_eint(R v) const { __stcs(a.eint + e, v); }
+  __device__ __forceinline__ void put_rho(R v) const { __stcs(a.rho + e, v); }
+  __device__ __forceinline__ void put_qvis(R v) const { __stcs(a.qvis + e, v); }
+  __device__ __forceinline__ void put_pla(R v) const { __stcs(a.pla + e, v); }
+  __device__ __forceinline__ void put_epsd(R v) const { a.epsd[e] = v; }
+  __device__ __forceinline__ void early(unsigned long long, unsigned long long) const {}
+  // PXH to the planes 11..22, PX, PY, PZ to 0..10 and 23
+  static __device__ __forceinline__ int plane(int q) { return q < 12 ? 11 + q : q < 23 ? q - 12 : 23; }
+  __device__ __forceinline__ void park(int q, R v) const { *(volatile R*)(sc + plane(q) * TILE + tid) = v; }
+  __device__ __forceinline__ R unpark(int q) const { return *(volatile R*)(sc + plane(q) * TILE + tid); }
+  __device__ __forceinline__ void corner(int k, R fx, R fy, R fz) const {
+    sc[(0 * 8 + k) * TILE + tid] = fx;
+    sc[(1 * 8 + k) * TILE + tid] = fy;
+    sc[(2 * 8 + k) * TILE + tid] = fz;
+  }
+};
+
+// One CTA per patch of TILE hexas, one hexa per thread: staging, hex_element, patch sums.
 // CORO = 1: groups may use the convected frame (JCVT /= 0, decided per group at
 // run time); CORO = 0 compiles that path out (the register budget of the default)
 template <class R, int TILE, int CORO>
@@ -584,391 +1016,8 @@ hex_patch_kernel(HexArgs<R> a, int parity, int second) {
   unsigned long long mykey = ~0ull, mybits = ~0ull;
   double my_ehou = 0.0, my_wpla = 0.0;
   if (active) {
-    const uint4 cw = sconn[tid];
-    // local node of corner k (the colour bits of corner 0 masked off)
-    auto corner = [&](int k) -> int {
-      const unsigned w = k < 2 ? cw.x : k < 4 ? cw.y : k < 6 ? cw.z : cw.w;
-      const int l = (k & 1) ? (int)(w >> 16) : (int)(w & 0xffffu);
-      return k == 0 ? (l & (int)LOCAL_MASK) : l;
-    };
-    const int st_eid = seid[tid];
-    // ---- SDERI3 in FP64 (sderi3.F:103-149, 264-298): the corner differences of the
-    // pairs 1-7, 2-8, 3-5, 4-6, and the coordinates relative to corner 1 (differences
-    // taken in FP64, then rounded to R: beyond the determinant nothing needs FP64, as in
-    // the reference's -prec=sp build, which forms the inverse Jacobian, the hourglass
-    // vectors and SDLEN3 in my_real) ----
-    double X17, X28, X35, X46, Y17, Y28, Y35, Y46, Z17, Z28, Z35, Z46;
-    R xr[8], yr[8], zr[8];
-    R R11 = R(1), R12 = R(0), R13 = R(0), R21 = R(0), R22 = R(1), R23 = R(0), R31 = R(0), R32 = R(0), R33 = R(1);
-    const bool corot = CORO && s_gd.jcvt;
-    if (corot) {
-      double XD[8], YD[8], ZD[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int l = corner(k);
-        const double2 xy = sxy[l];
-        XD[k] = xy.x; YD[k] = xy.y; ZD[k] = sz[l];
-      }
-      // SRCOOR3 (srcoor3.F, JCVT /= 0, ISORTH = 0): convected frame R = [e1 e2 e3] of
-      // SREPISO3 (FP64 differences, r, s, t in R) and SORTHO3 (three symmetric
-      // corrections, then Gram-Schmidt); coordinates (FP64) and velocities in it
-      const R x17 = R(XD[6] - XD[0]), x28 = R(XD[7] - XD[1]), x35 = R(XD[4] - XD[2]), x46 = R(XD[5] - XD[3]);
-      const R y17 = R(YD[6] - YD[0]), y28 = R(YD[7] - YD[1]), y35 = R(YD[4] - YD[2]), y46 = R(YD[5] - YD[3]);
-      const R z17 = R(ZD[6] - ZD[0]), z28 = R(ZD[7] - ZD[1]), z35 = R(ZD[4] - ZD[2]), z46 = R(ZD[5] - ZD[3]);
-      const R a17 = x17 + x46, a28 = x28 + x35, b17 = y17 + y46, b28 = y28 + y35, c17 = z17 + z46, c28 = z28 + z35;
-      R Ux = x17 + x28 - x35 - x46, Uy = y17 + y28 - y35 - y46, Uz = z17 + z28 - z35 - z46;
-      R Vx = a17 + a28, Vy = b17 + b28, Vz = c17 + c28;
-      R Wx = a17 - a28, Wy = b17 - b28, Wz = c17 - c28;
-      auto unit = [](R& x, R& y, R& z) {
-        R aa = ssqrt(x * x + y * y + z * z);
-        if (aa != R(0)) aa = R(1) / aa;
-        x *= aa; y *= aa; z *= aa;
-      };
-      unit(Ux, Uy, Uz); unit(Vx, Vy, Vz); unit(Wx, Wy, Wz);
-#pragma unroll
-      for (int it = 0; it < 3; ++it) {
-        R e1x = Vy * Wz - Vz * Wy + Ux, e1y = Vz * Wx - Vx * Wz + Uy, e1z = Vx * Wy - Vy * Wx + Uz;
-        R e2x = Wy * Uz - Wz * Uy + Vx, e2y = Wz * Ux - Wx * Uz + Vy, e2z = Wx * Uy - Wy * Ux + Vz;
-        R e3x = Uy * Vz - Uz * Vy + Wx, e3y = Uz * Vx - Ux * Vz + Wy, e3z = Ux * Vy - Uy * Vx + Wz;
-        unit(e1x, e1y, e1z); unit(e2x, e2y, e2z); unit(e3x, e3y, e3z);
-        Ux = e1x; Uy = e1y; Uz = e1z; Vx = e2x; Vy = e2y; Vz = e2z; Wx = e3x; Wy = e3y; Wz = e3z;
-      }
-      R e3x = Uy * Vz - Uz * Vy, e3y = Uz * Vx - Ux * Vz, e3z = Ux * Vy - Uy * Vx;
-      unit(e3x, e3y, e3z);
-      R11 = Ux; R21 = Uy; R31 = Uz;
-      R12 = e3y * Uz - e3z * Uy; R22 = e3z * Ux - e3x * Uz; R32 = e3x * Uy - e3y * Ux;
-      R13 = e3x; R23 = e3y; R33 = e3z;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const double xl = (double)R11 * XD[k] + (double)R21 * YD[k] + (double)R31 * ZD[k];
-        const double yl = (double)R12 * XD[k] + (double)R22 * YD[k] + (double)R32 * ZD[k];
-        const double zl = (double)R13 * XD[k] + (double)R23 * YD[k] + (double)R33 * ZD[k];
-        XD[k] = xl; YD[k] = yl; ZD[k] = zl;
-      }
-      X17 = XD[6] - XD[0]; X28 = XD[7] - XD[1]; X35 = XD[4] - XD[2]; X46 = XD[5] - XD[3];
-      Y17 = YD[6] - YD[0]; Y28 = YD[7] - YD[1]; Y35 = YD[4] - YD[2]; Y46 = YD[5] - YD[3];
-      Z17 = ZD[6] - ZD[0]; Z28 = ZD[7] - ZD[1]; Z35 = ZD[4] - ZD[2]; Z46 = ZD[5] - ZD[3];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) { xr[k] = R(XD[k] - XD[0]); yr[k] = R(YD[k] - YD[0]); zr[k] = R(ZD[k] - ZD[0]); }
-    } else {
-      // corner 1 first, then the pairs, so that at most two corners are held in FP64
-      const int l0 = corner(0);
-      const double2 q0 = sxy[l0];
-      const double x0 = q0.x, y0 = q0.y, z0 = sz[l0];
-      xr[0] = R(0); yr[0] = R(0); zr[0] = R(0);
-      auto ld = [&](int k, double& x, double& y, double& z) {
-        const int l = corner(k);
-        const double2 q = sxy[l];
-        x = q.x; y = q.y; z = sz[l];
-        xr[k] = R(x - x0); yr[k] = R(y - y0); zr[k] = R(z - z0);
-      };
-      double xk, yk, zk, xm, ym, zm;
-      ld(6, xk, yk, zk);
-      X17 = xk - x0; Y17 = yk - y0; Z17 = zk - z0;
-      ld(1, xm, ym, zm); ld(7, xk, yk, zk);
-      X28 = xk - xm; Y28 = yk - ym; Z28 = zk - zm;
-      ld(2, xm, ym, zm); ld(4, xk, yk, zk);
-      X35 = xk - xm; Y35 = yk - ym; Z35 = zk - zm;
-      ld(3, xm, ym, zm); ld(5, xk, yk, zk);
-      X46 = xk - xm; Y46 = yk - ym; Z46 = zk - zm;
-    }
-    const double J1 = X17 + X28 - X35 - X46, J2 = Y17 + Y28 - Y35 - Y46, J3 = Z17 + Z28 - Z35 - Z46;
-    const double xa = X17 + X46, xb = X28 + X35, ya = Y17 + Y46, yb = Y28 + Y35, za = Z17 + Z46, zb = Z28 + Z35;
-    const double J4 = xa + xb, J5 = ya + yb, J6 = za + zb, J7 = xa - xb, J8 = ya - yb, J9 = za - zb;
-    const double C1 = J5 * J9 - J6 * J8, C4 = J6 * J7 - J4 * J9, C7 = J4 * J8 - J5 * J7;
-    double det = (1.0 / 64.0) * (J1 * C1 + J2 * C4 + J3 * C7);
-    if (!(det > 0.0)) {   // SCHKJABT3: zero or negative volume stops the run
-      raise_error(a.err, 4, st_eid);
-      det = 1.0;
-    }
-    const R j1 = R(J1), j2 = R(J2), j3 = R(J3), j4 = R(J4), j5 = R(J5), j6 = R(J6), j7 = R(J7), j8 = R(J8), j9 = R(J9);
-    const R dett = R(1.0 / 64.0) / R(det);
-    const R I1 = dett * R(C1), I4 = dett * R(C4), I7 = dett * R(C7);
-    const R I2 = dett * (j3 * j8 - j2 * j9), I5 = dett * (j1 * j9 - j3 * j7), I8 = dett * (j2 * j7 - j1 * j8);
-    const R I3 = dett * (j2 * j6 - j3 * j5), I6 = dett * (j3 * j4 - j1 * j6), I9 = dett * (j1 * j5 - j2 * j4);
-    R PX[4], PY[4], PZ[4];
-    {
-      const R a12 = I1 + I2, a45 = I4 + I5, a78 = I7 + I8;
-      const R b12 = I1 - I2, b45 = I4 - I5, b78 = I7 - I8;
-      PX[0] = -a12 - I3; PY[0] = -a45 - I6; PZ[0] = -a78 - I9;
-      PX[1] = -a12 + I3; PY[1] = -a45 + I6; PZ[1] = -a78 + I9;
-      PX[2] = b12 + I3;  PY[2] = b45 + I6;  PZ[2] = b78 + I9;
-      PX[3] = b12 - I3;  PY[3] = b45 - I6;  PZ[3] = b78 - I9;
-    }
-    // hourglass projections PXiHj (sderi3.F:302-333): modes (+-+-+-+-), (++----++), (+--+-++-);
-    // the mode vectors sum to zero, so relative coordinates give the same products
-    R PXH[4][3];
-    {
-      const R hx1 = xr[0] - xr[1] + xr[2] - xr[3] + xr[4] - xr[5] + xr[6] - xr[7];
-      const R hy1 = yr[0] - yr[1] + yr[2] - yr[3] + yr[4] - yr[5] + yr[6] - yr[7];
-      const R hz1 = zr[0] - zr[1] + zr[2] - zr[3] + zr[4] - zr[5] + zr[6] - zr[7];
-      const R hx2 = xr[0] + xr[1] - xr[2] - xr[3] - xr[4] - xr[5] + xr[6] + xr[7];
-      const R hy2 = yr[0] + yr[1] - yr[2] - yr[3] - yr[4] - yr[5] + yr[6] + yr[7];
-      const R hz2 = zr[0] + zr[1] - zr[2] - zr[3] - zr[4] - zr[5] + zr[6] + zr[7];
-      const R hx3 = xr[0] - xr[1] - xr[2] + xr[3] - xr[4] + xr[5] + xr[6] - xr[7];
-      const R hy3 = yr[0] - yr[1] - yr[2] + yr[3] - yr[4] + yr[5] + yr[6] - yr[7];
-      const R hz3 = zr[0] - zr[1] - zr[2] + zr[3] - zr[4] + zr[5] + zr[6] - zr[7];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        PXH[q][0] = PX[q] * hx1 + PY[q] * hy1 + PZ[q] * hz1;
-        PXH[q][1] = PX[q] * hx2 + PY[q] * hy2 + PZ[q] * hz2;
-        PXH[q][2] = PX[q] * hx3 + PY[q] * hy3 + PZ[q] * hz3;
-      }
-    }
-    const double VOLN_D = det;
-    const R VOLN = R(det);
-    // ---- SDLEN3 / SLEN (sdlen3.F:110-166): 4 V / sqrt(max face (E G - F^2)) ----
-    R AREAM = R(EM20);
-    {
-      const int FC[6][4] = {{0, 1, 2, 3}, {4, 5, 6, 7}, {0, 1, 5, 4}, {1, 2, 6, 5}, {2, 3, 7, 6}, {3, 0, 4, 7}};
-#pragma unroll
-      for (int f = 0; f < 6; ++f) {
-        const R x13 = xr[FC[f][2]] - xr[FC[f][0]], x24 = xr[FC[f][3]] - xr[FC[f][1]];
-        const R y13 = yr[FC[f][2]] - yr[FC[f][0]], y24 = yr[FC[f][3]] - yr[FC[f][1]];
-        const R z13 = zr[FC[f][2]] - zr[FC[f][0]], z24 = zr[FC[f][3]] - zr[FC[f][1]];
-        const R s1 = x13 - x24, t1 = x13 + x24, s2 = y13 - y24, t2 = y13 + y24, s3 = z13 - z24, t3 = z13 + z24;
-        const R E = s1 * s1 + s2 * s2 + s3 * s3, Fm = s1 * t1 + s2 * t2 + s3 * t3, G = t1 * t1 + t2 * t2 + t3 * t3;
-        const R ar = E * G - Fm * Fm;
-        AREAM = ar > AREAM ? ar : AREAM;
-      }
-    }
-    const R DELTAX = R(4) * VOLN / ssqrt(AREAM);
-    // ---- SDEFO3 (sdefo3.F:114-170, JHBE=1) and the hourglass velocity modes of
-    // SHVIS3, from the velocities taken in the corner pairs (1,7) (2,8) (3,5) (4,6)
-    // that share a row of PX: the mode-j sum  sum_k g_jk v_k  with g_jk = s_jk -+ PXH
-    // splits into the sign sum  sum_k s_jk v_k  and  -sum_q PXH[q][j] (v_k1 - v_k2) ----
-    constexpr int sgn[3][8] = {{1, -1, 1, -1, 1, -1, 1, -1}, {1, 1, -1, -1, -1, -1, 1, 1}, {1, -1, -1, 1, -1, 1, 1, -1}};
-    constexpr int h4[8] = {1, -1, 1, -1, -1, 1, -1, 1};
-    constexpr int pk1[4] = {0, 1, 2, 3}, pk2[4] = {6, 7, 4, 5};
-    R DXX = R(0), DYY = R(0), DZZ = R(0), DXY = R(0), DXZ = R(0), DYX = R(0), DYZ = R(0), DZX = R(0), DZY = R(0);
-    R HGX[4] = {R(0), R(0), R(0), R(0)}, HGY[4] = {R(0), R(0), R(0), R(0)}, HGZ[4] = {R(0), R(0), R(0), R(0)};
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int k1 = pk1[q], k2 = pk2[q];
-      const R4 v1 = sv[corner(k1)], v2 = sv[corner(k2)];
-      R u1 = v1.x, w1 = v1.y, t1 = v1.z, u2 = v2.x, w2 = v2.y, t2 = v2.z;
-      if (corot) {
-        const R a1 = R11 * u1 + R21 * w1 + R31 * t1, b1 = R12 * u1 + R22 * w1 + R32 * t1, c1 = R13 * u1 + R23 * w1 + R33 * t1;
-        const R a2 = R11 * u2 + R21 * w2 + R31 * t2, b2 = R12 * u2 + R22 * w2 + R32 * t2, c2 = R13 * u2 + R23 * w2 + R33 * t2;
-        u1 = a1; w1 = b1; t1 = c1; u2 = a2; w2 = b2; t2 = c2;
-      }
-      const R dvx = u1 - u2, dvy = w1 - w2, dvz = t1 - t2;
-      DXX += PX[q] * dvx; DYY += PY[q] * dvy; DZZ += PZ[q] * dvz;
-      DXY += PY[q] * dvx; DXZ += PZ[q] * dvx; DYX += PX[q] * dvy;
-      DYZ += PZ[q] * dvy; DZX += PX[q] * dvz; DZY += PY[q] * dvz;
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const R s1 = R(sgn[j][k1]), s2 = R(sgn[j][k2]);
-        HGX[j] += s1 * u1 + s2 * u2 - PXH[q][j] * dvx;
-        HGY[j] += s1 * w1 + s2 * w2 - PXH[q][j] * dvy;
-        HGZ[j] += s1 * t1 + s2 * t2 - PXH[q][j] * dvz;
-      }
-      // the 4th mode (+-+--+-+) (shvis3.F:230-232)
-      HGX[3] += R(h4[k1]) * u1 + R(h4[k2]) * u2;
-      HGY[3] += R(h4[k1]) * w1 + R(h4[k2]) * w2;
-      HGZ[3] += R(h4[k1]) * t1 + R(h4[k2]) * t2;
-    }
-    // PXH is needed again only by SFINT3: parked in this thread's own entries of the
-    // corner planes 11..22 (free until its corners are written; volatile, so that the
-    // compiler reloads them instead of holding 12 registers across the material law)
-    volatile R* park = sc + 11 * TILE + tid;
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) park[(3 * q + j) * TILE] = PXH[q][j];
-    const R DT1D2 = R(0.5) * DT1;
-    const R D4 = DXY + DYX, D5 = DYZ + DZY, D6 = DXZ + DZX;
-    const R WZZ = DT1D2 * (DYX - DXY), WYY = DT1D2 * (DXZ - DZX), WXX = DT1D2 * (DZY - DYZ);
-    // ---- SRHO3 (srho3.F:122-156; FP64 volume ratios in the split form, srho3.F:230-245) ----
-    const R RHO0 = R(s_gd.rho0);
-    const R rho_old = sc[7 * TILE + tid];
-    const R VOLO = sc[9 * TILE + tid];
-    R DVOL, RHON, AMU;
-    if (split) {
-      const double v0 = svol0dp[tid];
-      DVOL = R(VOLN_D - ((double)RHO0 / (double)rho_old) * v0);
-      RHON = R((double)RHO0 * (v0 / VOLN_D));
-      AMU = R(v0 / VOLN_D - 1.0);
-    } else {
-      DVOL = VOLN - (RHO0 / rho_old) * VOLO;
-      RHON = RHO0 * (VOLO / VOLN);
-      AMU = RHON / RHO0 - R(1);
-    }
-    R EINT = sc[6 * TILE + tid] * VOLO;
-    // ---- SROTA3 Jaumann rotation (srota3.F:81-91) ----
-    const R S1 = sc[0 * TILE + tid], S2 = sc[1 * TILE + tid], S3 = sc[2 * TILE + tid];
-    const R S4 = sc[3 * TILE + tid], S5 = sc[4 * TILE + tid], S6 = sc[5 * TILE + tid];
-    R SG[6];
-    if (corot) {          // SRMALLA3 (srmall3.F): convected-frame stress, not rotated
-      SG[0] = S1; SG[1] = S2; SG[2] = S3; SG[3] = S4; SG[4] = S5; SG[5] = S6;
-    } else {
-      const R q1 = R(2) * S4 * WZZ, q2 = R(2) * S6 * WYY, q3 = R(2) * S5 * WXX;
-      SG[0] = S1 - q1 + q2;
-      SG[1] = S2 + q1 - q3;
-      SG[2] = S3 - q2 + q3;
-      SG[3] = S4 + WZZ * (S1 - S2) + WYY * S5 - WXX * S6;
-      SG[4] = S5 + WXX * (S2 - S3) + WZZ * S6 - WYY * S4;
-      SG[5] = S6 + WYY * (S3 - S1) + WXX * S4 - WZZ * S5;
-    }
-    const R VOL_AVG = VOLN - R(0.5) * DVOL;
-    const R QOLD = sc[8 * TILE + tid];
-    const R EPXE = sc[10 * TILE + tid];
-    // the state planes 0..10 are read: PX, PY, PZ (needed again only by SFINT3) are
-    // parked in this thread's entries of planes 0..10 and 23 likewise
-    volatile R* park2 = sc + tid;
-    constexpr int pplane[12] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 23};
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      park2[pplane[q] * TILE] = PX[q];
-      park2[pplane[4 + q] * TILE] = PY[q];
-      park2[pplane[8 + q] * TILE] = PZ[q];
-    }
-    // ---- elastic predictor (m1law.F:124-140 / m2law.F:187-200) ----
-    const R OFF = R(1);
-    const R Gs = R(s_gd.shear) * OFF;
-    const R G1 = DT1 * Gs, G2 = R(2) * G1;
-    const R SSP = ssqrt((R(1.333) * Gs + R(s_gd.bulk)) / RHO0);
-    {
-      const R P = -R(1.0 / 3.0) * (SG[0] + SG[1] + SG[2]);
-      const R DAV = -R(1.0 / 3.0) * (DXX + DYY + DZZ);
-      SG[0] = SG[0] + P + G2 * (DXX + DAV);
-      SG[1] = SG[1] + P + G2 * (DYY + DAV);
-      SG[2] = SG[2] + P + G2 * (DZZ + DAV);
-      SG[3] = SG[3] + G1 * D4;
-      SG[4] = SG[4] + G1 * D5;
-      SG[5] = SG[5] + G1 * D6;
-    }
-    R DPLA = R(0), SIGY = R(0);
-    if (s_gd.law == 2) {
-      // ---- M2LAW radial return (m2law.F:197-352), CC=0, FISOKIN=0 ----
-      R AJ2 = R(0.5) * (SG[0] * SG[0] + SG[1] * SG[1] + SG[2] * SG[2]) + SG[3] * SG[3] + SG[4] * SG[4] + SG[5] * SG[5];
-      AJ2 = ssqrt(R(3) * AJ2);
-      {   // MSTRAIN_RATE, ISRATE = 0, total strain rate
-        const R e4 = R(0.5) * D4, e5 = R(0.5) * D5, e6 = R(0.5) * D6;
-        a.epsd[e] = ssqrt(DXX * DXX + DYY * DYY + DZZ * DZZ + R(2) * (e4 * e4 + e5 * e5 + e6 * e6));
-      }
-      const R CA = R(s_gd.jc_a), CB = R(s_gd.jc_b), CN = R(s_gd.jc_n);
-      R AK, QH;
-      if (CN == R(1)) { AK = CA + CB * EPXE; QH = CB; }
-      else if (EPXE > R(0)) {
-        AK = CA + CB * pow_(EPXE, CN);
-        QH = (CN > R(1)) ? CB * CN * pow_(EPXE, CN - R(1)) : CB * CN / pow_(EPXE, R(1) - CN);
-      } else { AK = CA; QH = R(0); }
-      if (R(s_gd.sigmax) < AK) { AK = R(s_gd.sigmax); QH = R(0); }
-      SIGY = AK;
-      if (EPXE > R(s_gd.epsmax)) { AK = R(0); QH = R(0); }
-      R SCALE = AK / (AJ2 > R(EM15) ? AJ2 : R(EM15));
-      SCALE = SCALE < R(1) ? SCALE : R(1);
-      const R den = R(3) * Gs + QH;
-      DPLA = (R(1) - SCALE) * AJ2 / (den > R(EM15) ? den : R(EM15));
-      AK = AK + DPLA * QH;
-      SCALE = AK / (AJ2 > R(EM15) ? AJ2 : R(EM15));
-      SCALE = SCALE < R(1) ? SCALE : R(1);
-#pragma unroll
-      for (int c = 0; c < 6; ++c) SG[c] = SCALE * SG[c];
-      __stcs(a.pla + e, EPXE + DPLA);
-      SIGY = SIGY > AK ? SIGY : AK;
-    }
-    // ---- MQVISCB (mqviscb.F:139-354) ----
-    R QNEW;
-    const R AL = VOLN > R(0) ? cbrt_(VOLN) : R(0);
-    {
-      const R DD = -DXX - DYY - DZZ;
-      const R AD = DD > R(0) ? DD : R(0);
-      const R QA = R(s_gd.qa), QB = R(s_gd.qb);
-      const R QAA = QA * QA * AD;
-      const R QX = QB * SSP + AL * QAA;
-      QNEW = RHON * AD * AL * (QAA * AL + QB * SSP);
-      R SSP_EQ = QX + ssqrt(QX * QX + SSP * SSP);
-      SSP_EQ = SSP_EQ > R(EM20) ? SSP_EQ : R(EM20);
-      const R DTX = R(s_gd.dtfac) * (DELTAX / SSP_EQ);
-      if ((double)DTX <= s_gd.dtmin) raise_error(a.err, 5, st_eid);
-      const double dtd = (double)DTX;
-      mykey = dt_key(dtd, 1, st_eid);
-      mybits = (unsigned long long)__double_as_longlong(dtd);
-    }
-    // ---- pressure and internal energy (m1law.F:172-190 / m2law.F:434-461) ----
-    const R PNEW = R(s_gd.bulk) * AMU;
-    SG[0] = (SG[0] - PNEW) * OFF; SG[1] = (SG[1] - PNEW) * OFF; SG[2] = (SG[2] - PNEW) * OFF;
-    SG[3] = SG[3] * OFF; SG[4] = SG[4] * OFF; SG[5] = SG[5] * OFF;
-    const R DTA = R(0.5) * DT1;
-    R EINC;
-    if (s_gd.law == 1) {
-      const R P2 = -(S1 + SG[0] + S2 + SG[1] + S3 + SG[2]) * R(1.0 / 3.0);
-      EINC = VOL_AVG * (DXX * (S1 + SG[0] + P2) + DYY * (S2 + SG[1] + P2) + DZZ * (S3 + SG[2] + P2) +
-                        D4 * (S4 + SG[3]) + D5 * (S5 + SG[4]) + D6 * (S6 + SG[5])) * DTA -
-             R(0.5) * DVOL * (QOLD + QNEW + P2);
-    } else {
-      EINC = VOL_AVG * (DXX * (S1 + SG[0]) + DYY * (S2 + SG[1]) + DZZ * (S3 + SG[2]) +
-                        D4 * (S4 + SG[3]) + D5 * (S5 + SG[4]) + D6 * (S6 + SG[5])) * DTA -
-             R(0.5) * DVOL * (QOLD + QNEW);
-      my_wpla = (double)SIGY * (double)DPLA * (double)VOLN;
-    }
-    const R vdiv = VOLO > R(EM15) ? VOLO : R(EM15);
-    EINT = (EINT + EINC * OFF) / vdiv;
-#pragma unroll
-    for (int c = 0; c < 6; ++c) __stcs(a.sig + c * nelpad + e, SG[c]);
-    __stcs(a.eint + e, EINT);
-    __stcs(a.rho + e, RHON);
-    __stcs(a.qvis + e, QNEW);
-    // ---- SHVIS3 Flanagan-Belytschko viscous hourglass (shvis3.F:156-424, JHBE>=1) ----
-    const R CAQ = R(0.25) * OFF * R(s_gd.qh);
-    R FCL = CAQ * RHON * (AL * AL);   // VOL**TWO_THIRD
-    const R FCQ = FCL * CAQ * R(100);
-    FCL = FCL * SSP;
-    R HX[4], HY[4], HZ[4];
-    {
-      R ehou = R(0);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        HX[j] = HGX[j] * (FCL + fabs(HGX[j]) * FCQ);
-        HY[j] = HGY[j] * (FCL + fabs(HGY[j]) * FCQ);
-        HZ[j] = HGZ[j] * (FCL + fabs(HGZ[j]) * FCQ);
-        ehou += HX[j] * HGX[j] + HY[j] * HGY[j] + HZ[j] * HGZ[j];
-      }
-      my_ehou = (double)(DT1 * ehou);
-    }
-    // ---- SFINT3 (sfint3.F:256-321), antisymmetric pairs 1-7, 2-8, 3-5, 4-6: corner
-    // k1 gets -f_q, corner k2 gets +f_q, added to the hourglass force; the hourglass
-    // force  -sum_j g_jk H_j - h4_k H_4  splits like the mode sums above ----
-    const R s1 = (SG[0] - QNEW) * VOLN, s2 = (SG[1] - QNEW) * VOLN, s3 = (SG[2] - QNEW) * VOLN;
-    const R s4 = SG[3] * VOLN, s5 = SG[4] * VOLN, s6 = SG[5] * VOLN;
-    // PXH, PX, PY, PZ back from their parking planes, before any corner is written
-    R PH[4][3], QX[4], QY[4], QZ[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-#pragma unroll
-      for (int j = 0; j < 3; ++j) PH[q][j] = park[(3 * q + j) * TILE];
-      QX[q] = park2[pplane[q] * TILE];
-      QY[q] = park2[pplane[4 + q] * TILE];
-      QZ[q] = park2[pplane[8 + q] * TILE];
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int k1 = pk1[q], k2 = pk2[q];
-      // common part of the pair: sum_j PXH[q][j] H_j minus the stress term
-      const R ux = PH[q][0] * HX[0] + PH[q][1] * HX[1] + PH[q][2] * HX[2] - (s1 * QX[q] + s4 * QY[q] + s6 * QZ[q]);
-      const R uy = PH[q][0] * HY[0] + PH[q][1] * HY[1] + PH[q][2] * HY[2] - (s2 * QY[q] + s4 * QX[q] + s5 * QZ[q]);
-      const R uz = PH[q][0] * HZ[0] + PH[q][1] * HZ[1] + PH[q][2] * HZ[2] - (s3 * QZ[q] + s6 * QX[q] + s5 * QY[q]);
-#pragma unroll
-      for (int side = 0; side < 2; ++side) {
-        const int k = side ? k2 : k1;
-        const R sg = side ? R(-1) : R(1);
-        R fx = -R(sgn[0][k]) * HX[0] - R(sgn[1][k]) * HX[1] - R(sgn[2][k]) * HX[2] - R(h4[k]) * HX[3] + sg * ux;
-        R fy = -R(sgn[0][k]) * HY[0] - R(sgn[1][k]) * HY[1] - R(sgn[2][k]) * HY[2] - R(h4[k]) * HY[3] + sg * uy;
-        R fz = -R(sgn[0][k]) * HZ[0] - R(sgn[1][k]) * HZ[1] - R(sgn[2][k]) * HZ[2] - R(h4[k]) * HZ[3] + sg * uz;
-        if (corot) {        // SRROTA3 with R transposed (sforc3.F:1603-1614): back to global axes
-          const R gx = R11 * fx + R12 * fy + R13 * fz;
-          const R gy = R21 * fx + R22 * fy + R23 * fz;
-          const R gz = R31 * fx + R32 * fy + R33 * fz;
-          fx = gx; fy = gy; fz = gz;
-        }
-        // planes 0..10 held this thread's own state, read above
-        sc[(0 * 8 + k) * TILE + tid] = fx;
-        sc[(1 * 8 + k) * TILE + tid] = fy;
-        sc[(2 * 8 + k) * TILE + tid] = fz;
-      }
-    }
+    const HexPatchIO<R, TILE> io{a, sc, seid, svol0dp, sxy, sz, sv, sconn[tid], tid, (size_t)e};
+    hex_element<R, CORO>(s_gd, DT1, io, a.err, mykey, mybits, my_ehou, my_wpla);
   }
   // ---- patch assembly: each patch node sums its incident corners in ascending
   // (element, corner) order ----

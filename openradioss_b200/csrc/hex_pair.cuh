@@ -1,13 +1,12 @@
-// hex_element.cuh -- the SFORC3 chain of the 8-node 1-point hexa as the persistent cycle
-// runs it, one thread's share.
+// hex_pair.cuh -- the SFORC3 chain of two 8-node 1-point hexas at once in the split form,
+// for the persistent cycle.
 //
-// In the split form a thread computes two hexas of a patch at once, one in each half of
-// the packed FP32 type F2 (sm_100 add/mul/fma.f32x2): a packed instruction does both
-// elements' arithmetic in one issue slot at the same lane throughput (measured 126
-// lane-operations per clock and SM against 122 scalar).  Each half rounds exactly like the
-// scalar instruction.  In FP64 a thread computes one hexa.  Against hex_patch_kernel the
-// sums over corners and the face areas are arranged in fewer operations (below), so the
-// two agree to rounding.
+// A thread computes two hexas of a patch, one in each half of the packed FP32 type F2
+// (sm_100 add/mul/fma.f32x2): a packed instruction does both elements' arithmetic in one
+// issue slot at the same lane throughput (measured 126 lane-operations per clock and SM
+// against 122 scalar), and a CTA holds twice the hexas of one per thread.  Each half rounds
+// exactly like the scalar instruction.  Against hex_element the sums over corners and the
+// face areas are arranged in fewer operations (below), so the two agree to rounding.
 #pragma once
 
 namespace orb {
@@ -56,13 +55,11 @@ __device__ __forceinline__ F2 operator-(F2 a, F2 b) {
   asm(ORB_F2("sub.rn") "%0, %1, %2;" : "=l"(r.u) : "l"(a.u), "l"(b.u));
   return r;
 }
-__device__ __forceinline__ double fma_(double a, double b, double c) { return a * b + c; }   // contracted by the compiler
 // a b - c d (a packed negation costs two instructions, a subtraction one)
-template <class W> __device__ __forceinline__ W mul_sub(W a, W b, W c, W d) { return a * b - c * d; }
+__device__ __forceinline__ F2 mul_sub(F2 a, F2 b, F2 c, F2 d) { return a * b - c * d; }
 
-// The values of a thread's N hexas in precision R.
-template <class R> struct Pack;
-template <> struct Pack<float> {
+// the values of a thread's two hexas
+struct Pair {
   typedef F2 W;
   static constexpr int N = 2;
   static __device__ __forceinline__ F2 of(const float (&a)[2]) { return f2(a[0], a[1]); }
@@ -70,30 +67,23 @@ template <> struct Pack<float> {
   static __device__ __forceinline__ float get(F2 a, int i) { return f2_get(a, i); }
   template <class F> static __device__ __forceinline__ F2 map(F f) { return f2(f(0), f(1)); }
 };
-template <> struct Pack<double> {
-  typedef double W;
-  static constexpr int N = 1;
-  static __device__ __forceinline__ double of(const double (&a)[1]) { return a[0]; }
-  static __device__ __forceinline__ double all(double a) { return a; }
-  static __device__ __forceinline__ double get(double a, int) { return a; }
-  template <class F> static __device__ __forceinline__ double map(F f) { return f(0); }
-};
 
 // SCOOR3 / SRCOOR3 and the FP64 part of SDERI3 (sderi3.F:103-149, 264-298) of one hexa:
 // the corner differences of the pairs 1-7, 2-8, 3-5, 4-6 and the coordinates relative to
 // corner 1 are taken in FP64, then rounded to R: beyond the determinant nothing needs
 // FP64, as in the reference's -prec=sp build, which forms the inverse Jacobian, the
 // hourglass vectors and SDLEN3 in my_real.
-template <class R>
 struct HexGeom {
+  typedef float R;
   R x[8][3];        // relative to corner 1 (x[0] = 0)
   R j[9];           // Jacobian terms
   R c[3];           // first cofactors
   double det;       // volume
   R fr[9];          // convected frame, columns e1 e2 e3 (CORO)
 };
-template <class R, int CORO, class IO>
-__device__ __forceinline__ void hex_geometry(const IO& io, const int i, const bool corot, HexGeom<R>& g) {
+template <int CORO, class IO>
+__device__ __forceinline__ void hex_geometry(const IO& io, const int i, const bool corot, HexGeom& g) {
+  typedef float R;
   double X17, X28, X35, X46, Y17, Y28, Y35, Y46, Z17, Z28, Z35, Z46;
   if (CORO && corot) {
     double XD[8], YD[8], ZD[8];
@@ -181,9 +171,9 @@ __device__ __forceinline__ void hex_geometry(const IO& io, const int i, const bo
 }
 
 // M2LAW's yield stress and hardening slope at plastic strain e (m2law.F:204-226)
-template <class R>
-__device__ __forceinline__ void hex_yield(const R e, const R CA, const R CB, const R CN, const R sigmax, const R epsmax,
-                                          R& AK, R& QH, R& SIGY) {
+__device__ __forceinline__ void hex_yield(const float e, const float CA, const float CB, const float CN, const float sigmax, const float epsmax,
+                                          float& AK, float& QH, float& SIGY) {
+  typedef float R;
   if (CN == R(1)) { AK = CA + CB * e; QH = CB; }
   else if (e > R(0)) {
     AK = CA + CB * pow_(e, CN);
@@ -204,18 +194,18 @@ __device__ __forceinline__ void hex_yield(const R e, const R CA, const R CB, con
 // Against the sums written out corner by corner this takes 11 operations for three modes
 // of a component instead of 21, and 18 for a component's forces instead of 36.
 //
-// SFORC3 of a thread's N hexas: SDERI3, SDLEN3, SDEFO3, SRHO3, SROTA3, M1LAW / M2LAW,
+// SFORC3 of a thread's two hexas: SDERI3, SDLEN3, SDEFO3, SRHO3, SROTA3, M1LAW / M2LAW,
 // MQVISCB, SHVIS3, SFINT3.  IO gives the state and takes the new state and the corner
 // forces; act[i]: whether hexa i exists (the others' arithmetic is carried along unused).
 // io.early(key, bits) hands in the thread's time step minimum as soon as it is known, every
 // calling thread once.
-template <class R, int CORO, class IO>
-__device__ __forceinline__ void hex_element(const HexGroupDesc& gd, const bool (&act)[Pack<R>::N], const R DT1, IO& io,
-                                            ErrorWord* err, double& my_ehou, double& my_wpla) {
-  typedef Pack<R> K;
-  typedef typename K::W W;
+template <int CORO, class IO>
+__device__ __forceinline__ void hex_pair(const HexGroupDesc& gd, const bool (&act)[2], const float DT1, IO& io,
+                                         ErrorWord* err, double& my_ehou, double& my_wpla) {
+  typedef float R;
+  typedef Pair K;
+  typedef F2 W;
   constexpr int N = K::N;
-  constexpr bool split = sizeof(R) == 4;
   const bool corot = CORO && gd.jcvt;
   auto all = [](R a) { return K::all(a); };
   constexpr int pk1[4] = {0, 1, 2, 3}, pk2[4] = {6, 7, 4, 5};
@@ -224,10 +214,10 @@ __device__ __forceinline__ void hex_element(const HexGroupDesc& gd, const bool (
   W VOLN;
   double vold[N];
   {
-    HexGeom<R> g[N];
+    HexGeom g[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      hex_geometry<R, CORO>(io, i, corot, g[i]);
+      hex_geometry<CORO>(io, i, corot, g[i]);
       if (!(g[i].det > 0.0)) {   // SCHKJABT3: zero or negative volume stops the run
         if (act[i]) raise_error(err, 4, io.eid(i));
         g[i].det = 1.0;
@@ -370,7 +360,7 @@ __device__ __forceinline__ void hex_element(const HexGroupDesc& gd, const bool (
   const W D4 = DXY + DYX, D5 = DYZ + DZY, D6 = DXZ + DZX;
   const W half = all(R(0.5) * DT1);
   const W WZZ = half * (DYX - DXY), WYY = half * (DXZ - DZX), WXX = half * (DZY - DYZ);
-  // ---- SRHO3 (srho3.F:122-156; FP64 volume ratios in the split form, srho3.F:230-245) ----
+  // ---- SRHO3 (srho3.F:122-156; FP64 volume ratios, srho3.F:230-245) ----
   const R RHO0 = R(gd.rho0);
   const W rho_old = io.rho();
   const W VOLO = io.vol0();
@@ -379,18 +369,11 @@ __device__ __forceinline__ void hex_element(const HexGroupDesc& gd, const bool (
     R dv[N], rn[N], mu[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      if (split) {
-        const double v0 = io.vol0dp(i);
-        dv[i] = R(vold[i] - ((double)RHO0 / (double)K::get(rho_old, i)) * v0);
-        const double ratio = v0 / vold[i];
-        rn[i] = R((double)RHO0 * ratio);
-        mu[i] = R(ratio - 1.0);
-      } else {
-        const R vo = K::get(VOLO, i), vn = K::get(VOLN, i);
-        dv[i] = vn - (RHO0 / K::get(rho_old, i)) * vo;
-        rn[i] = RHO0 * (vo / vn);
-        mu[i] = rn[i] / RHO0 - R(1);
-      }
+      const double v0 = io.vol0dp(i);
+      dv[i] = R(vold[i] - ((double)RHO0 / (double)K::get(rho_old, i)) * v0);
+      const double ratio = v0 / vold[i];
+      rn[i] = R((double)RHO0 * ratio);
+      mu[i] = R(ratio - 1.0);
     }
     DVOL = K::of(dv); RHON = K::of(rn); AMU = K::of(mu);
   }
@@ -442,7 +425,7 @@ __device__ __forceinline__ void hex_element(const HexGroupDesc& gd, const bool (
     R ak[N], qh[N], sy[N];
 #pragma unroll
     for (int i = 0; i < N; ++i)
-      hex_yield<R>(K::get(EPXE, i), R(gd.jc_a), R(gd.jc_b), R(gd.jc_n), R(gd.sigmax), R(gd.epsmax), ak[i], qh[i], sy[i]);
+      hex_yield(K::get(EPXE, i), R(gd.jc_a), R(gd.jc_b), R(gd.jc_n), R(gd.sigmax), R(gd.epsmax), ak[i], qh[i], sy[i]);
     W AK = K::of(ak);
     const W QH = K::of(qh);
     auto ratio = [&](const W& a) {       // min(1, a / AJ2)

@@ -29,8 +29,8 @@
 // Only the shared nodes' slots and the time-step reduction cross between SMs (through
 // L2).  The slots are double-buffered by cycle parity and the reduction is
 // triple-buffered: a CTA reaches the reuse of a buffer only after a counter that every
-// reader has passed.  For shells the result is that of the patch and node kernels: the
-// same operations in the same order (for hexas see hex_element.cuh).  After the last cycle each node's owner (the lowest CTA that
+// reader has passed.  The result is that of the patch and node kernels: the same
+// operations in the same order (for hexas in the split form see hex_pair.cuh).  After the last cycle each node's owner (the lowest CTA that
 // holds it) writes it back, the element state is written back, and the kinetic
 // energy is summed per node tile exactly as the node pass sums it.
 //
@@ -39,7 +39,7 @@
 // the launch always ends.
 #pragma once
 #include "ecycle_kernels.cuh"
-#include "hex_element.cuh"
+#include "hex_pair.cuh"
 
 namespace orb {
 
@@ -213,7 +213,6 @@ struct PersistShell {
     ehou += h;
     wpla += w;
   }
-  static __host__ __device__ int offset(int sub, int t, int k) { return sub * 12 * TILE + k * TILE + t; }
   static __device__ __forceinline__ void corner(const R* all, int o, R (&f)[C]) {
     const R2* q = reinterpret_cast<const R2*>(all);
     const R2 p0 = q[o], p1 = q[4 * TILE + o], p2 = q[8 * TILE + o];
@@ -231,14 +230,14 @@ struct PersistShell {
   }
 };
 
-// N hexas (hex_element.cuh); corner forces in three planes of TILE x 8, corner k of
-// element t at k * TILE + t
-template <class R, int TILE_, int CORO>
-struct PersistHexa {
+// two hexas in the split form (hex_pair.cuh); corner forces in three planes of TILE x 8,
+// corner k of element t at k * TILE + t
+template <int TILE_, int CORO>
+struct PersistHexPair {
+  typedef float R;
   typedef HexArgs<R> Args;
-  typedef Pack<R> K;
-  typedef typename K::W W;
-  typedef typename Vec4<R>::T R4;
+  typedef Pair K;
+  typedef F2 W;
   static constexpr int N = K::N, TILE = TILE_, NT = TILE / N, C = 3, NODE_R = 5, CORNER_R = 24 * TILE, STATE_R = 0;
   W sig_[6], eint_, rho_, qvis_, vol0_, pla_, epsd_;
   double v0_[N];
@@ -270,7 +269,7 @@ struct PersistHexa {
   // what hex_element asks for
   template <class Early>
   struct IO {
-    PersistHexa& h;
+    PersistHexPair& h;
     const double *sx, *sy, *sz;
     const R* sv;
     const int NC;
@@ -302,8 +301,7 @@ struct PersistHexa {
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         R* q = h.sc + (8 * c + k) * TILE + h.t0;
-        if constexpr (N == 2) *reinterpret_cast<float2*>(q) = make_float2(f2_get(f[c], 0), f2_get(f[c], 1));
-        else *q = f[c];
+        *reinterpret_cast<float2*>(q) = make_float2(f2_get(f[c], 0), f2_get(f[c], 1));
       }
     }
   };
@@ -312,9 +310,8 @@ struct PersistHexa {
                                           const double* sz, const R* sv, const int NC, const Early& early,
                                           double& ehou, double& wpla) {
     IO<Early> io{*this, sx, sy, sz, sv, NC, early};
-    hex_element<R, CORO>(gd, act, DT1, io, a.err, ehou, wpla);
+    hex_pair<CORO>(gd, act, DT1, io, a.err, ehou, wpla);
   }
-  static __host__ __device__ int offset(int sub, int t, int k) { return sub * 24 * TILE + k * TILE + t; }
   static __device__ __forceinline__ void corner(const R* all, int o, R (&f)[C]) {
     f[0] += all[o]; f[1] += all[8 * TILE + o]; f[2] += all[16 * TILE + o];
   }
@@ -331,6 +328,91 @@ struct PersistHexa {
       a.pla[e + i] = K::get(pla_, i);
       a.epsd[e + i] = K::get(epsd_, i);
     }
+  }
+};
+
+// one FP64 hexa (hex_element), corner forces as above
+template <int TILE_, int CORO>
+struct PersistHexa {
+  typedef double R;
+  typedef HexArgs<R> Args;
+  static constexpr int TILE = TILE_, NT = TILE, C = 3, NODE_R = 5, CORNER_R = 24 * TILE, STATE_R = 0;
+  R sig_[6], eint_, rho_, qvis_, vol0_, pla_, epsd_;
+  int eid_, lc[8], e, t;
+  HexGroupDesc gd;
+  R* sc;
+  __device__ __forceinline__ bool load(const Args& a, const PersistArgs& pa, const float*, int p, bool has, int lt, R* c,
+                                       R*) {
+    sc = c; t = lt; e = (has ? p : 0) * TILE + t;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) sig_[k] = a.sig[(size_t)k * a.nelpad + e];
+    eint_ = a.eint[e]; rho_ = a.rho[e]; qvis_ = a.qvis[e]; vol0_ = a.vol0[e]; pla_ = a.pla[e]; epsd_ = a.epsd[e];
+    eid_ = a.elem_id[e];
+    const uint4 w = reinterpret_cast<const uint4*>(pa.pconn)[e];
+    const unsigned q[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) lc[k] = (q[k / 2] >> (16 * (k & 1))) & 0xffffu;
+    gd = a.groups[has ? a.patch[p].group : 0];
+    return has && t < a.patch[p].nel;
+  }
+  // what hex_element asks for
+  template <class Early>
+  struct IO {
+    PersistHexa& h;
+    R (&held)[24];
+    const double *sx, *sy, *sz;
+    const R* sv;
+    const int NC;
+    const Early& hand_in;
+    __device__ __forceinline__ void x(int k, double& x, double& y, double& z) const {
+      const int l = h.lc[k];
+      x = sx[l]; y = sy[l]; z = sz[l];
+    }
+    __device__ __forceinline__ double4 v(int k) const {
+      const int l = h.lc[k];
+      return make_double4(sv[l], sv[NC + l], sv[2 * NC + l], 0.0);
+    }
+    __device__ __forceinline__ int eid() const { return h.eid_; }
+    __device__ __forceinline__ double vol0dp() const { return h.vol0_; }
+    __device__ __forceinline__ R sig(int c) const { return h.sig_[c]; }
+    __device__ __forceinline__ R eint() const { return h.eint_; }
+    __device__ __forceinline__ R rho() const { return h.rho_; }
+    __device__ __forceinline__ R qvis() const { return h.qvis_; }
+    __device__ __forceinline__ R vol0() const { return h.vol0_; }
+    __device__ __forceinline__ R pla() const { return h.pla_; }
+    __device__ __forceinline__ void put_sig(int c, R v) const { h.sig_[c] = v; }
+    __device__ __forceinline__ void put_eint(R v) const { h.eint_ = v; }
+    __device__ __forceinline__ void put_rho(R v) const { h.rho_ = v; }
+    __device__ __forceinline__ void put_qvis(R v) const { h.qvis_ = v; }
+    __device__ __forceinline__ void put_pla(R v) const { h.pla_ = v; }
+    __device__ __forceinline__ void put_epsd(R v) const { h.epsd_ = v; }
+    __device__ __forceinline__ void early(unsigned long long k, unsigned long long b) const { hand_in(k, b); }
+    __device__ __forceinline__ void park(int q, R v) const { held[q] = v; }
+    __device__ __forceinline__ R unpark(int q) const { return held[q]; }
+    __device__ __forceinline__ void corner(int k, R fx, R fy, R fz) const {
+      h.sc[k * TILE + h.t] = fx; h.sc[(8 + k) * TILE + h.t] = fy; h.sc[(16 + k) * TILE + h.t] = fz;
+    }
+  };
+  template <class Early>
+  __device__ __forceinline__ void element(const Args& a, const R DT1, const double* sx, const double* sy,
+                                          const double* sz, const R* sv, const int NC, const Early& early,
+                                          double& ehou, double& wpla) {
+    R held[24];
+    const IO<Early> io{*this, held, sx, sy, sz, sv, NC, early};
+    unsigned long long key = ~0ull, bits = ~0ull;
+    double h = 0.0, w = 0.0;
+    hex_element<R, CORO>(gd, DT1, io, a.err, key, bits, h, w);
+    ehou += h;
+    wpla += w;
+  }
+  static __device__ __forceinline__ void corner(const R* all, int o, R (&f)[C]) {
+    f[0] += all[o]; f[1] += all[8 * TILE + o]; f[2] += all[16 * TILE + o];
+  }
+  __device__ __forceinline__ void store(const Args& a, bool has) const {
+    if (!has) return;
+#pragma unroll
+    for (int c = 0; c < 6; ++c) a.sig[(size_t)c * a.nelpad + e] = sig_[c];
+    a.eint[e] = eint_; a.rho[e] = rho_; a.qvis[e] = qvis_; a.pla[e] = pla_; a.epsd[e] = epsd_;
   }
 };
 
