@@ -13,28 +13,37 @@
 //                   minimum to the grid, counts the CTA as arrived and waits for the others,
 //                   all while the elements' arithmetic goes on.
 //   shared nodes    partial sums, patch by patch, of the nodes other CTAs hold too, to the
-//                   node-major slot skyline; the CTA arrives at the grid's second counter
+//                   node-major slot skyline; then the node's slots of all CTAs are polled
+//                   until they are there, summed (ASSPAR4) and the node updated
 //   own nodes       all other nodes: patch partials summed from shared memory in the same
 //                   order, then the dt logic, ACCELE, BCS10, VELOCITY, DEPLA (node_update
-//                   of the node pass).  They need nothing from other CTAs but the time step,
-//                   so their update runs while the shared nodes' slots travel.
-//   shared nodes    wait for the second counter, ASSPAR4 over the slots, node update
+//                   of the node pass), by other threads at the same time
+//
+// A slot is its own flag: until its CTA has written it, every word of it holds NO_SLOT, a
+// NaN that is never written as a value.  The node phases need no barrier, fence or counter
+// then; a CTA's threads meet once after the elements and once after the nodes.  Against a
+// second grid counter between the write and the read of the slots (B200): the 200x200 split
+// plate 7.3 us a cycle, now 6.75; 22,801 FP64 shells with the Newton return 13.0, now 12.5;
+// 40,687 FP64 hexas 20.0, now 19.6; 4,000 FP64 hexas 7.70, now 7.82 (the clearing stores).
 //
 // With one grid barrier between all elements and all nodes, and every patch partial
-// through L2, the 200x200 split plate took 7.5 us a cycle, now 7.0, and 10,000 shells with
-// the Newton return 8.8, now 6.2.  Hexas took two launches a cycle: 4,000 in FP64 9.9 us, now
-// 7.3; 28,952 in the split form 12.6, now 9.1.  What is left is latency: an element's chain
-// (3.2 us of the split plate's cycle), the assembly from shared memory, two L2 round trips.
+// through L2, the split plate took 7.5 us.  Hexas took two launches a cycle: 4,000 in FP64
+// 9.9 us; 28,952 in the split form 12.6, with the second counter 9.1.  What is left is
+// latency: an element's chain (3.2 us of the split plate's cycle), the assembly from shared
+// memory, an L2 round trip for the time step and one for the slots.
 //
 // Only the shared nodes' slots and the time-step reduction cross between SMs (through
-// L2).  The slots are double-buffered by cycle parity and the reduction is
-// triple-buffered: a CTA reaches the reuse of a buffer only after a counter that every
-// reader has passed.  The result is that of the patch and node kernels: the same
-// operations in the same order (for hexas in the split form see hex_pair.cuh).  After the last cycle each node's owner (the lowest CTA that
-// holds it) writes it back, the element state is written back, and the kinetic
-// energy is summed per node tile exactly as the node pass sums it.
+// L2).  The slots are double-buffered by cycle parity, and a CTA clears its slots of the
+// other parity when it writes a cycle's: it has passed the cycle's time-step counter, which
+// every CTA reaches after it has read the cycle before, and nobody polls them until the next
+// one, which this CTA reaches after it has cleared them.  The reduction is triple-buffered:
+// a CTA reaches the reuse of a buffer only after a counter that every reader has passed.
+// The result is that of the patch and node kernels: the same operations in the same order
+// (for hexas in the split form see hex_pair.cuh).  After the last cycle each node's owner
+// (the lowest CTA that holds it) writes it back, the element state is written back, and the
+// kinetic energy is summed per node tile exactly as the node pass sums it.
 //
-// The counters are monotonic and polled with a time limit: past the limit a CTA sets an
+// The counter and the slots are polled with a time limit: past the limit a CTA sets an
 // abort flag and the OR_E_TIMEOUT error word, and every CTA leaves at its next wait, so
 // the launch always ends.
 #pragma once
@@ -61,7 +70,7 @@ struct PersistArgs {
   PartAcc* acc3;              // triple-buffered time-step reduction
   double* ek_node;            // last cycle's kinetic energy of every node (owners write)
   double* ekr_node;
-  unsigned* sync;             // [0] time-step counter, [1] abort flag, [SYNC_SLOTS] slot counter
+  unsigned* sync;             // [0] time-step counter, [1] abort flag, [SYNC_END] counter of the launch's end
   int patches_per_cta;        // P
   int ncmax;                  // node capacity of a CTA (stride of the shared planes)
   int nlist;                  // list capacity of a CTA
@@ -69,21 +78,39 @@ struct PersistArgs {
   int stall_cta;              // test hook (OR_ECYCLE_TEST_STALL_CTA): this CTA does not arrive at the
                               // first cycle's counter, so the others' bounded waits run out; -1 off
 };
-constexpr int SYNC_SLOTS = 32, SYNC_WORDS = 64;      // the two counters on lines of their own
+constexpr int SYNC_END = 32, SYNC_WORDS = 64;        // the two counters on lines of their own
 
-// L2-coherent loads and stores (bypassing L1) of the data other SMs write during
-// the launch: the slot skyline and the reduction
-__device__ __forceinline__ float4 ld_cg(const float4* p) { return __ldcg(p); }
-__device__ __forceinline__ double4 ld_cg(const double4* p) {
-  const double2 a = __ldcg(reinterpret_cast<const double2*>(p));
-  const double2 b = __ldcg(reinterpret_cast<const double2*>(p) + 1);
-  return make_double4(a.x, a.y, b.x, b.y);
+// Loads and stores of the slots, which CTAs exchange during the launch: relaxed at GPU
+// scope, every word (4 bytes in the split form, 8 in FP64) written and read as a whole
+__device__ __forceinline__ float4 ld_slot(const float4* p) {
+  float4 v;
+  asm volatile("ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  return v;
 }
-__device__ __forceinline__ void st_cg(float4* p, float4 v) { __stcg(p, v); }
-__device__ __forceinline__ void st_cg(double4* p, double4 v) {
-  __stcg(reinterpret_cast<double2*>(p), make_double2(v.x, v.y));
-  __stcg(reinterpret_cast<double2*>(p) + 1, make_double2(v.z, v.w));
+__device__ __forceinline__ double4 ld_slot(const double4* p) {
+  double4 v;
+  asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
+  asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];"
+               : "=d"(v.z) : "l"(reinterpret_cast<const double*>(p) + 2) : "memory");
+  v.w = 0.0;
+  return v;
 }
+__device__ __forceinline__ void st_slot(float4* p, float x, float y, float z) {
+  asm volatile("st.relaxed.gpu.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(0.f) : "memory");
+}
+__device__ __forceinline__ void st_slot(double4* p, double x, double y, double z) {
+  asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(x), "d"(y) : "memory");
+  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(reinterpret_cast<double*>(p) + 2), "d"(z) : "memory");
+}
+// NO_SLOT: all ones.  Arithmetic makes no such NaN but by negating its own, so a NaN force is
+// written as another one.
+__device__ __forceinline__ float no_slot(float) { return __uint_as_float(0xffffffffu); }
+__device__ __forceinline__ double no_slot(double) { return __longlong_as_double(-1ll); }
+__device__ __forceinline__ bool is_slot(float x) { return __float_as_uint(x) != 0xffffffffu; }
+__device__ __forceinline__ bool is_slot(double x) { return __double_as_longlong(x) != -1ll; }
+__device__ __forceinline__ float slot_value(float x) { return is_slot(x) ? x : __uint_as_float(0x7fffffffu); }
+__device__ __forceinline__ double slot_value(double x) { return is_slot(x) ? x : __longlong_as_double(0x7fffffffffffffffll); }
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
   unsigned v;
@@ -511,7 +538,18 @@ cycle_persistent_kernel(typename Kind::Args a, NodeArgs<R> na, PersistArgs pa, i
   R4* fs[2] = {a.fslot, reinterpret_cast<R4*>(pa.fslot2)};
   R4* ms_[2] = {const_cast<R4*>(na.mslot), reinterpret_cast<R4*>(pa.mslot2)};
   unsigned* const abort = pa.sync + 1;
-  unsigned* const slot_count = pa.sync + SYNC_SLOTS;
+  // the slots this CTA writes, in both buffers
+  for (int i = tid; i < nsh; i += blockDim.x) {
+    const int first = pa.list_ofs[n0 + i], end = pa.list_ofs[n0 + i + 1];
+    for (int w = first; w < end; w += 1 + (pa.list[w] & 0xff)) {
+      const int s = pa.list[w] >> 8;
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        st_slot(&fs[b][s], no_slot(R(0)), no_slot(R(0)), no_slot(R(0)));
+        if constexpr (ROT) st_slot(&ms_[b][s], no_slot(R(0)), no_slot(R(0)), no_slot(R(0)));
+      }
+    }
+  }
   __syncthreads();
 
   // one patch's partial of a node: its corners from word w on; returns its slot
@@ -526,8 +564,8 @@ cycle_persistent_kernel(typename Kind::Args a, NodeArgs<R> na, PersistArgs pa, i
   };
 
   for (int c = 0; c < ncycles; ++c) {
-    R4* fslot = fs[c & 1];
-    R4* mslot = ms_[c & 1];
+    R4 *fslot = fs[c & 1], *mslot = ms_[c & 1];
+    R4 *fclear = fs[1 - (c & 1)], *mclear = ms_[1 - (c & 1)];
     // ---------------- element phase ----------------
     if (active) {
       auto early = [&](unsigned long long key, unsigned long long bits) {
@@ -585,31 +623,27 @@ cycle_persistent_kernel(typename Kind::Args a, NodeArgs<R> na, PersistArgs pa, i
       if constexpr (ROT) { sv[3 * NC + i] = w.x; sv[4 * NC + i] = w.y; sv[5 * NC + i] = w.z; }
       if (last && sown[i]) { pa.ek_node[g] = ek; pa.ekr_node[g] = ekr; }
     };
-    // shared nodes: this CTA's patch partials to their slots
+    // shared nodes: this CTA's patch partials to their slots, and the next cycle's cleared
     for (int i = tid; i < nsh; i += blockDim.x) {
       const int2 lr = slist[i];
       for (int w = lr.x; w < lr.y;) {
         R f[C];
         const int s = partial(w, f);
-        st_cg(&fslot[s], mk4(f[0], f[1], f[2], R(0)));
-        if constexpr (ROT) st_cg(&mslot[s], mk4(f[3], f[4], f[5], R(0)));
+        st_slot(&fslot[s], slot_value(f[0]), slot_value(f[1]), slot_value(f[2]));
+        if constexpr (ROT) st_slot(&mslot[s], slot_value(f[3]), slot_value(f[4]), slot_value(f[5]));
+        st_slot(&fclear[s], no_slot(R(0)), no_slot(R(0)), no_slot(R(0)));
+        if constexpr (ROT) st_slot(&mclear[s], no_slot(R(0)), no_slot(R(0)), no_slot(R(0)));
       }
     }
-    __syncthreads();
-    if (tid == 0) grid_arrive(slot_count);
-    // the CTA's own nodes while the shared nodes' slots travel, then those; the own ones by
-    // the threads from the last down, so that the first have the shared ones.  For shells one
-    // loop, so that the node update is in the kernel once: in FP64 they spill less for it.
-    // Hexas do not, and ran 5 % faster with the two phases apart.
+    // the CTA's own nodes, by the threads from the last down, then the shared ones by the
+    // threads from the first up, so that few have one of each.  For shells one loop, so that
+    // the node update is in the kernel once: in FP64 they spill less for it.  Hexas do not,
+    // and ran 5 % faster with the two apart.  Four slots are polled at a time (FP64 shells
+    // two, for their registers): two ran the 4,000 hexas in 8.47 us a cycle, eight in 7.94.
 #pragma unroll (ROT ? 1 : 2)
     for (int shared = 0; shared < 2; ++shared) {
-      if (shared) {
-        if (tid == 0 && grid_wait(slot_count, (unsigned)(c + 1) * (unsigned)G, abort, a.err)) s_abort = 1;
-        __syncthreads();
-        if (s_abort) return;
-      }
       const int last_node = shared ? nsh - 1 : nn - 1, first_node = shared ? 0 : nsh;
-      const int i0 = shared ? last_node - (nsh - 1 - tid) : last_node - (int)(blockDim.x - 1 - tid);
+      const int i0 = shared ? tid : last_node - (int)(blockDim.x - 1 - tid);
       const int dir = shared ? (int)blockDim.x : -(int)blockDim.x;
       for (int i = i0; i >= first_node && i <= last_node; i += dir) {
         R f[C];
@@ -625,17 +659,34 @@ cycle_persistent_kernel(typename Kind::Args a, NodeArgs<R> na, PersistArgs pa, i
             for (int q = 0; q < C; ++q) f[q] = first ? h[q] : f[q] + h[q];
           }
         } else {
-          // ASSPAR4: the node's slots in ascending patch order, U read at a time
+          // ASSPAR4: the node's slots in ascending patch order, U at a time
           constexpr int U = ROT && sizeof(R) == 8 ? 2 : 4;
           const int2 rg = srange[i];
           for (int k = rg.x; k < rg.y; k += U) {
             R4 F[U], M[U];
+            long long t0 = 0;
+            for (int tries = 0;; ++tries) {
+              bool all = true;
 #pragma unroll
-            for (int u = 0; u < U; ++u)
-              if (k + u < rg.y) {
-                F[u] = ld_cg(&fslot[k + u]);
-                if constexpr (ROT) M[u] = ld_cg(&mslot[k + u]);
+              for (int u = 0; u < U; ++u)
+                if (k + u < rg.y) {
+                  F[u] = ld_slot(&fslot[k + u]);
+                  if constexpr (ROT) M[u] = ld_slot(&mslot[k + u]);
+                }
+#pragma unroll
+              for (int u = 0; u < U; ++u)
+                if (k + u < rg.y) {
+                  all = all && is_slot(F[u].x) && is_slot(F[u].y) && is_slot(F[u].z);
+                  if constexpr (ROT) all = all && is_slot(M[u].x) && is_slot(M[u].y) && is_slot(M[u].z);
+                }
+              if (all) break;
+              if ((tries & 63) == 63) {
+                if (!t0) t0 = clock64();
+                const bool late = clock64() - t0 > (1ll << 31);       // about a second at the SM clock
+                if (late) { atomicExch(abort, 1u); raise_error(a.err, 7, cta); }
+                if (late || __ldcg(abort)) { s_abort = 1; break; }
               }
+            }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
               if (k + u >= rg.y) break;
@@ -655,6 +706,7 @@ cycle_persistent_kernel(typename Kind::Args a, NodeArgs<R> na, PersistArgs pa, i
     t.tt = t.tt + DT2; t.dt2 = DT2; t.dt2old = DT2; t.dt1 = DTc1; t.dt12 = DT12;
     t.ncycle = t.ncycle + 1; t.ityptst = ityp; t.neltst = nelt; t.pad = 0;
     __syncthreads();
+    if (s_abort) return;
   }
 
   // ---- write back: held nodes by their owner, element state, energies, time ----
@@ -684,8 +736,8 @@ cycle_persistent_kernel(typename Kind::Args a, NodeArgs<R> na, PersistArgs pa, i
   // kinetic energy per node tile of 128, summed as the node pass sums it
   __syncthreads();
   if (tid == 0) {
-    grid_arrive(slot_count);
-    if (grid_wait(slot_count, (unsigned)(ncycles + 1) * (unsigned)G, abort, a.err)) s_abort = 1;
+    grid_arrive(pa.sync + SYNC_END);
+    if (grid_wait(pa.sync + SYNC_END, (unsigned)G, abort, a.err)) s_abort = 1;
   }
   __syncthreads();
   if (s_abort) return;
