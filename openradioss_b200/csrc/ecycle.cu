@@ -590,11 +590,11 @@ int launch_loads(or_ecycle* h, Impl<R>& m, int parity, bool pdl) {
   h->launches++;
   return OR_OK;
 }
-// node tiles beyond one wave of node_kernel_wide (1024 threads per SM): the
-// streaming form
+// node tiles beyond one wave of node_kernel: the streaming form, whose 8 CTAs per SM
+// finish them sooner than a second wave would: 1,048 tiles 5.5 against 6.3 us (B200)
 template <class R>
 bool node_wide(const or_ecycle* h, const Impl<R>& m) {
-  return m.ntiles > (long long)h->nsm * (1024 / NODE_TILE);
+  return m.ntiles > (long long)h->nsm * m.node_ctas;
 }
 template <class R>
 int launch_node(or_ecycle* h, Impl<R>& m, int parity, bool pdl = false) {
