@@ -704,82 +704,88 @@ int persist_build(or_ecycle* h, Impl<R>& m) {
   const int P = std::max((npatch + h->nsm - 1) / h->nsm, shells ? (128 + tile - 1) / tile : 1);
   if (P * NT > PERSIST_THREADS) return OR_OK;
   const int G = (npatch + P - 1) / P;
-  std::vector<std::vector<int>> lists(G);
-  std::vector<char> held(m.nnodpad, 0);
-  for (int c = 0; c < G; ++c) {
-    for (int p = c * P; p < std::min(npatch, (c + 1) * P); ++p)
-      for (int j = 0; j < ps.info[p].nloc; ++j) lists[c].push_back(ps.nodes[ps.info[p].node_ofs + j]);
-    std::sort(lists[c].begin(), lists[c].end());
-    lists[c].erase(std::unique(lists[c].begin(), lists[c].end()), lists[c].end());
-    for (int g : lists[c]) held[g] = 1;
-  }
   const HPart& Pt = h->parts[0];
-  for (int i = 0, k = 0; i < Pt.numnod; ++i)
-    if (!held[Pt.node_start + i]) lists[(k++) % G].push_back(Pt.node_start + i);
-  std::vector<int> holders(m.nnodpad, 0);
+  std::vector<std::vector<int>> lists(G);       // every CTA's nodes
+  std::vector<int> holders(m.nnodpad, 0), seen(m.nnodpad, -1);
   for (int c = 0; c < G; ++c)
-    for (int g : lists[c]) holders[g]++;
+    for (int p = c * P; p < std::min(npatch, (c + 1) * P); ++p)
+      for (int j = 0; j < ps.info[p].nloc; ++j) {
+        const int g = ps.nodes[ps.info[p].node_ofs + j];
+        if (seen[g] == c) continue;
+        seen[g] = c;
+        holders[g]++;
+        lists[c].push_back(g);
+      }
+  for (int i = 0, k = 0; i < Pt.numnod; ++i)
+    if (!holders[Pt.node_start + i]) {
+      lists[(k++) % G].push_back(Pt.node_start + i);
+      holders[Pt.node_start + i] = 1;
+    }
   std::vector<int> ofs(G + 1, 0), glob, nshared(G, 0);
   std::vector<unsigned char> own;
-  std::vector<int> first(m.nnodpad, -1);
+  std::fill(seen.begin(), seen.end(), -1);
   int ncmax = 0;
-  // a CTA's nodes: those other CTAs hold too, then its own, both in ascending order
-  auto before = [&](int a, int b) { return (holders[a] > 1) != (holders[b] > 1) ? holders[a] > 1 : a < b; };
   for (int c = 0; c < G; ++c) {
-    std::sort(lists[c].begin(), lists[c].end(), before);
-    ncmax = std::max(ncmax, (int)lists[c].size());
-    for (int g : lists[c]) nshared[c] += holders[g] > 1;
-    for (int g : lists[c]) {
+    // the nodes that other CTAs hold too, then the CTA's own, both in ascending order
+    std::vector<int>& L = lists[c];
+    const auto mid = std::partition(L.begin(), L.end(), [&](int g) { return holders[g] > 1; });
+    std::sort(L.begin(), mid);
+    std::sort(mid, L.end());
+    nshared[c] = (int)(mid - L.begin());
+    ncmax = std::max(ncmax, (int)L.size());
+    for (int g : L) {
       glob.push_back(g);
-      own.push_back(first[g] < 0 ? 1 : 0);
-      if (first[g] < 0) first[g] = c;
+      own.push_back(seen[g] < 0 ? 1 : 0);
+      if (seen[g] < 0) seen[g] = c;
     }
     ofs[c + 1] = (int)glob.size();
   }
   if (ncmax > 65535) return OR_OK;
+  // corner indices, and the corner lists of the held nodes: per patch of the CTA its slot
+  // and corners (the patch lists are visited in ascending patch order, their corners ascend)
   std::vector<unsigned short> pconn((size_t)ps.nelpad * K, 0);
-  for (int c = 0; c < G; ++c) {
-    const std::vector<int>& L = lists[c];
-    for (int p = c * P; p < std::min(npatch, (c + 1) * P); ++p) {
-      const PatchInfo& pi = ps.info[p];
-      for (int t = 0; t < pi.nel; ++t)
-        for (int k = 0; k < K; ++k) {
-          const size_t q = (size_t)(pi.elem0 + t) * K + k;
-          const int g = ps.nodes[pi.node_ofs + (ps.local[q] & LOCAL_MASK)];
-          pconn[q] = (unsigned short)(std::lower_bound(L.begin(), L.end(), g, before) - L.begin());
-        }
-    }
-  }
-  // corner lists of the held nodes: per patch of the CTA its slot and corners (the patch
-  // lists are visited in ascending patch order, their corners ascend)
-  std::vector<int> list_ofs, words;
+  std::vector<int> list_ofs(glob.size() + 1, 0), words, at(m.nnodpad, 0), fill, count, head;
   int nlist = 0;
   for (int c = 0; c < G; ++c) {
     const std::vector<int>& L = lists[c];
-    std::vector<std::vector<int>> of(L.size());
-    for (int p = c * P; p < std::min(npatch, (c + 1) * P); ++p) {
+    const int p0 = c * P, p1 = std::min(npatch, (c + 1) * P), w0 = (int)words.size();
+    fill.assign(L.size() + 1, 0);
+    for (int i = 0; i < (int)L.size(); ++i) at[L[i]] = i;
+    for (int p = p0; p < p1; ++p) {
       const PatchInfo& pi = ps.info[p];
-      std::vector<std::vector<int>> corners(pi.nloc);
-      for (int t = 0; t < pi.nel; ++t)
-        for (int k = 0; k < K; ++k)        // as Kind::corner reads them
-          corners[ps.local[(size_t)(pi.elem0 + t) * K + k] & LOCAL_MASK].push_back(
-              (p - c * P) * (shells ? 12 : 24) * tile + k * tile + t);
-      for (int j = 0; j < pi.nloc; ++j) {
-        const int g = ps.nodes[pi.node_ofs + j], slot = ps.slots[pi.node_ofs + j];
-        std::vector<int>& o = of[std::lower_bound(L.begin(), L.end(), g, before) - L.begin()];
-        if (corners[j].size() > 0xff || slot >= 1 << 23) return OR_OK;
-        o.push_back(slot << 8 | (int)corners[j].size());
-        o.insert(o.end(), corners[j].begin(), corners[j].end());
+      for (int j = 0; j < pi.nloc; ++j) fill[at[ps.nodes[pi.node_ofs + j]] + 1]++;
+      for (int q = 0; q < pi.nel * K; ++q) {
+        const size_t e = (size_t)pi.elem0 * K + q;
+        const int i = at[ps.nodes[pi.node_ofs + (ps.local[e] & LOCAL_MASK)]];
+        pconn[e] = (unsigned short)i;
+        fill[i + 1]++;
       }
     }
-    const int w0 = (int)words.size();
-    for (auto& o : of) {
-      list_ofs.push_back((int)words.size());
-      words.insert(words.end(), o.begin(), o.end());
+    for (size_t i = 0; i < L.size(); ++i) {
+      fill[i + 1] += fill[i];
+      list_ofs[ofs[c] + i + 1] = w0 + fill[i + 1];
+    }
+    words.resize(w0 + fill[L.size()]);
+    for (int p = p0; p < p1; ++p) {
+      const PatchInfo& pi = ps.info[p];
+      count.assign(pi.nloc, 0);
+      head.resize(pi.nloc);
+      for (int q = 0; q < pi.nel * K; ++q) count[ps.local[(size_t)pi.elem0 * K + q] & LOCAL_MASK]++;
+      for (int j = 0; j < pi.nloc; ++j) {
+        const int slot = ps.slots[pi.node_ofs + j];
+        if (count[j] > 0xff || slot >= 1 << 23) return OR_OK;
+        int& w = fill[at[ps.nodes[pi.node_ofs + j]]];
+        words[w0 + w] = slot << 8 | count[j];
+        head[j] = w0 + w + 1;
+        w += 1 + count[j];
+      }
+      for (int t = 0; t < pi.nel; ++t)
+        for (int k = 0; k < K; ++k)        // as Kind::corner reads them
+          words[head[ps.local[(size_t)(pi.elem0 + t) * K + k] & LOCAL_MASK]++] =
+              (p - p0) * (shells ? 12 : 24) * tile + k * tile + t;
     }
     nlist = std::max(nlist, (int)words.size() - w0);
   }
-  list_ofs.push_back((int)words.size());
   // the points of the shell kernel that keeps their state on the chip (PersistShell); in
   // FP64 it lies in shared memory, and where that does not fit it stays in global memory
   int npt = shells && (m.same_npt == 5 || m.same_npt == 3) ? m.same_npt : 0;
