@@ -360,6 +360,7 @@ struct Impl {
   DBuf<double4> X; DBuf<double> DX, DY, DZ; DBuf<R4> V, VR; DBuf<unsigned char> code;
   DBuf<unsigned> rotmask; std::vector<unsigned> rotmask_h;   // NodeArgs::rotmask, and its host copy
   int rot_sparse = 0;                                         // NodeArgs::rot_sparse
+  int node_ctas = 8;                                          // resident CTAs of node_kernel per SM
   DBuf<int> adsky, tile_part; DBuf<PartDesc> partd;
   DBuf<R4> fslot, mslot;
   // Control words of the cycle in one block, so that a step sends and reads them by one
@@ -924,7 +925,10 @@ int finalize_impl(or_ecycle* h) {
   m.ntiles = nt;
   // tiles left to the library (cfg.block_hex / block_shell 0): 64 elements per patch
   // when the patches at 64 fit one wave of the kernel's resident CTAs (a latency-bound
-  // mesh gains from more CTAs), 128 otherwise; the autotuner times all three
+  // mesh gains from more CTAs), 128 otherwise; the autotuner times all three.  Split hexas
+  // keep 64 only as far as the persistent cycle reaches (12 patches of 32 threads,
+  // two hexas each, per CTA): beyond it the patches at 64 ran 125,911 hexas in 25.1 us a cycle,
+  // those at 128 in 21.0 (B200), although 64 still fit one wave up to 132,600.
   {
     auto tile_for = [&](long long nel, int ctas128) {
       return nel <= (long long)h->nsm * (2 * ctas128) * 64 ? 64 : 128;
@@ -932,7 +936,9 @@ int finalize_impl(or_ecycle* h) {
     long long nh = 0, ns = 0;
     for (auto& g : h->hex) nh += g.nel;
     for (auto& g : h->shell) ns += g.nel;
-    if (h->cfg.block_hex == 0) h->tile_hex = tile_for(nh, Occupancy<R>::hex);
+    if (h->cfg.block_hex == 0)
+      h->tile_hex = sizeof(R) == 4 && nh > (long long)h->nsm * (PERSIST_THREADS / 32) * 64
+                        ? 128 : tile_for(nh, Occupancy<R>::hex);
     if (h->cfg.block_shell == 0) h->tile_shell = tile_for(ns, Occupancy<R>::shell);
   }
   // patches
@@ -1231,6 +1237,7 @@ int finalize_impl(or_ecycle* h) {
   }
   rc = set_smem_attrs<R>(h, m);
   if (rc) return rc;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m.node_ctas, node_kernel<R, NODE_TILE>, NODE_TILE, 0));
   if ((rc = persist_build<R>(h, m))) return rc;
   CK(cudaDeviceSynchronize());
   return OR_OK;
