@@ -364,8 +364,9 @@ struct Impl {
   DBuf<int> adsky, tile_part; DBuf<PartDesc> partd;
   DBuf<R4> fslot, mslot;
   // Control words of the cycle in one block, so that a step sends and reads them by one
-  // copy each: time[2][part], acc[2][part], the error word.  The pinned images are the
-  // step's: what goes to the device and what came back.
+  // copy each: time[2][part], acc[2][part], the error word, the flag of the second element
+  // pass (publish_nodes).  The pinned images are the step's: what goes to the device and what
+  // came back.
   DBuf<unsigned char> ctl;
   struct { PartTime* p; } time{nullptr};
   struct { PartAcc* p; } acc{nullptr};
@@ -373,7 +374,8 @@ struct Impl {
   unsigned char *ctl_in = nullptr, *ctl_out = nullptr;
   size_t acc_ofs() const { return 2 * (size_t)nparts * sizeof(PartTime); }
   size_t err_ofs() const { return acc_ofs() + 2 * (size_t)nparts * sizeof(PartAcc); }
-  size_t ctl_bytes() const { return err_ofs() + sizeof(ErrorWord); }
+  size_t flag_ofs() const { return err_ofs() + sizeof(ErrorWord); }
+  size_t ctl_bytes() const { return flag_ofs() + sizeof(unsigned); }
   DBuf<double> ekin, ekinr;
   // hexas
   PatchSet hps;
@@ -429,6 +431,7 @@ struct Impl {
     a.sig = hsig.p; a.eint = heint.p; a.rho = hrho.p; a.qvis = hqvis.p; a.pla = hpla.p; a.epsd = hepsd.p;
     a.vol0 = hvol0.p; a.vol0dp = hvol0dp.p; a.fslot = fslot.p; a.time = time.p; a.acc = acc.p;
     a.blk_ehour = hehour.p; a.blk_wpla = hwpla.p; a.err = err.p;
+    a.nodes_flag = (const unsigned*)(ctl.p + flag_ofs());
     a.nelpad = hps.nelpad; a.nparts = nparts; a.npatch = (int)hps.info.size(); a.nlmax = hps.nlmax;
     a.inc = hinc.p; a.inc_stride = hinc_stride;
     return a;
@@ -440,6 +443,7 @@ struct Impl {
     a.sig = ssig.p; a.pla = spla.p; a.thk = sthk.p; a.thke = sthke.p; a.hourg = shourg.p; a.eint = seint.p;
     a.jca = sjca.p; a.fslot = fslot.p; a.mslot = mslot.p; a.time = time.p; a.acc = acc.p;
     a.blk_ehour = sehour.p; a.blk_wpla = swpla.p; a.err = err.p;
+    a.nodes_flag = hps.info.empty() ? nullptr : (unsigned*)(ctl.p + flag_ofs());
     a.nelpad = sps.nelpad; a.nparts = nparts; a.npatch = (int)sps.info.size(); a.maxnpt = maxnpt;
     a.nlmax = sps.nlmax;
     a.inc = sinc.p; a.inc_stride = sinc_stride;
@@ -1349,7 +1353,7 @@ int step_impl(or_ecycle* h, int ncycles, or_ecycle_time* t) {
   int rc;
   if (h->late && (rc = wait_queued(h))) return rc;
   // the time state at parity 0 (the other parity's follows from the first cycle), an
-  // empty reduction, no error
+  // empty reduction, no error, no cycle's nodes published
   PartTime* pt = (PartTime*)m.ctl_in;
   std::memset(m.ctl_in, 0, m.ctl_bytes());
   std::memset(m.ctl_in + m.acc_ofs(), 0xff, 2 * (size_t)np * sizeof(PartAcc));

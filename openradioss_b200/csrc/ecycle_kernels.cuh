@@ -131,6 +131,7 @@ struct HexArgs {
   double* blk_ehour;          // per patch cumulative hourglass energy
   double* blk_wpla;           // per patch cumulative plastic work
   ErrorWord* err;
+  const unsigned* nodes_flag; // second element pass of a cycle: await_nodes
   int nelpad, nparts, npatch;
   int nlmax;                  // stride of patch_nodes / patch_slots (padded per patch)
   int inc_stride;
@@ -160,6 +161,7 @@ struct ShellArgs {
   double* blk_ehour;
   double* blk_wpla;
   ErrorWord* err;
+  unsigned* nodes_flag;       // publish_nodes for the hexa pass beside this one, null without one
   int nelpad, nparts, npatch, maxnpt;
   int nlmax;                  // stride of patch_nodes / patch_slots (padded per patch)
   int inc_stride;
@@ -247,12 +249,34 @@ __host__ __device__ inline size_t halo_buffer_bytes(int nhalo) {
 // completed whenever a kernel starts: its prologue may read that grid's output.
 //
 // A mesh of hexas and shells has two element passes in a cycle, which depend on the
-// node pass before them but not on one another.  The second (SECOND below) does not
-// wait at its start: it starts once every CTA of the first has seen the node pass
-// complete, so it may read what the node pass wrote.  It waits at its end, so that
-// its own completion, on which the next node pass waits, includes the first's.
+// node pass before them but not on one another.  The second (`second` below) does not
+// wait at its start, which would wait for the first.  What the node pass wrote reaches it
+// through a flag instead: a thread of the first, past its own wait and so with the node
+// pass's writes visible to it, releases the flag (publish_nodes), and every thread of the
+// second acquires it before it reads nodes or time (await_nodes).  The second starts only
+// when every CTA of the first has triggered, so the flag is already set or on its way.  It
+// executes the wait at its end, so that its own completion, on which the next node pass
+// waits, includes the first's.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+// The flag holds 1 + the parity of the last cycle published (0 before a step's first), so a
+// cycle's value differs from the one before.
+__device__ __forceinline__ void publish_nodes(unsigned* flag, int parity) {
+  if (flag && blockIdx.x == 0 && threadIdx.x == 0)
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag), "r"(1u + (unsigned)parity) : "memory");
+}
+// false if the flag did not come within `tries` polls
+__device__ __forceinline__ bool await_nodes(const unsigned* flag, int parity, int tries) {
+  while (ld_acquire(flag) != 1u + (unsigned)parity)
+    if (--tries < 0) return false;
+  return true;
+}
 
 // BCS1V (bcs1.F): zero the components of (x, y, z) along the fixed directions of
 // code lcod (4 = x, 2 = y, 1 = z) of skew frame sk (rows x', y', z'), projecting
@@ -991,10 +1015,15 @@ hex_patch_kernel(HexArgs<R> a, int parity, int second) {
   if (tid == 0) { pre_ehour = a.blk_ehour[p]; pre_wpla = a.blk_wpla[p]; }
   // X, V and the cycle's time come from the previous node pass: gathered after the
   // wait, straight into shared memory
+  // (the node list read ahead of it: with the flag's round trip and the list's in a row, 200
+  // cycles of 2 M hexas with a skin took 64.4 ms, so 62.8; with the passes in turn 63.4)
+  const int node0 = tid < NLM ? a.patch_nodes[p * NLM + tid] : 0;
+  const int node1 = tid + TILE < NLM ? a.patch_nodes[p * NLM + tid + TILE] : 0;
   if (!second) pdl_wait();
+  else if (!await_nodes(a.nodes_flag, parity, STAGE_WAIT_TRIES)) raise_error(a.err, 7, p);
   pdl_trigger();
   for (int j = tid; j < NLM; j += TILE) {
-    const int g = a.patch_nodes[p * NLM + j];
+    const int g = j == tid ? node0 : j == tid + TILE ? node1 : a.patch_nodes[p * NLM + j];
     const double* xg = reinterpret_cast<const double*>(a.X + g);
     cp_async16(sxy + j, xg);
     cp_async8(sz + j, xg + 2);
@@ -1833,6 +1862,7 @@ shell_patch_kernel(ShellArgs<R> a, int parity, const float* __restrict__ zw) {
   int* sidx = reinterpret_cast<int*>(sc);   // NLM <= 4 * TILE entries
   for (int j = tid; j < NLM; j += TILE) sidx[j] = a.patch_nodes[p * NLM + j];
   pdl_wait();
+  publish_nodes(a.nodes_flag, parity);
   pdl_trigger();
   for (int j = tid; j < NLM; j += TILE) {
     const int g = sidx[j];
@@ -1935,6 +1965,7 @@ shell_patch_staged_kernel(ShellArgs<R> a, int parity, const float* __restrict__ 
   const int node1 = tid + TILE < NLM ? a.patch_nodes[p * NLM + tid + TILE] : 0;
   // X, V, VR and the cycle's time come from the previous node pass
   pdl_wait();
+  publish_nodes(a.nodes_flag, parity);
   pdl_trigger();
   for (int j = tid; j < NLM; j += TILE) {
     const int g = j == tid ? node0 : j == tid + TILE ? node1 : a.patch_nodes[p * NLM + j];

@@ -112,11 +112,6 @@ __device__ __forceinline__ bool is_slot(double x) { return __double_as_longlong(
 __device__ __forceinline__ float slot_value(float x) { return is_slot(x) ? x : __uint_as_float(0x7fffffffu); }
 __device__ __forceinline__ double slot_value(double x) { return is_slot(x) ? x : __longlong_as_double(0x7fffffffffffffffll); }
 
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
 // One thread's part of a grid-wide counter.  Arrive: release what the CTA wrote before.
 __device__ __forceinline__ void grid_arrive(unsigned* count) {
   __threadfence();
