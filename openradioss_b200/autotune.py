@@ -1,9 +1,10 @@
 """Autotuner for the cycle's launch form.
 
 For a deck and precision, builds one handle per candidate: each tile (elements
-per patch = threads per CTA of the hexa and shell kernels), and for a deck
-that can run the persistent shell cycle, each tile both with it and with the
-per-phase kernels.  It times a few hundred graph-replayed cycles of each with
+per patch = threads per CTA of the hexa and shell kernels), and where the handle
+runs the persistent cycle, the tile both with it and with the per-phase kernels.
+Which of the two a handle runs is read off its launches (one for all the cycles of
+a call, or two and more a cycle), which holds for shells and hexas alike.  It times a few hundred graph-replayed cycles of each with
 CUDA events on the handle's stream.  For a deck with both hexas and shells the
 two element kernels are independent launches, so their tiles are chosen apart:
 each candidate handle also times its hexa and shell kernels alone
@@ -23,6 +24,7 @@ from . import abi, decks
 
 CANDIDATES = (64, 128, 256)
 CACHE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "autotune_cache.json")
+CACHE_VERSION = 2      # entries of the first timed hexas' persistent cycle as the per-phase kernels
 
 
 def _key(deck, precision, gpu):
@@ -30,9 +32,11 @@ def _key(deck, precision, gpu):
 
 
 def _time_cycles(h, ncycles):
+    """(ms per cycle, whether the handle ran the persistent cycle)"""
     import torch
     s = torch.cuda.ExternalStream(h.stream())
     h.step(min(ncycles, 64))          # first replay captures the graph
+    persistent = h.launch_count() == 1
     h.reset()
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     torch.cuda.synchronize()
@@ -40,7 +44,7 @@ def _time_cycles(h, ncycles):
     h.step(ncycles)
     e1.record(s)
     torch.cuda.synchronize()
-    return e0.elapsed_time(e1) / ncycles
+    return e0.elapsed_time(e1) / ncycles, persistent
 
 
 def tune(deck, precision=abi.OR_PREC_SPLIT, ncycles=256, use_cache=True, device=0, verbose=False):
@@ -57,7 +61,7 @@ def tune(deck, precision=abi.OR_PREC_SPLIT, ncycles=256, use_cache=True, device=
             cache = json.load(open(CACHE))
         except (OSError, ValueError):
             cache = {}
-    if use_cache and key in cache and "persistent" in cache[key]:
+    if use_cache and cache.get(key, {}).get("version") == CACHE_VERSION:
         c = cache[key]
         return c["block_hex"], c["block_shell"], c["persistent"], c["ms_per_cycle"]
     has_hex = any(p["hex"] for p in deck["parts"])
@@ -69,14 +73,13 @@ def tune(deck, precision=abi.OR_PREC_SPLIT, ncycles=256, use_cache=True, device=
         for pers in (0, -1):
             h = ECycle(deck, precision=precision, device=device, graph=1, block_hex=t, block_shell=t,
                        persistent=pers)
-            on = h.persistent_info()[0]
-            k = (t, t, 0 if on else -1)
-            timings[k] = _time_cycles(h, ncycles)
+            ms, on = _time_cycles(h, ncycles)
+            timings[(t, t, 0 if on else -1)] = ms
             if mixed and not on:
                 kern[t] = h.kernel_times(reps=16)
             h.close()
             if verbose:
-                print(f"tile {t} {'persistent' if on else 'phase kernels'}: {timings[k] * 1e3:.2f} us/cycle",
+                print(f"tile {t} {'persistent' if on else 'phase kernels'}: {ms * 1e3:.2f} us/cycle",
                       flush=True)
             if not on:
                 break                     # no persistent form at this tile: the phase kernels are timed
@@ -86,7 +89,7 @@ def tune(deck, precision=abi.OR_PREC_SPLIT, ncycles=256, use_cache=True, device=
         if th != ts:                      # the two fastest kernels at different tiles: time the pair
             h = ECycle(deck, precision=precision, device=device, graph=1, block_hex=th, block_shell=ts,
                        persistent=-1)
-            timings[(th, ts, -1)] = _time_cycles(h, ncycles)
+            timings[(th, ts, -1)] = _time_cycles(h, ncycles)[0]
             h.close()
             if verbose:
                 print(f"hexa tile {th}, shell tile {ts}: {timings[(th, ts, -1)] * 1e3:.2f} us/cycle", flush=True)
@@ -97,7 +100,7 @@ def tune(deck, precision=abi.OR_PREC_SPLIT, ncycles=256, use_cache=True, device=
     def name(k):
         base = f"{k[0]}" if k[0] == k[1] else f"h{k[0]}s{k[1]}"
         return base + ("p" if k[2] == 0 else "")
-    cache[key] = {"block_hex": bh, "block_shell": bs, "persistent": best[2],
+    cache[key] = {"version": CACHE_VERSION, "block_hex": bh, "block_shell": bs, "persistent": best[2],
                   "ms_per_cycle": {name(k): v for k, v in timings.items()}}
     try:
         json.dump(cache, open(CACHE, "w"), indent=1, sort_keys=True)
