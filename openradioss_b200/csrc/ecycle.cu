@@ -625,7 +625,9 @@ constexpr int MAX_DYN_SMEM = 200 * 1024, PERSIST_MAX_SMEM = 224 * 1024;
 template <class R>
 int set_smem_attrs(or_ecycle* h, Impl<R>& m) {
   const size_t hs = hex_smem<R>(m.hps.nlmax, h->tile_hex, m.hinc_stride);
-  const size_t ss = shell_smem<R>(m.sps.nlmax, h->tile_shell, m.sinc_stride, 5);   // the largest: the 5-point kernels
+  // the largest form there is: the staged 5-point kernel in the split form.  256 shells of 1,024
+  // nodes, the most a patch can hold, take 116 KB staged and in FP64 124 KB unstaged
+  const size_t ss = shell_smem<R>(m.sps.nlmax, h->tile_shell, m.sinc_stride, sizeof(R) == 4 ? 5 : 0);
   if (hs > MAX_DYN_SMEM || ss > MAX_DYN_SMEM) return fail(h, OR_E_UNSUPPORTED, "patch shared memory above 200 KB");
   auto set = [](auto* f) { return set_smem(f, MAX_DYN_SMEM); };
   CK(set(hex_patch_kernel<R, 64, 0>));
