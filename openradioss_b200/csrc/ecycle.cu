@@ -416,7 +416,7 @@ struct Impl {
     bool on = false;
     int G = 0, P = 0, ncmax = 0;
     int T = 0;                 // threads per CTA
-    int stall_cta = -1;        // test hook, OR_ECYCLE_TEST_STALL_CTA
+    int stall_cta = -1, stall_slots = -1;   // test hooks, OR_ECYCLE_TEST_STALL_CTA and _SLOTS
     size_t smem = 0;
     int nlist = 0;             // words of a CTA's corner lists, at most
     int npt = 0;               // points whose state stays on the chip (PersistShell), 0: in memory
@@ -492,7 +492,7 @@ struct Impl {
     a.fslot2 = per.fslot2.p; a.mslot2 = per.mslot2.p; a.acc3 = per.acc3.p; a.ek_node = per.ek.p;
     a.ekr_node = per.ekr.p; a.sync = per.sync.p; a.patches_per_cta = per.P; a.ncmax = per.ncmax;
     a.ntiles_node = ntiles;
-    a.stall_cta = per.stall_cta;
+    a.stall_cta = per.stall_cta; a.stall_slots = per.stall_slots;
     return a;
   }
 };
@@ -819,8 +819,9 @@ int persist_build(or_ecycle* h, Impl<R>& m) {
       (rc = dput(h, q.ek, std::vector<double>(m.nnodpad, 0.0))) ||
       (rc = dput(h, q.ekr, std::vector<double>(m.nnodpad, 0.0))))
     return rc;
-  q.stall_cta = -1;
+  q.stall_cta = q.stall_slots = -1;
   if (const char* st = std::getenv("OR_ECYCLE_TEST_STALL_CTA")) q.stall_cta = std::atoi(st);
+  if (const char* st = std::getenv("OR_ECYCLE_TEST_STALL_SLOTS")) q.stall_slots = std::atoi(st);
   q.on = true;
   q.G = G; q.P = P; q.T = T; q.ncmax = ncmax; q.nlist = nlist; q.npt = npt; q.smem = smem;
   return OR_OK;

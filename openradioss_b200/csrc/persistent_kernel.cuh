@@ -43,9 +43,9 @@
 // (the lowest CTA that holds it) writes it back, the element state is written back, and the
 // kinetic energy is summed per node tile exactly as the node pass sums it.
 //
-// The counter and the slots are polled with a time limit: past the limit a CTA sets an
-// abort flag and the OR_E_TIMEOUT error word, and every CTA leaves at its next wait, so
-// the launch always ends.
+// The counter and the slots are polled with a time limit: past the limit a CTA sets the
+// OR_E_TIMEOUT error word and an abort flag, and every CTA leaves at its next wait, so
+// the launch always ends, with nothing written back.
 #pragma once
 #include "ecycle_kernels.cuh"
 #include "hex_pair.cuh"
@@ -75,8 +75,10 @@ struct PersistArgs {
   int ncmax;                  // node capacity of a CTA (stride of the shared planes)
   int nlist;                  // list capacity of a CTA
   int ntiles_node;            // node tiles of NODE tile size 128 (kinetic energy partials)
-  int stall_cta;              // test hook (OR_ECYCLE_TEST_STALL_CTA): this CTA does not arrive at the
-                              // first cycle's counter, so the others' bounded waits run out; -1 off
+  // Test hooks, -1 off: this CTA does not arrive at the first cycle's counter
+  // (OR_ECYCLE_TEST_STALL_CTA), or does not write that cycle's slots
+  // (OR_ECYCLE_TEST_STALL_SLOTS), so that the others' bounded waits run out.
+  int stall_cta, stall_slots;
 };
 constexpr int SYNC_END = 32, SYNC_WORDS = 64;        // the two counters on lines of their own
 
@@ -117,6 +119,13 @@ __device__ __forceinline__ void grid_arrive(unsigned* count) {
   __threadfence();
   atomicAdd(count, 1u);
 }
+// Ends the launch with OR_E_TIMEOUT: the error word first, so that no CTA that leaves on the
+// flag raises an error of its own before it
+__device__ __forceinline__ void give_up(unsigned* abort, ErrorWord* err) {
+  raise_error(err, 7, (int)blockIdx.x);
+  __threadfence();
+  atomicExch(abort, 1u);
+}
 // Wait until `target` arrivals were counted; true when the launch must end (a CTA gave up)
 __device__ __forceinline__ bool grid_wait(unsigned* count, unsigned target, unsigned* abort, ErrorWord* err) {
   const long long t0 = clock64();
@@ -124,8 +133,7 @@ __device__ __forceinline__ bool grid_wait(unsigned* count, unsigned target, unsi
     if (ld_acquire(count) >= target) return false;  // acquire: every CTA's writes before its arrival
     if (__ldcg(abort)) break;
     if (clock64() - t0 > (1ll << 31)) {             // about a second at the SM clock
-      atomicExch(abort, 1u);
-      raise_error(err, 7, (int)blockIdx.x);
+      give_up(abort, err);
       break;
     }
     __nanosleep(20);
@@ -577,7 +585,7 @@ cycle_persistent_kernel(typename Kind::Args a, NodeArgs<R> na, PersistArgs pa, i
     }
     if (courier) {
       bool out = !mbar_wait(&s_dtbar, c & 1, STAGE_WAIT_TRIES);
-      if (out) { atomicExch(abort, 1u); raise_error(a.err, 7, cta); }
+      if (out) give_up(abort, a.err);
       PartAcc* acc = &pa.acc3[c % 3];
       atomicMin(&acc->dtkey, s_dt[0]);
       atomicMin(&acc->dtbits, s_dt[1]);
@@ -619,7 +627,8 @@ cycle_persistent_kernel(typename Kind::Args a, NodeArgs<R> na, PersistArgs pa, i
       if (last && sown[i]) { pa.ek_node[g] = ek; pa.ekr_node[g] = ekr; }
     };
     // shared nodes: this CTA's patch partials to their slots, and the next cycle's cleared
-    for (int i = tid; i < nsh; i += blockDim.x) {
+    const int nwrite = c == 0 && cta == pa.stall_slots ? 0 : nsh;
+    for (int i = tid; i < nwrite; i += blockDim.x) {
       const int2 lr = slist[i];
       for (int w = lr.x; w < lr.y;) {
         R f[C];
@@ -678,8 +687,10 @@ cycle_persistent_kernel(typename Kind::Args a, NodeArgs<R> na, PersistArgs pa, i
               if ((tries & 63) == 63) {
                 if (!t0) t0 = clock64();
                 const bool late = clock64() - t0 > (1ll << 31);       // about a second at the SM clock
-                if (late) { atomicExch(abort, 1u); raise_error(a.err, 7, cta); }
-                if (late || __ldcg(abort)) { s_abort = 1; break; }
+                if (late) give_up(abort, a.err);
+                // on without the slots: the NaN in their place reaches no result, and the error
+                // that the node's update raises for it comes after the abort's own
+                if (late || __ldcg(abort)) { __threadfence(); s_abort = 1; break; }
               }
             }
 #pragma unroll
