@@ -119,11 +119,9 @@ __device__ __forceinline__ void grid_arrive(unsigned* count) {
   __threadfence();
   atomicAdd(count, 1u);
 }
-// Ends the launch with OR_E_TIMEOUT: the error word first, so that no CTA that leaves on the
-// flag raises an error of its own before it
+// Ends the launch with OR_E_TIMEOUT.  A CTA that leaves on the flag raises nothing of its own.
 __device__ __forceinline__ void give_up(unsigned* abort, ErrorWord* err) {
   raise_error(err, 7, (int)blockIdx.x);
-  __threadfence();
   atomicExch(abort, 1u);
 }
 // Wait until `target` arrivals were counted; true when the launch must end (a CTA gave up)
@@ -708,9 +706,16 @@ cycle_persistent_kernel(typename Kind::Args a, NodeArgs<R> na, PersistArgs pa, i
                 if (!t0) t0 = clock64();
                 const bool late = clock64() - t0 > (1ll << 31);       // about a second at the SM clock
                 if (late) give_up(abort, a.err);
-                // on without the slots: the NaN in their place reaches no result, and the error
-                // that the node's update raises for it comes after the abort's own
-                if (late || __ldcg(abort)) { __threadfence(); s_abort = 1; break; }
+                if (late || __ldcg(abort)) {
+                  // zeros for the slots that did not come: their NaN would raise OR_E_NAN
+#pragma unroll
+                  for (int u = 0; u < U; ++u) {
+                    F[u] = mk4(R(0), R(0), R(0), R(0));
+                    if constexpr (ROT) M[u] = F[u];
+                  }
+                  s_abort = 1;
+                  break;
+                }
               }
             }
 #pragma unroll
