@@ -420,6 +420,7 @@ struct Impl {
     size_t smem = 0;
     int nlist = 0;             // words of a CTA's corner lists, at most
     int npt = 0;               // points whose state stays on the chip (PersistShell), 0: in memory
+    bool planes = false;       // FP64: in shared planes
     DBuf<int> node_ofs, node_glob, node_nshared, list_ofs, list; DBuf<unsigned char> owner; DBuf<unsigned short> pconn;
     DBuf<R4> fslot2, mslot2; DBuf<PartAcc> acc3; DBuf<double> ek, ekr; DBuf<unsigned> sync;
   } per;
@@ -658,12 +659,14 @@ int set_smem_attrs(or_ecycle* h, Impl<R>& m) {
 // too; for anything else with the points' state in memory.  22,801 shells of 3 points with
 // the Newton return in FP64 took 16.4 us a cycle from memory, 12.7 so.
 template <class R, int TILE, int MAXT>
-const void* persist_fn_tile(const Impl<R>& m, bool shells, int npt) {
+const void* persist_fn_tile(const Impl<R>& m, bool shells, int npt, bool planes) {
 #define ORB_FN(...) (const void*)cycle_persistent_kernel<__VA_ARGS__, R, MAXT>
   if (!shells) {
     if constexpr (sizeof(R) == 4) return m.any_corot ? ORB_FN(PersistHexPair<64, 1>) : ORB_FN(PersistHexPair<64, 0>);
     else return m.any_corot ? ORB_FN(PersistHexa<64, 1>) : ORB_FN(PersistHexa<64, 0>);
   }
+  if constexpr (sizeof(R) == 8 && MAXT == PERSIST_THREADS && TILE < 256)
+    if (npt == 5 && m.uniform_npt == 5 && !planes) return ORB_FN(PersistShell<R, TILE, 5, false, true>);
   if (npt == 5 && m.uniform_npt == 5) return ORB_FN(PersistShell<R, TILE, 5, false>);
   if (npt == 5) return ORB_FN(PersistShell<R, TILE, 5, true>);
   if (npt == 3) return ORB_FN(PersistShell<R, TILE, 3, true>);
@@ -671,17 +674,17 @@ const void* persist_fn_tile(const Impl<R>& m, bool shells, int npt) {
 #undef ORB_FN
 }
 template <class R>
-const void* persist_fn(const or_ecycle* h, const Impl<R>& m, int threads, int npt) {
+const void* persist_fn(const or_ecycle* h, const Impl<R>& m, int threads, int npt, bool planes) {
   const bool shells = h->hex.empty();
   const int tile = shells ? h->tile_shell : h->tile_hex;
   if constexpr (sizeof(R) == 8) {
     if (persist_maxt(threads, true) == 256)
-      return tile == 64 ? persist_fn_tile<R, 64, 256>(m, shells, npt)
-             : tile == 128 ? persist_fn_tile<R, 128, 256>(m, shells, npt) : persist_fn_tile<R, 256, 256>(m, shells, npt);
+      return tile == 64 ? persist_fn_tile<R, 64, 256>(m, shells, npt, planes)
+             : tile == 128 ? persist_fn_tile<R, 128, 256>(m, shells, npt, planes) : persist_fn_tile<R, 256, 256>(m, shells, npt, planes);
   }
-  return tile == 64 ? persist_fn_tile<R, 64, PERSIST_THREADS>(m, shells, npt)
-         : tile == 128 ? persist_fn_tile<R, 128, PERSIST_THREADS>(m, shells, npt)
-                       : persist_fn_tile<R, 256, PERSIST_THREADS>(m, shells, npt);
+  return tile == 64 ? persist_fn_tile<R, 64, PERSIST_THREADS>(m, shells, npt, planes)
+         : tile == 128 ? persist_fn_tile<R, 128, PERSIST_THREADS>(m, shells, npt, planes)
+                       : persist_fn_tile<R, 256, PERSIST_THREADS>(m, shells, npt, planes);
 }
 
 // Sets up the persistent launch when the handle qualifies: step() through a graph
@@ -794,11 +797,12 @@ int persist_build(or_ecycle* h, Impl<R>& m) {
     nlist = std::max(nlist, (int)words.size() - w0);
   }
   // the points of the shell kernel that keeps their state on the chip (PersistShell); in
-  // FP64 it lies in shared memory, and where that does not fit it stays in global memory
+  // FP64 it lies in shared memory
   int npt = shells && (m.same_npt == 5 || m.same_npt == 3) ? m.same_npt : 0;
   size_t smem = persist_smem<R>(node_r, corner_r + (sizeof(R) == 8 ? 6 * npt * tile : 0), ncmax, P, nlist);
-  if (npt && sizeof(R) == 8 && smem > PERSIST_MAX_SMEM) {
-    npt = 0;
+  bool planes = npt && sizeof(R) == 8;
+  if (planes && smem > PERSIST_MAX_SMEM) {
+    planes = false;
     smem = persist_smem<R>(node_r, corner_r, ncmax, P, nlist);
   }
   if (smem > PERSIST_MAX_SMEM) return OR_OK;
@@ -806,7 +810,11 @@ int persist_build(or_ecycle* h, Impl<R>& m) {
   // nodes than that (node phases of one node per thread), in whole TILE groups
   const int want = std::max(P * NT + 32, ncmax), unit = shells ? tile : 128;
   const int T = std::min(PERSIST_THREADS / unit * unit, (want + unit - 1) / unit * unit);
-  const void* fn = persist_fn<R>(h, m, T, npt);
+  // and where that does not fit, in registers for 5 points of Ishell 1 (the kernels for
+  // PERSIST_THREADS), else in global memory
+  if (sizeof(R) == 8 && !planes && !(npt == 5 && m.uniform_npt == 5 && tile < 256 && persist_maxt(T, true) == PERSIST_THREADS))
+    npt = 0;
+  const void* fn = persist_fn<R>(h, m, T, npt, planes);
   CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, PERSIST_MAX_SMEM));
   int nb = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, T, smem));
@@ -823,7 +831,7 @@ int persist_build(or_ecycle* h, Impl<R>& m) {
   if (const char* st = std::getenv("OR_ECYCLE_TEST_STALL_CTA")) q.stall_cta = std::atoi(st);
   if (const char* st = std::getenv("OR_ECYCLE_TEST_STALL_SLOTS")) q.stall_slots = std::atoi(st);
   q.on = true;
-  q.G = G; q.P = P; q.T = T; q.ncmax = ncmax; q.nlist = nlist; q.npt = npt; q.smem = smem;
+  q.G = G; q.P = P; q.T = T; q.ncmax = ncmax; q.nlist = nlist; q.npt = npt; q.planes = planes; q.smem = smem;
   return OR_OK;
 }
 
@@ -839,7 +847,7 @@ int launch_persistent(or_ecycle* h, Impl<R>& m, int ncycles, int parity0) {
   PersistArgs pa = m.pargs();
   const float* zw = m.zw.p;
   void* args[] = {h->hex.empty() ? (void*)&sa : (void*)&ha, &na, &pa, &ncycles, &parity0, &zw};
-  const void* fn = persist_fn<R>(h, m, q.T, q.npt);
+  const void* fn = persist_fn<R>(h, m, q.T, q.npt, q.planes);
   Trace tr("persistent cycles");
   const cudaError_t e =
       cudaLaunchCooperativeKernel(fn, dim3(q.G), dim3(q.T), args, q.smem, h->stream);

@@ -191,11 +191,13 @@ constexpr int persist_maxt(int threads, bool fp64) { return fp64 && threads <= 2
 // corner k of element t at pair k * TILE + t.  In FP64 the integration points' state (60
 // registers for 5 points) is kept in shared planes instead of registers, which spilled:
 // the 200x200 plate 18.9 -> 16.1 us a cycle together with the single node update below.
-template <class R, int TILE_, int NPT, bool GEN>
+// Where the planes do not fit (six patches of 64 a CTA), 5 points of Ishell 1 stay in
+// registers (REGS): 47,961 shells 20.6 us a cycle, 24.7 with the state read from memory.
+template <class R, int TILE_, int NPT, bool GEN, bool REGS = false>
 struct PersistShell {
   typedef ShellArgs<R> Args;
   typedef typename Vec2<R>::T R2;
-  static constexpr bool KEEP = NPT > 0, PLANES = KEEP && sizeof(R) == 8;
+  static constexpr bool KEEP = NPT > 0, PLANES = KEEP && sizeof(R) == 8 && !REGS;
   static constexpr int TILE = TILE_, NT = TILE, C = 6, NODE_R = 8, CORNER_R = 24 * TILE,
                        STATE_R = PLANES ? 6 * NPT * TILE : 0;
   ShellState<R, NPT> st;
