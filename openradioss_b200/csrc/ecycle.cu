@@ -941,9 +941,13 @@ int finalize_impl(or_ecycle* h) {
   // tiles left to the library (cfg.block_hex / block_shell 0): 64 elements per patch
   // when the patches at 64 fit one wave of the kernel's resident CTAs (a latency-bound
   // mesh gains from more CTAs), 128 otherwise; the autotuner times all three.  Split hexas
-  // keep 64 only as far as the persistent cycle reaches (12 patches of 32 threads,
-  // two hexas each, per CTA): beyond it the patches at 64 ran 125,911 hexas in 25.1 us a cycle,
-  // those at 128 in 21.0 (B200), although 64 still fit one wave up to 132,600.
+  // keep 64 only as far as the persistent cycle reaches (12 patches of 32 threads, two hexas
+  // each, per CTA, 113,664 hexas).  Microseconds a cycle at 64 and at 128 beyond it (B200): one
+  // part of 120,000 21.2 and 20.2, of 125,911 25.1 and 21.0, whether it could run the persistent
+  // cycle or not; 120,000 with a skin 28.5 and 28.0; 2 to 40 parts of 113,700 to 123,000 beside
+  // plates 0.975 to 1.17 times as long at 64, the most where the plates are small.  Parts of
+  // hexas alone are 0 to 3 % faster at 64 up to 13 patches per SM, what its registers and
+  // shared memory hold (122,112 in 16 parts 22.0 and 22.7; 124,416 24.4 and 23.0).
   {
     auto tile_for = [&](long long nel, int ctas128) {
       return nel <= (long long)h->nsm * (2 * ctas128) * 64 ? 64 : 128;
@@ -952,7 +956,7 @@ int finalize_impl(or_ecycle* h) {
     for (auto& g : h->hex) nh += g.nel;
     for (auto& g : h->shell) ns += g.nel;
     if (h->cfg.block_hex == 0)
-      h->tile_hex = sizeof(R) == 4 && nh > (long long)h->nsm * (PERSIST_THREADS / 32) * 64
+      h->tile_hex = sizeof(R) == 4 && nh > (long long)h->nsm * (m.nparts > 1 && !ns ? 13 : PERSIST_THREADS / 32) * 64
                         ? 128 : tile_for(nh, Occupancy<R>::hex);
     if (h->cfg.block_shell == 0) h->tile_shell = tile_for(ns, Occupancy<R>::shell);
   }
