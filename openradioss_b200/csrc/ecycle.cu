@@ -1531,10 +1531,11 @@ double* pinned_device_ptr(double* host, size_t bytes) {
 
 // Nodes that one kernel writes straight into the caller's pinned arrays, instead of a
 // kernel and a copy through the staging buffer per array: three arrays of 1,403 nodes 45 -> 20 us,
-// of 40,401 nodes 95 -> 73 us, two of 134,064 148 -> 140 us.  From there on the link's rate
-// decides (262,701 nodes 257 us either way), and at 2 M nodes the copy engine is ahead (1778
-// against 1886 us).
-constexpr int DIRECT_NODES = 1 << 18;
+// of 40,401 nodes 95 -> 73 us, two of 131,769 145 -> 138 us.  From there on the link's rate
+// decides (two of 262,144 nodes 257 us either way), and at 2 M nodes the copy engine is ahead
+// (1778 against 1886 us).  One array alone saves nothing but its latency: 63,001 nodes 46 us
+// either way, 160,801 88 by the copy and 90 by the kernel, 262,144 132 and 138.
+constexpr int DIRECT_NODES = 1 << 18, DIRECT_NODES_ONE = 1 << 16;
 
 template <class R>
 int get_nodes_impl(or_ecycle* h, int part, double* x, double* d, double* v, double* vr) {
@@ -1544,7 +1545,8 @@ int get_nodes_impl(or_ecycle* h, int part, double* x, double* d, double* v, doub
   if (n == 0) return OR_OK;
   if (vr && !m.VR.p) std::fill(vr, vr + 3 * (size_t)n, 0.0);
   double* dst[4] = {x, d, v, m.VR.p ? vr : nullptr};
-  if (n <= DIRECT_NODES) {
+  const int wanted = (dst[0] != nullptr) + (dst[1] != nullptr) + (dst[2] != nullptr) + (dst[3] != nullptr);
+  if (n <= (wanted > 1 ? DIRECT_NODES : DIRECT_NODES_ONE)) {
     double* dev[4] = {nullptr, nullptr, nullptr, nullptr};
     bool direct = true;
     for (int kind = 0; kind < 4 && direct; ++kind)
