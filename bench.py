@@ -341,7 +341,7 @@ def adjoint_timing(device, ncycles=500, checkpoint=50, reps=3):
 def kernel_roofline(h, deck, cycles, workload, s=4, step_ms=None):
     """Per-kernel device times (each phase kernel launched back to back from a graph
     on the state a full run leaves, CUDA events on the handle's stream) and the
-    roofline of the dominant one.  When the handle steps with the persistent shell
+    roofline of the dominant one.  When the handle steps with the persistent
     cycle, that kernel is the dominant one: one launch per step of ``cycles``
     cycles, timed live (``step_ms``), and its algorithmic bytes are those of the
     work it does, the per-cycle element and node bytes times the cycles (the
@@ -350,6 +350,7 @@ def kernel_roofline(h, deck, cycles, workload, s=4, step_ms=None):
     from openradioss_b200 import roofline
     h.reset()
     h.step(cycles)
+    persistent = h.launch_count() == 1
     kt = h.kernel_times(reps=64)            # microseconds per launch; resets the handle
     eb_hex = sum(g["ixs"].shape[0] * roofline.hex_bytes(s, g["mat"]["law"]) for p in deck["parts"] for g in p["hex"])
     eb_shell = sum(g["ixc"].shape[0] * roofline.shell_bytes(s, g["prop"]["npt"])
@@ -374,7 +375,7 @@ def kernel_roofline(h, deck, cycles, workload, s=4, step_ms=None):
             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "traffic": traffic, "algorithmic_bytes_per_launch": dom_bytes,
             "avg_launch_ms": dom_ms, "peak_source": peak_src}
-    if h.persistent_info()[0] and step_ms:
+    if persistent and step_ms:
         pb = (eb + nb) * cycles
         ptraffic = None
         if os.path.exists(tpath):     # staged once per launch: the DRAM bytes do not grow with its cycles
@@ -383,7 +384,7 @@ def kernel_roofline(h, deck, cycles, workload, s=4, step_ms=None):
             except (OSError, ValueError):
                 ptraffic = None
         pa = pb / (step_ms * 1e-3) / 1e9
-        roof = {"bound": "hbm", "kernel": "shell_persistent_kernel", "achieved": pa, "peak": peak, "unit": "GB/s",
+        roof = {"bound": "hbm", "kernel": "cycle_persistent_kernel", "achieved": pa, "peak": peak, "unit": "GB/s",
                 "frac": pa / peak, "traffic": ptraffic, "algorithmic_bytes_per_launch": pb, "avg_launch_ms": step_ms,
                 "cycles_per_launch": cycles, "peak_source": peak_src,
                 "note": "per-phase kernels below are timed alone for comparison; the timed steps ran this kernel"}
@@ -465,8 +466,8 @@ def main():
     # ---- split form (the headline) ----
     hs = ECycle(deck, precision=abi.OR_PREC_SPLIT, device=local, graph=1, block_hex=bh_s, block_shell=bs_s,
                 persistent=pe_s)
-    persistent_on = bool(hs.persistent_info()[0])
     timed_runs(hs, cycles, 0, 1)              # graph capture + first-touch outside timing
+    persistent_on = hs.launch_count() == 1    # all the cycles of a step in one launch
     sampler = ClockSampler(local)
     sampler.start()
     ms_split, launches = timed_runs(hs, cycles, args.steps, args.warmup)
@@ -535,7 +536,7 @@ def main():
             "tuning": {"cuda_graph_cycles": 32, "tile_hex": bh_s, "tile_shell": bs_s,
                        "persistent_cycle": persistent_on,
                        "autotune_ms_per_cycle": {"split": tune_s, "fp64": tune_d},
-                       "autotune_keys": "tile (hAsB: hexa tile A, shell tile B), p = persistent shell cycle"},
+                       "autotune_keys": "tile (hAsB: hexa tile A, shell tile B), p = persistent cycle"},
             "fp64": {"value": value_fp64, "ms_per_step": t_fp64, "dtype": "f64", "tile_hex": bh_d, "tile_shell": bs_d,
                      "persistent_cycle": pe_d == 0},
             "split_over_fp64": value / value_fp64,
