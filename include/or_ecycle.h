@@ -324,8 +324,10 @@ int  or_ecycle_stream(or_ecycle* h, void** stream);
 int  or_ecycle_device_bytes(or_ecycle* h, long long* bytes);
 /* Whether or_ecycle_step runs a shell mesh's cycles in the persistent form: one
    cooperative launch per call in which each CTA (one per SM) keeps its patches'
-   element state in registers and their nodes in shared memory, with one grid
-   barrier per cycle.  Chosen at finalize for one part of shell groups with no
+   elements on the chip (3 or 5 integration points in registers, in FP64 in shared
+   memory where they fit; other points are read from memory) and their nodes in
+   shared memory.  CTAs meet at one grid-wide counter per cycle, for the time step,
+   and at the force slots of the nodes they share, each its own flag.  Chosen at finalize for one part of shell groups with no
    rigid links and no /CLOAD or /PLOAD loads, graph = 1, whose patches fit one
    wave; cfg.persistent = -1, or OR_ECYCLE_PERSISTENT=0 in the environment, turns
    it off.  It performs the per-phase kernels' operations in the same order, so
@@ -334,7 +336,8 @@ int  or_ecycle_device_bytes(or_ecycle* h, long long* bytes);
    fuse a multiply-add in one kernel and not in the other, and the two agree to
    rounding.  ctas, threads: its launch shape (0 when off; either may be NULL).
    One part of hexa groups that fits likewise runs in a persistent form of its own,
-   under the same conditions and switches; it is not reported here (on = 0).  In
+   under the same conditions and switches; it is not reported here (on = 0), but by
+   or_ecycle_launch_count, which is 1 after a step in either persistent form.  In
    FP64 it too performs the per-phase kernels' operations in their order; in the
    split form the two agree to rounding.
    No counterpart in the reference. */

@@ -45,7 +45,7 @@
 namespace {
 
 // 64 hexas per CTA: the largest group is then 512 CTAs, one wave at the 4 CTAs per SM
-// that the element kernel's 210 registers allow; at 128 the 216 CTAs of a 27,648-hexa
+// that the element kernel's 214 registers allow; at 128 the 216 CTAs of a 27,648-hexa
 // group left most SMs with one CTA and some with two.
 constexpr int NOALLOC_TILE = 64;
 constexpr int NOALLOC_NODE_TILE = 128;
